@@ -1020,24 +1020,118 @@ bool term_breaks_constraint(const DeviceConstraint& c, uint64_t l, uint64_t r) {
          __builtin_popcountll(l & ~lo) != __builtin_popcountll(r & ~lo);
 }
 
-// Device layout: v (double2, 16-byte aligned) first, then m, l, r, x, s (uint64), xinfo (uint32).
-int upload_terms(const TermTable& t, const DeviceConstraint& cons, DeviceTermSet* out) {
-  const size_t n = (size_t)std::max(t.n, 1);
-  const size_t bytes = n * (16 + 5 * 8 + 4);
-  std::vector<uint8_t> host(bytes, 0);
-  uint8_t* p = host.data();
-  auto put = [&](const void* src, size_t sz, size_t off) {
-    if (t.n > 0) memcpy(p + off, src, sz);
+// Host image of the row-group tables (DeviceRowTerms): one byte block and the offsets of its arrays.
+struct RowTables {
+  DeviceRowTerms shape;  // counts only
+  std::vector<uint64_t> sm, sl1, sl2, xmask;
+  std::vector<uint32_t> st, tinfo;
+  std::vector<double> cval;  // interleaved
+};
+
+// The class of coefficient v (equal up to sign) in cval, appended when new; *neg: v = -class value.
+int coefficient_class(std::vector<double>* cval, double re, double im, bool* neg) {
+  const int n = (int)(cval->size() / 2);
+  for (int c = 0; c < n; ++c) {
+    const double a = (*cval)[2 * c], b = (*cval)[2 * c + 1];
+    if (a == re && b == im) return *neg = false, c;
+    if (a == -re && b == -im) return *neg = true, c;
+  }
+  cval->push_back(re);
+  cval->push_back(im);
+  *neg = false;
+  return n;
+}
+
+constexpr int kMaxRowClasses = 64;
+
+// Slots, patterns and classes of off-diagonal terms (matched through t.l).
+RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons) {
+  RowTables R;
+  if (t.n > 32767) return R;
+  std::unordered_map<uint64_t, int> pattern;
+  std::unordered_map<uint64_t, std::vector<int>> open;  // mask -> slots with a free second pattern
+  R.tinfo.assign((size_t)std::max(t.n, 1), 0);
+  for (int k = 0; k < t.n; ++k) {
+    const auto it = pattern.emplace(t.x[k], (int)pattern.size());
+    if (it.second) R.xmask.push_back(t.x[k]);
+    bool neg = false;
+    const int cls = coefficient_class(&R.cval, t.v[2 * k], t.v[2 * k + 1], &neg);
+    if (cls >= kMaxRowClasses) return R;
+    R.tinfo[k] = (uint32_t)it.first->second | ((uint32_t)cls << 16) | (neg ? 1u << 31 : 0u) |
+                 (term_breaks_constraint(cons, t.l[k], t.r[k]) ? kRowTermNeedsCheck : 0u);
+    std::vector<int>& free_slots = open[t.m[k]];
+    size_t f = 0;
+    while (f < free_slots.size() && R.sl1[free_slots[f]] == t.l[k]) ++f;
+    if (f < free_slots.size()) {
+      const int s = free_slots[f];
+      R.sl2[s] = t.l[k];
+      R.st[s] |= (uint32_t)k << 16;
+      free_slots.erase(free_slots.begin() + f);
+    } else {
+      free_slots.push_back((int)R.sm.size());
+      R.sm.push_back(t.m[k]);
+      R.sl1.push_back(t.l[k]);
+      R.sl2.push_back(~0ull);
+      R.st.push_back((uint32_t)k);
+    }
+  }
+  R.shape.n_slots = (int)R.sm.size();
+  R.shape.slot_blocks = (R.shape.n_slots + 31) / 32;
+  R.sm.resize(32 * (size_t)R.shape.slot_blocks, 0);
+  R.sl1.resize(R.sm.size(), ~0ull);
+  R.sl2.resize(R.sm.size(), ~0ull);
+  R.st.resize(R.sm.size(), 0);
+  R.shape.n_pat = (int)R.xmask.size();
+  R.shape.n_cls = (int)(R.cval.size() / 2);
+  R.shape.ok = 1;
+  return R;
+}
+
+// Blocks of 32 diagonal terms of one class each (matched through t.r).
+RowTables diag_rows(const TermTable& t) {
+  RowTables R;
+  std::vector<std::vector<std::pair<int, bool>>> members;
+  for (int k = 0; k < t.n; ++k) {
+    bool neg = false;
+    const int cls = coefficient_class(&R.cval, t.v[2 * k], t.v[2 * k + 1], &neg);
+    if (cls >= kMaxRowClasses) return R;
+    if (cls >= (int)members.size()) members.resize(cls + 1);
+    members[cls].push_back({k, neg});
+  }
+  for (size_t c = 0; c < members.size(); ++c) {
+    for (size_t b = 0; b < members[c].size(); b += 32) {
+      const size_t n = std::min<size_t>(32, members[c].size() - b);
+      uint32_t signs = 0;
+      for (size_t i = 0; i < 32; ++i) {
+        const int k = i < n ? members[c][b + i].first : -1;
+        R.sm.push_back(k >= 0 ? t.m[k] : 0);
+        R.sl1.push_back(k >= 0 ? t.r[k] : ~0ull);
+        R.sl2.push_back(k >= 0 ? t.s[k] : 0);
+        if (k >= 0 && members[c][b + i].second) signs |= 1u << i;
+      }
+      R.st.push_back(signs);
+      R.tinfo.push_back((uint32_t)c | (b + 32 >= members[c].size() ? 1u << 31 : 0u));
+    }
+  }
+  R.shape.slot_blocks = (int)R.st.size();
+  R.shape.n_slots = t.n;
+  R.shape.n_cls = (int)(R.cval.size() / 2);
+  // one class per block: many classes of few terms would spend whole blocks on them
+  R.shape.ok = R.shape.slot_blocks <= t.n / 32 + 8;
+  return R;
+}
+
+// Device layout: v (double2, 16-byte aligned) first, then m, l, r, x, s (uint64), xinfo (uint32),
+// then the row-group tables, each array on a 16-byte boundary.
+int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal, DeviceTermSet* out) {
+  std::vector<uint8_t> host;
+  auto put = [&](const void* src, size_t sz) {
+    const size_t at = (host.size() + 15) & ~(size_t)15;
+    host.resize(at + std::max<size_t>(sz, 16), 0);
+    if (sz > 0) memcpy(host.data() + at, src, sz);
+    return at;
   };
-  const size_t ov = 0, om = n * 16, ol = om + n * 8, orr = ol + n * 8, ox = orr + n * 8, os = ox + n * 8;
-  const size_t oi = os + n * 8;
-  put(t.v.data(), t.n * 16, ov);
-  put(t.m.data(), t.n * 8, om);
-  put(t.l.data(), t.n * 8, ol);
-  put(t.r.data(), t.n * 8, orr);
-  put(t.x.data(), t.n * 8, ox);
-  put(t.s.data(), t.n * 8, os);
-  std::vector<uint32_t> xinfo(n, 0);
+  std::vector<uint32_t> xinfo((size_t)std::max(t.n, 1), 0);
   int all_two = t.n > 0 ? 1 : 0;
   for (int k = 0; k < t.n; ++k) {
     const uint64_t x = t.x[k];
@@ -1049,10 +1143,18 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, DeviceTermSet
     xinfo[k] = info;
     if (cnt != 2 || (info & kTermNeedsCheck)) all_two = 0;
   }
-  put(xinfo.data(), t.n * 4, oi);
+  const RowTables R = diagonal ? diag_rows(t) : off_diag_rows(t, cons);
+  const size_t n = (size_t)t.n;
+  const size_t ov = put(t.v.data(), n * 16), om = put(t.m.data(), n * 8), ol = put(t.l.data(), n * 8);
+  const size_t orr = put(t.r.data(), n * 8), ox = put(t.x.data(), n * 8), os = put(t.s.data(), n * 8);
+  const size_t oi = put(xinfo.data(), n * 4);
+  const size_t rsm = put(R.sm.data(), R.sm.size() * 8), rl1 = put(R.sl1.data(), R.sl1.size() * 8);
+  const size_t rl2 = put(R.sl2.data(), R.sl2.size() * 8), rst = put(R.st.data(), R.st.size() * 4);
+  const size_t rti = put(R.tinfo.data(), R.tinfo.size() * 4), rxm = put(R.xmask.data(), R.xmask.size() * 8);
+  const size_t rcv = put(R.cval.data(), R.cval.size() * 8);
   out->terms.all_two_site = all_two;
-  if (!cuda_ok(cudaMalloc(&out->block, bytes), "cudaMalloc(terms)")) return LS_GPU_ERR_CUDA;
-  if (!cuda_ok(cudaMemcpy(out->block, host.data(), bytes, cudaMemcpyHostToDevice), "upload terms"))
+  if (!cuda_ok(cudaMalloc(&out->block, host.size()), "cudaMalloc(terms)")) return LS_GPU_ERR_CUDA;
+  if (!cuda_ok(cudaMemcpy(out->block, host.data(), host.size(), cudaMemcpyHostToDevice), "upload terms"))
     return LS_GPU_ERR_CUDA;
   uint8_t* d = (uint8_t*)out->block;
   out->terms.n = t.n;
@@ -1063,6 +1165,15 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, DeviceTermSet
   out->terms.x = (const uint64_t*)(d + ox);
   out->terms.s = (const uint64_t*)(d + os);
   out->terms.xinfo = (const uint32_t*)(d + oi);
+  DeviceRowTerms& r = out->terms.rows;
+  r = R.shape;
+  r.sm = (const uint64_t*)(d + rsm);
+  r.sl1 = (const uint64_t*)(d + rl1);
+  r.sl2 = (const uint64_t*)(d + rl2);
+  r.st = (const uint32_t*)(d + rst);
+  r.tinfo = (const uint32_t*)(d + rti);
+  r.xmask = (const uint64_t*)(d + rxm);
+  r.cval = (const double2*)(d + rcv);
   return 0;
 }
 
@@ -1085,8 +1196,10 @@ OperatorCache* operator_cache(const ls_hs_operator* op) {
   c->off = read_terms(op->off_diag_terms);
   c->diag = read_terms(op->diag_terms);
   const DeviceConstraint cons = op->basis ? basis_constraint(op->basis) : DeviceConstraint{};
-  if (upload_terms(c->off, cons, &c->fwd_off) || upload_terms(adjoint_terms(c->off), cons, &c->adj_off) ||
-      upload_terms(c->diag, cons, &c->fwd_diag) || upload_terms(adjoint_terms(c->diag), cons, &c->adj_diag)) {
+  if (upload_terms(c->off, cons, false, &c->fwd_off) ||
+      upload_terms(adjoint_terms(c->off), cons, false, &c->adj_off) ||
+      upload_terms(c->diag, cons, true, &c->fwd_diag) ||
+      upload_terms(adjoint_terms(c->diag), cons, true, &c->adj_diag)) {
     free_cache(c);
     return nullptr;
   }

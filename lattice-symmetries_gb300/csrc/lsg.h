@@ -97,6 +97,27 @@ struct DeviceConstraint {
   int w0 = 0, w1 = 0;
 };
 
+// Term tables of the row-group kernels (rowgroup.cuh).
+// Off-diagonal: terms with the same mask m and different patterns l exclude each other, so up to
+// two of them share a slot (a row matches at most one) and 32 slots are tested by one ballot; terms
+// with equal flip masks share a pattern; coefficients equal up to sign share a class.
+// Diagonal: blocks of 32 terms of one class, whose signed count times the class value is summed.
+struct DeviceRowTerms {
+  int ok = 0;                      // the tables describe the terms (else too many classes or terms)
+  int n_slots = 0, slot_blocks = 0;  // slots, and blocks of 32 (padded with slots that never match)
+  const uint64_t* sm = nullptr;    // [32 * blocks] masks
+  const uint64_t* sl1 = nullptr;   // first pattern (diagonal: the pattern)
+  const uint64_t* sl2 = nullptr;   // second pattern, all ones without (diagonal: the sign mask s)
+  const uint32_t* st = nullptr;    // terms of the patterns, first | second << 16 (diagonal: per
+                                   // block, the signs of its 32 terms)
+  const uint32_t* tinfo = nullptr;  // [terms] pattern | class << 16 | check << 30 | sign << 31
+                                    // (diagonal: per block, class | last block of the class << 31)
+  int n_pat = 0, n_cls = 0;
+  const uint64_t* xmask = nullptr;  // [n_pat] flip masks
+  const double2* cval = nullptr;    // [n_cls]
+};
+constexpr uint32_t kRowTermNeedsCheck = 1u << 30;
+
 // Off-diagonal / diagonal term tables on the device.
 struct DeviceTerms {
   int n = 0;
@@ -112,6 +133,7 @@ struct DeviceTerms {
   const uint32_t* xinfo = nullptr;
   int all_two_site = 0;               // every term flips exactly two sites and keeps the basis'
                                       // conserved numbers (no term needs a constraint check)
+  DeviceRowTerms rows;
 };
 constexpr uint32_t kTermNeedsCheck = 1u << 24;
 
@@ -230,6 +252,14 @@ struct MatvecProblem {
   const double* xs = nullptr;
   int64_t ldxs = 0;
 };
+
+// Row-group kernels (matvec_rows.cu): y = H x with one lane per generated element.
+// rows_fit tells whether the tables of `p` fit; launch_rows runs k columns (complex: at most 16,
+// real: at most 32) from the prescaled gather source p.xs (leading dimension p.ldxs; even for two
+// or more real columns).
+bool rows_fit(const MatvecProblem& p);
+int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y, int64_t ldy,
+                int* d_err, const uint64_t* binom, cudaStream_t s);
 
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,
                   double* d_y, int64_t ldy, int* d_err, cudaStream_t s);
