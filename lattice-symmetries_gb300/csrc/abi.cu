@@ -1065,21 +1065,21 @@ RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons) {
     if (f < free_slots.size()) {
       const int s = free_slots[f];
       R.sl2[s] = t.l[k];
-      R.st[s] |= (uint32_t)k << 16;
+      R.st[s] = (R.st[s] & 0xffffu) | ((uint32_t)k << 16);
       free_slots.erase(free_slots.begin() + f);
     } else {
       free_slots.push_back((int)R.sm.size());
       R.sm.push_back(t.m[k]);
       R.sl1.push_back(t.l[k]);
-      R.sl2.push_back(~0ull);
+      R.sl2.push_back(t.l[k]);  // a slot of one term has it twice
       R.st.push_back((uint32_t)k);
     }
   }
   R.shape.n_slots = (int)R.sm.size();
   R.shape.slot_blocks = (R.shape.n_slots + 31) / 32;
   R.sm.resize(32 * (size_t)R.shape.slot_blocks, 0);
-  R.sl1.resize(R.sm.size(), ~0ull);
-  R.sl2.resize(R.sm.size(), ~0ull);
+  R.sl1.resize(R.sm.size(), 1);  // mask 0, pattern 1: never matches
+  R.sl2.resize(R.sm.size(), 1);
   R.st.resize(R.sm.size(), 0);
   R.shape.n_pat = (int)R.xmask.size();
   R.shape.n_cls = (int)(R.cval.size() / 2);
@@ -1105,7 +1105,7 @@ RowTables diag_rows(const TermTable& t) {
       for (size_t i = 0; i < 32; ++i) {
         const int k = i < n ? members[c][b + i].first : -1;
         R.sm.push_back(k >= 0 ? t.m[k] : 0);
-        R.sl1.push_back(k >= 0 ? t.r[k] : ~0ull);
+        R.sl1.push_back(k >= 0 ? t.r[k] : 1);
         R.sl2.push_back(k >= 0 ? t.s[k] : 0);
         if (k >= 0 && members[c][b + i].second) signs |= 1u << i;
       }

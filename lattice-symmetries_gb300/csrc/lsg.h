@@ -107,7 +107,7 @@ struct DeviceRowTerms {
   int n_slots = 0, slot_blocks = 0;  // slots, and blocks of 32 (padded with slots that never match)
   const uint64_t* sm = nullptr;    // [32 * blocks] masks
   const uint64_t* sl1 = nullptr;   // first pattern (diagonal: the pattern)
-  const uint64_t* sl2 = nullptr;   // second pattern, all ones without (diagonal: the sign mask s)
+  const uint64_t* sl2 = nullptr;   // second pattern, the first without one (diagonal: the sign mask s)
   const uint32_t* st = nullptr;    // terms of the patterns, first | second << 16 (diagonal: per
                                    // block, the signs of its 32 terms)
   const uint32_t* tinfo = nullptr;  // [terms] pattern | class << 16 | check << 30 | sign << 31
@@ -257,7 +257,7 @@ struct MatvecProblem {
 // rows_fit tells whether the tables of `p` fit; launch_rows runs k columns (complex: at most 16,
 // real: at most 32) from the prescaled gather source p.xs (leading dimension p.ldxs; even for two
 // or more real columns).
-bool rows_fit(const MatvecProblem& p);
+bool rows_fit(const MatvecProblem& p, int n_sectors = 0);
 int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y, int64_t ldy,
                 int* d_err, const uint64_t* binom, cudaStream_t s);
 

@@ -184,8 +184,8 @@ static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const do
 }
 
 // Row-group kernels wherever their tables fit (faster than the packed kernels at every measured size
-// and group: 1.4x at 576 images, 2.1x at 56, 8.7x at 150 with five columns; level at 257 rows,
-// where launches count); otherwise splits k right-hand sides into launches of
+// and group: 2.0x at 576 images, 2.3x at 56 with 16 columns, 9.7x at 150 with five; level at 257
+// rows, where launches count); otherwise splits k right-hand sides into launches of
 // 16, 8, 4 and 1 columns of the packed kernels.
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,
                   double* d_y, int64_t ldy, int* d_err, cudaStream_t s) {
@@ -318,6 +318,7 @@ struct SectorPlan {
   int64_t ldx = 0, ldy = 0;
   bool batched = false;      // the sectors can share one launch
   bool use_batched = true;   // ... and run() does so (else one launch per sector)
+  bool rows = false;         // the row-group form's tables fit
   MatvecProblem shared{};          // tables of the first sector (batched form)
   int64_t total_rows = 0;
   struct Chunk {
@@ -349,7 +350,8 @@ int sector_plan_build(const std::vector<MatvecProblem>& problems, bool shareable
                   p0.group.gpl <= kSectorMaxGpl && p0.group.onehot_packed != nullptr;
   if (plan->batched) {
     plan->shared = p0;
-    if (!packed_fits(p0, n)) plan->batched = false;
+    plan->rows = rows_fit(p0, n);
+    if (!plan->rows && !packed_fits(p0, n)) plan->batched = false;
   }
   if (plan->batched) {
     std::vector<SectorDesc> h(n);
@@ -366,6 +368,8 @@ int sector_plan_build(const std::vector<MatvecProblem>& problems, bool shareable
     int done = 0;
     while (done < k) {
       const int left = k - done;
+      // the packed kernels' column counts: they remain the form without memory for the scaled
+      // vectors and of the FP32-pair arithmetic
       const int chunk = left >= 16 ? 16 : left >= 8 ? 8 : left >= 4 ? 4 : 1;
       for (int i = 0; i < n; ++i) {
         h[i].x = xs[i] + (size_t)done * 2;
@@ -414,6 +418,55 @@ __global__ void k_prescale_pairs_sectors(const SectorDesc* __restrict__ desc, in
   }
 }
 
+// xs[row_begin_s + i][c] = x_s[i][c] * n_s[i] for every sector s (blockIdx.y) and all k complex columns.
+__global__ void k_prescale_sectors(const SectorDesc* __restrict__ desc, int n_sectors, int64_t total_rows, int k,
+                                   int64_t ldx, double2* __restrict__ xs) {
+  const int s = blockIdx.y;
+  const int64_t begin = desc[s].row_begin;
+  const int64_t n = (s + 1 < n_sectors ? desc[s + 1].row_begin : total_rows) - begin;
+  const double2* __restrict__ x = reinterpret_cast<const double2*>(desc[s].x);
+  const double* __restrict__ norms = desc[s].index.norms;
+  double2* __restrict__ out = xs + (size_t)begin * k;
+  const int64_t total = n * k;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = e / k, c = e - i * k;
+    const double nrm = __ldg(norms + i);
+    const double2 v = __ldg(x + i * ldx + c);
+    out[e] = make_double2(v.x * nrm, v.y * nrm);
+  }
+}
+
+// The batched launch by the row-group kernels.  Returns 1 when there is no memory for the prescaled
+// gather source (nothing has been launched).
+static int sector_plan_run_rows(const SectorPlan* plan, int* d_err, const uint64_t* binom, cudaStream_t s) {
+  const int n = plan->n_sectors;
+  double2* d_xs = nullptr;
+  if (cudaMallocAsync((void**)&d_xs, (size_t)plan->total_rows * plan->k * sizeof(double2), s) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  int rc = 0;
+  {
+    const int64_t per_sector = (plan->total_rows * plan->k + n - 1) / n;
+    const int bx = (int)std::max<int64_t>(1, std::min<int64_t>((per_sector + 255) / 256,
+                                                               ((int64_t)num_sms() * 16 + n - 1) / n));
+    StageScope stage("sectors.prescale", s);
+    k_prescale_sectors<<<dim3((unsigned)bx, (unsigned)n), 256, 0, s>>>(plan->chunks[0].d_desc, n, plan->total_rows,
+                                                                       plan->k, plan->ldx, d_xs);
+    if (!cuda_ok(cudaGetLastError(), "k_prescale_sectors")) rc = LS_GPU_ERR_CUDA;
+  }
+  // 16 columns per launch and the rest in one: the last starts at the first of the smaller chunks
+  for (const SectorPlan::Chunk& c : plan->chunks) {
+    if (rc != 0) break;
+    if (c.col % 16 != 0) continue;
+    StageScope stage("sectors.kernel", s);
+    rc = launch_rows_sectors(plan->shared, std::min(16, plan->k - c.col), c.col, c.d_desc, n, plan->total_rows, plan->ldx, plan->ldy,
+                             reinterpret_cast<const double*>(d_xs), plan->k, d_err, binom, s);
+  }
+  cudaFreeAsync(d_xs, s);
+  return rc;
+}
+
 int sector_plan_run(const SectorPlan* plan, int* d_err, cudaStream_t s) {
   if (!plan->batched || !plan->use_batched) {
     for (int i = 0; i < plan->n_sectors; ++i) {
@@ -430,6 +483,11 @@ int sector_plan_run(const SectorPlan* plan, int* d_err, cudaStream_t s) {
   // chunks of 8 or 16 columns run the FP32-pair kernels from a prescaled pair copy of all
   // sectors' columns (one streaming pass); the others gather x and the norms in FP64
   float4* d_xp = nullptr;
+  if (plan->rows && !(use_pairs(plan->shared.group.gpl) && packed_fits(plan->shared, plan->n_sectors))) {
+    const int rc = sector_plan_run_rows(plan, d_err, binom, s);
+    if (rc != 1) return rc;
+    if (!packed_fits(plan->shared, plan->n_sectors)) return fail(LS_GPU_ERR_CUDA, "no memory for the scaled vectors");
+  }
   const bool want_pairs = use_pairs(plan->shared.group.gpl) && plan->shared.nnz_counter == nullptr &&
                           std::any_of(plan->chunks.begin(), plan->chunks.end(),
                                       [](const SectorPlan::Chunk& c) { return c.k >= 8; });

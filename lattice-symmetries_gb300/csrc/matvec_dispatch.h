@@ -53,6 +53,11 @@ int launch_sectors_pair(int k, int gpl, bool inv, const MatvecProblem& p, int n_
 // x_j * n_j as float pairs.
 int launch_packed_pair(int k, int gpl, bool inv, const MatvecProblem& p, const double* x, int64_t ldx, double* y,
                        int64_t ldy, int* err, const uint64_t* binom, cudaStream_t s);
+// Row-group form (complex, at most 16 columns); xs_all holds x_j * n_j of all sectors (leading
+// dimension ldxs), col is the launch's first column.
+int launch_rows_sectors(const MatvecProblem& p, int k, int col, const SectorDesc* d_desc, int n_sectors,
+                        int64_t total_rows, int64_t ldx, int64_t ldy, const double* xs_all, int64_t ldxs, int* d_err,
+                        const uint64_t* binom, cudaStream_t st);
 constexpr int kSectorMaxGpl = 4;
 constexpr int kMaxSectors = 256;
 

@@ -5,24 +5,27 @@
 //   1. keeps g.a of every group element for each row in shared memory (the rows are sorted, so a
 //      row's images follow from the previous row's by the few bits that changed),
 //   2. lists the matching terms of all rows (one ballot per 32 term slots and row),
-//   3. resolves 32 elements at a time, one per lane: the lane walks the group elements, forms the
-//      candidates g.a ^ g.x from the row's images and the image of the term's flip pattern (a
-//      table over the distinct patterns), keeps their minimum and the element that reached it,
-//      and looks the representative up; the element becomes {column index, coefficient word},
-//   4. hands the resolved elements, row by row, to the caller (sums over right-hand sides, inner
-//      products).
+//   3. resolves them, one element (KEEP = false: two) per lane at a time: the lane walks the group elements,
+//      forms the candidates g.a ^ g.x from the row's images and the image of the element's flip
+//      pattern (a table over the distinct patterns), keeps the minimum and the element that
+//      reached it, and looks the representatives up,
+//   4. hands every resolved element {column index, coefficient word} to the caller.
 //
 // What bounds it and why this split.  With one warp per element every element costs the warp-wide
 // minimum, the tie pass, the term decoding and the bookkeeping of 32 lanes (~100 warp
 // instructions, whatever the group's size); with one lane per element these are shared by 32
 // elements and the scan is left with two 32-bit shared-memory loads, an XOR and half a
 // three-input minimum (with spin inversion also half a maximum) per group element and 32
-// elements.
+// elements.  Lanes take elements in one of two ways.  KEEP = false (one column): 32 / R lanes share
+// a row and sum their own elements in registers; a lane's two elements read the row's images once.
+// KEEP = true (several columns): the elements of all R rows are dealt to the lanes in the order of
+// the term slots, so that no lane idles (short rows filled only 70 % of the lanes the other way)
+// and neighbouring lanes read neighbouring patterns (few bank conflicts), and go to shared memory.
 //
-// Measured (GB300, warp per row before -> lane per element): T x C6 on 25 sites, 150 elements, 34.7e3
-// rows, 5 complex columns 1330 -> 154 us (the ragged block also scans once instead of twice);
-// 28-site chain, 56 images, 16 columns 3614 -> 1697 us; 4x4 Hubbard, 128 elements, 8 columns
-// 6735 -> 2967 us; 6x6 torus, 576 images, one column 169.8 -> 120.6 ms.
+// Measured (GB300, warp per row -> lane per element): T x C6 on 25 sites, 150 elements, 34.7e3 rows, 5
+// complex columns 1328 -> 137 us (the ragged block also scans once instead of twice); 28-site
+// chain, 56 images, 16 columns 3609 -> 1538 us; 4x4 Hubbard, 128 elements, 8 columns 6724 ->
+// 2351 us; 6x6 torus, 576 images, one column 169.3 -> 85.2 ms.
 //
 // Modes.  N32 (states of at most 32 bits): candidates are whole states, so their minimum is the
 // representative; the scan remembers the chunk of 8 elements that first reached it and a second
@@ -40,16 +43,20 @@
 namespace lsg {
 
 constexpr int kModeN32 = 0, kModeP16 = 1;
+// Elements that a lane takes at a time (6x6 torus, one column: 1 / 2 / 4 at a time 86.4 / 85.2 / 98 ms;
+// 4x4 Hubbard, 8 columns: 1 / 2 / 4 at a time 2444 / 2534 / 3600 us).
+template <bool KEEP>
+constexpr int kLaneElements = KEEP ? 1 : 2;
 
 // Shared-memory layout and shape of a row-group kernel (bytes from the start of dynamic shared
 // memory; w_* relative to a warp's area).
 struct RowsLayout {
-  int threads, R, cap, T, n_slots, slot_blocks, n_pat, n_diag_blocks;
+  int threads, R, lanes_per_row, lane_shift, cap, T, n_slots, slot_blocks, n_pat, n_diag_blocks;
   int G, words, stride, site_words;  // words of g-images per row / pattern, their padded strides
-  int nlow, perm_stride;             // P16: bits below the 16-bit prefix, bytes per element
+  int nlow, nlow_pad, perm_stride;   // P16: bits below the 16-bit prefix, rounded up to 4, bytes per element
   uint32_t off_site, off_img, off_perm, off_coef, off_sm, off_sl1, off_sl2, off_st, off_ti, off_ts, off_xm;
-  uint32_t off_dm, off_dr, off_ds, off_db, off_dv, off_fs, off_warp;
-  uint32_t warp_bytes, w_ent, w_ord, w_a;
+  uint32_t off_dm, off_dr, off_ds, off_db, off_dv, off_fs, off_sectors, off_first, off_warp;
+  uint32_t warp_bytes, w_ent, w_list, w_a;  // w_list: KEEP the elements' positions in scan order
   uint32_t total;
 };
 
@@ -68,41 +75,61 @@ __device__ __forceinline__ uint64_t shfl_u64(uint64_t v, int src) {
          __shfl_sync(0xffffffffu, (uint32_t)v, src);
 }
 
+// States as the tables hold them: 32-bit words where they fit.
+template <int MODE>
+struct StateWord {
+  using T = uint64_t;
+};
+template <>
+struct StateWord<kModeN32> {
+  using T = uint32_t;
+};
+__device__ __forceinline__ uint32_t shfl_state(uint32_t v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ uint64_t shfl_state(uint64_t v, int src) { return shfl_u64(v, src); }
+__device__ __forceinline__ int popc_state(uint32_t v) { return __popc(v); }
+__device__ __forceinline__ int popc_state(uint64_t v) { return __popcll(v); }
+__device__ __forceinline__ int low_bit(uint32_t v) { return __ffs(v) - 1; }
+__device__ __forceinline__ int low_bit(uint64_t v) { return __ffsll((long long)v) - 1; }
+
 // One warp's view of the tables and its own area.
-template <int MODE, bool INV, bool FERMI>
+template <int MODE, bool INV, bool FERMI, bool KEEP>
 struct RowGroup {
   static constexpr unsigned FULL = 0xffffffffu;
+  using State = typename StateWord<MODE>::T;
   static constexpr uint32_t kAbsent = 0xffffffffu;  // column index of an element outside the basis
 
   const RowsLayout& L;
   const MatvecProblem& p;
   unsigned char* smem;
   uint32_t* ga;       // [R][stride]
-  uint2* entries;     // [R][cap]: {t | row << 16, -} when listed, {column, coefficient word} resolved
-  uint16_t* order;    // listed elements in scan order (positions in entries)
-  uint64_t* rows;     // [R] row states
+  uint16_t* list;     // [R][cap]: the terms of each row's elements; KEEP: positions in entries, in scan order
+  uint2* entries;     // KEEP: [R][cap], {term | row << 16, -} when listed, {column, coefficient word} resolved
+  State* rows;        // [R] row states
   uint32_t img_s, ga_s;
   int lane;
-  uint64_t prev;      // state whose images are in row `prev_row` of ga
+  State prev;         // state whose images are in row `prev_row` of ga
   int prev_row;
+  bool minus;         // the spin inversion's character is -1
   // per group of rows: lane r < nr holds row r's state, inverse norm and number of elements
-  uint64_t a_l;
+  State a_l;
   double inv_l;
   int cnt_l;
   int nr;
+  int total;          // KEEP: elements of all rows
 
   __device__ __forceinline__ RowGroup(const RowsLayout& L_, const MatvecProblem& p_, unsigned char* s)
       : L(L_), p(p_), smem(s) {
     unsigned char* w = s + L.off_warp + (threadIdx.x >> 5) * L.warp_bytes;
     ga = (uint32_t*)w;
     entries = (uint2*)(w + L.w_ent);
-    order = (uint16_t*)(w + L.w_ord);
-    rows = (uint64_t*)(w + L.w_a);
+    list = (uint16_t*)(w + L.w_list);
+    rows = (State*)(w + L.w_a);
     img_s = (uint32_t)__cvta_generic_to_shared(s + L.off_img);
     ga_s = (uint32_t)__cvta_generic_to_shared(ga);
     lane = threadIdx.x & 31;
     prev = 0;
     prev_row = -1;
+    minus = p.group.spin_inversion == -1;
   }
 
   template <typename T>
@@ -114,58 +141,71 @@ struct RowGroup {
   __device__ __forceinline__ static void stage(const RowsLayout& L, const MatvecProblem& p, unsigned char* smem) {
     const int G = L.G, nb = p.group.n_bits;
     const int tid = threadIdx.x, nt = blockDim.x;
-    auto word = [&](uint64_t x, int w) -> uint32_t {  // word w of the images of the bits of x
-      if constexpr (MODE == kModeN32) {
-        const int g = w < G ? w : 0;
-        uint64_t v = 0;
-        for (; x != 0; x &= x - 1) v ^= __ldg(p.group.onehot + (__ffsll((long long)x) - 1) * G + g);
-        return (uint32_t)v;
-      } else {
-        const int g0 = 2 * w < G ? 2 * w : 0, g1 = 2 * w + 1 < G ? 2 * w + 1 : 0;
-        uint64_t v0 = 0, v1 = 0;
-        for (; x != 0; x &= x - 1) {
-          const uint64_t* r = p.group.onehot + (__ffsll((long long)x) - 1) * G;
-          v0 ^= __ldg(r + g0);
-          v1 ^= __ldg(r + g1);
-        }
-        return (uint32_t)(v0 >> (nb - 16)) | ((uint32_t)(v1 >> (nb - 16)) << 16);
-      }
-    };
     uint32_t* site = (uint32_t*)(smem + L.off_site);
+#pragma unroll 4
     for (int i = tid; i < nb * L.site_words; i += nt) {
       const int b = i / L.site_words, w = i - b * L.site_words;
-      site[i] = w < L.words ? word(1ull << b, w) : 0u;
-    }
-    uint32_t* img = (uint32_t*)(smem + L.off_img);
-    for (int i = tid; i < L.n_pat * L.words; i += nt) {
-      const int x = i / L.words, w = i - x * L.words;
-      img[x * L.stride + w] = word(__ldg(p.off.rows.xmask + x), w);
+      const uint64_t* r = p.group.onehot + b * G;
+      if constexpr (MODE == kModeN32) {
+        site[i] = w < L.words ? (uint32_t)__ldg(r + (w < G ? w : 0)) : 0u;
+      } else {
+        const uint64_t v0 = __ldg(r + (2 * w < G ? 2 * w : 0)), v1 = __ldg(r + (2 * w + 1 < G ? 2 * w + 1 : 0));
+        site[i] = w < L.words ? (uint32_t)(v0 >> (nb - 16)) | ((uint32_t)(v1 >> (nb - 16)) << 16) : 0u;
+      }
     }
     if constexpr (MODE == kModeP16) {
+      // source positions of an element's low bits, most significant first, after bits that are zero
+      // in every state (position 63)
       unsigned char* perm = smem + L.off_perm;
+      const int pad = L.nlow_pad - L.nlow;
+      for (int i = tid; i < G * pad; i += nt) perm[(i / pad) * L.perm_stride + i % pad] = 63;
       for (int i = tid; i < nb * G; i += nt) {
         const int b = i / G, g = i - b * G;
         const int to = __ffsll((long long)__ldg(p.group.onehot + i)) - 1;
-        if (to < L.nlow) perm[g * L.perm_stride + (L.nlow - 1 - to)] = (unsigned char)b;
+        if (to < L.nlow) perm[g * L.perm_stride + (L.nlow_pad - 1 - to)] = (unsigned char)b;
       }
     }
-    stage_u64((uint64_t*)(smem + L.off_sm), p.off.rows.sm, 32 * L.slot_blocks);
-    stage_u64((uint64_t*)(smem + L.off_sl1), p.off.rows.sl1, 32 * L.slot_blocks);
-    stage_u64((uint64_t*)(smem + L.off_sl2), p.off.rows.sl2, 32 * L.slot_blocks);
+    auto states = [&](uint32_t off, const uint64_t* src, int n) {
+      State* dst = (State*)(smem + off);
+      for (int i = tid; i < n; i += nt) dst[i] = (State)__ldg(src + i);
+    };
+    states(L.off_sm, p.off.rows.sm, 32 * L.slot_blocks);
+    states(L.off_sl1, p.off.rows.sl1, 32 * L.slot_blocks);
+    states(L.off_sl2, p.off.rows.sl2, 32 * L.slot_blocks);
     uint32_t* st = (uint32_t*)(smem + L.off_st);
     for (int i = tid; i < 32 * L.slot_blocks; i += nt) st[i] = __ldg(p.off.rows.st + i);
     uint32_t* ti = (uint32_t*)(smem + L.off_ti);
     for (int i = tid; i < L.T; i += nt) ti[i] = __ldg(p.off.rows.tinfo + i);
-    stage_u64((uint64_t*)(smem + L.off_ts), p.off.s, L.T);
-    stage_u64((uint64_t*)(smem + L.off_xm), p.off.rows.xmask, L.n_pat);
-    stage_u64((uint64_t*)(smem + L.off_dm), p.diag.rows.sm, 32 * L.n_diag_blocks);
-    stage_u64((uint64_t*)(smem + L.off_dr), p.diag.rows.sl1, 32 * L.n_diag_blocks);
-    stage_u64((uint64_t*)(smem + L.off_ds), p.diag.rows.sl2, 32 * L.n_diag_blocks);
+    states(L.off_ts, p.off.s, L.T);
+    states(L.off_xm, p.off.rows.xmask, L.n_pat);
+    states(L.off_dm, p.diag.rows.sm, 32 * L.n_diag_blocks);
+    states(L.off_dr, p.diag.rows.sl1, 32 * L.n_diag_blocks);
+    states(L.off_ds, p.diag.rows.sl2, 32 * L.n_diag_blocks);
     uint2* db = (uint2*)(smem + L.off_db);
     for (int i = tid; i < L.n_diag_blocks; i += nt)
       db[i] = make_uint2(__ldg(p.diag.rows.st + i), __ldg(p.diag.rows.tinfo + i));
     stage_d2((double2*)(smem + L.off_dv), p.diag.rows.cval, p.diag.rows.n_cls);
-    if constexpr (FERMI) stage_u64((uint64_t*)(smem + L.off_fs), p.group.fsign_packed, nb * 32 * p.group.gpl);
+    if constexpr (FERMI) states(L.off_fs, p.group.fsign_packed, nb * 32 * p.group.gpl);
+    __syncthreads();
+    // images of the flip patterns, from those of their sites
+    uint32_t* img = (uint32_t*)(smem + L.off_img);
+    const State* xm = (const State*)(smem + L.off_xm);
+    for (int i = tid; i < L.n_pat * L.words; i += nt) {
+      const int x = i / L.words, w = i - x * L.words;
+      uint32_t v = 0;
+      for (State m = xm[x]; m != 0; m &= m - 1) v ^= site[low_bit(m) * L.site_words + w];
+      img[x * L.stride + w] = v;
+    }
+  }
+
+  // (-1)^n of group element g on the occupied orbitals of `state`: the reversed pairs
+  // sum_k popcount(state & L_g[k]) over occupied k have the parity of state & XOR_k L_g[k].
+  __device__ __forceinline__ uint32_t fermion_sign(uint32_t g, State state) const {
+    const State* l = tab<State>(L.off_fs) + g;
+    const int stride = 32 * p.group.gpl;
+    State crossed = 0;
+    for (State m = state; m != 0; m &= m - 1) crossed ^= l[low_bit(m) * stride];
+    return (uint32_t)popc_state((State)(state & crossed));
   }
 
   // Forgets the images of earlier rows (before a block of rows that does not follow them).
@@ -174,102 +214,136 @@ struct RowGroup {
     prev_row = -1;
   }
 
-  // Steps 1 and 2 for the rows [row0, row0 + n).  Returns the number of listed elements.
-  __device__ __forceinline__ int load_rows(const DeviceIndex& ix, int64_t row0, int n) {
+  // Steps 1 and 2 for the rows [row0, row0 + n).
+  __device__ __forceinline__ void load_rows(const DeviceIndex& ix, int64_t row0, int n) {
     nr = n;
     __syncwarp();  // the previous group's readers are done
-    a_l = lane < nr ? __ldg(ix.reps + row0 + lane) : 0ull;
+    a_l = lane < nr ? (State)__ldg(ix.reps + row0 + lane) : (State)0;
     inv_l = lane < nr ? __ldg(ix.inv_norms + row0 + lane) : 0.0;
     cnt_l = 0;
     if (lane < nr) rows[lane] = a_l;
-    const uint32_t site_s = (uint32_t)__cvta_generic_to_shared(smem + L.off_site);
+    const uint32_t site_s = (uint32_t)__cvta_generic_to_shared(smem + L.off_site) + 4u * (uint32_t)lane;
+    const uint32_t row_bytes = 4u * (uint32_t)L.site_words;
     for (int r = 0; r < nr; ++r) {
-      const uint64_t a = shfl_u64(a_l, r);
-      const uint64_t diff = a ^ prev;
-      for (int w0 = lane; w0 < L.words; w0 += 96) {
-        // three words per lane at a time; site rows are padded to whole warps, image rows are not
-        const bool in1 = w0 + 32 < L.words, in2 = w0 + 64 < L.words;
-        uint32_t v0 = 0, v1 = 0, v2 = 0;
+      const State a = shfl_state(a_l, r);
+      const State diff = a ^ prev;
+      // four words per lane at a time; site rows are padded to whole warps, image rows are not
+      for (int w0 = 0; w0 < L.words; w0 += 128) {
+        const int left = L.words - w0;  // uniform
+        const int wl = w0 + lane;
+        uint32_t v[4] = {0, 0, 0, 0};
         if (prev_row >= 0) {
-          const uint32_t* g = ga + prev_row * L.stride + w0;
-          v0 = g[0];
-          v1 = in1 ? g[32] : 0u;
-          v2 = in2 ? g[64] : 0u;
+          const uint32_t* g = ga + prev_row * L.stride + wl;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v[k] = lane + 32 * k < left ? g[32 * k] : 0u;
         }
         const uint32_t base = site_s + 4u * (uint32_t)w0;
-        for (uint64_t d = diff; d != 0; d &= d - 1) {
-          const uint32_t s = base + (uint32_t)(__ffsll((long long)d) - 1) * (uint32_t)(4 * L.site_words);
-          v0 ^= lds_u32(s);
-          if (in1) v1 ^= lds_u32(s + 128);
-          if (in2) v2 ^= lds_u32(s + 256);
+        for (State d = diff; d != 0;) {
+          const uint32_t s0 = base + (uint32_t)low_bit(d) * row_bytes;
+          d &= d - 1;
+          const bool pair = d != 0;  // uniform
+          const uint32_t s1 = base + (pair ? (uint32_t)low_bit(d) : 0u) * row_bytes;
+          d &= pair ? d - 1 : (State)0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (32 * k < left) v[k] ^= lds_u32(s0 + 128 * k) ^ (pair ? lds_u32(s1 + 128 * k) : 0u);
         }
-        uint32_t* g = ga + r * L.stride + w0;
-        g[0] = v0;
-        if (in1) g[32] = v1;
-        if (in2) g[64] = v2;
+        uint32_t* g = ga + r * L.stride + wl;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (lane + 32 * k < left) g[32 * k] = v[k];
       }
       prev = a;
       prev_row = r;
     }
     // zero-norm rows take no part (their outputs are zero)
     const unsigned live = __ballot_sync(FULL, inv_l != 0.0);
-    int total = 0;
     const unsigned below = (1u << lane) - 1u;
+    total = 0;
     for (int b = 0; b < L.slot_blocks; ++b) {
-      const uint64_t m = tab<uint64_t>(L.off_sm)[32 * b + lane];
-      const uint64_t l1 = tab<uint64_t>(L.off_sl1)[32 * b + lane], l2 = tab<uint64_t>(L.off_sl2)[32 * b + lane];
+      const State m = tab<State>(L.off_sm)[32 * b + lane];
+      const State l1 = tab<State>(L.off_sl1)[32 * b + lane], l2 = tab<State>(L.off_sl2)[32 * b + lane];
       const uint32_t t12 = tab<uint32_t>(L.off_st)[32 * b + lane];
       for (int r = 0; r < nr; ++r) {
-        uint64_t x;
-        bool h1, h2;
-        if constexpr (MODE == kModeN32) {
-          const uint32_t v = __shfl_sync(FULL, (uint32_t)a_l, r) & (uint32_t)m;
-          h1 = v == (uint32_t)l1 && (l1 >> 32) == 0;
-          h2 = v == (uint32_t)l2 && (l2 >> 32) == 0;
-        } else {
-          x = shfl_u64(a_l, r) & m;
-          h1 = x == l1;
-          h2 = x == l2;
-        }
+        const State x = shfl_state(a_l, r) & m;
+        const bool h1 = x == l1, h2 = x == l2;
         const bool hit = (h1 || h2) && ((live >> r) & 1u);
         const unsigned hits = __ballot_sync(FULL, hit);
         const int before = __shfl_sync(FULL, cnt_l, r);
         if (hit) {
-          const int rank = __popc(hits & below);
-          const int at = r * L.cap + before + rank;
-          entries[at] = make_uint2((h1 ? t12 & 0xffffu : t12 >> 16) | ((uint32_t)r << 16), 0u);
-          order[total + rank] = (uint16_t)at;
+          const int rank = __popc(hits & below), at = r * L.cap + before + rank;
+          const uint32_t t = h1 ? t12 & 0xffffu : t12 >> 16;
+          if constexpr (KEEP) {
+            entries[at].x = t | ((uint32_t)r << 16);
+            list[total + rank] = (uint16_t)at;
+          } else {
+            list[at] = (uint16_t)t;
+          }
         }
-        const int c = __popc(hits);
-        if (lane == r) cnt_l += c;
-        total += c;
+        if (lane == r) cnt_l += __popc(hits);
+        if (KEEP) total += __popc(hits);
       }
     }
     __syncwarp();
-    return total;
   }
 
-  // The candidate minimum over the group for the element whose row images start at shared address
-  // gp and pattern images at ip.  beta is the generated state.  Returns the representative; *key
-  // is 2 * element + flipped.
-  __device__ __forceinline__ uint64_t scan(uint32_t gp, uint32_t ip, uint64_t beta, uint32_t* key) const {
-    if constexpr (MODE == kModeN32) {
-      const uint32_t flip = (uint32_t)p.group.flip;
-      uint32_t best = 0xffffffffu, at = 0;
-      for (int c = 0; c < L.words; c += 8) {
-        uint32_t mn = 0xffffffffu, mx = 0u;
+  // Pass 1 for E elements: images of their rows at gp (one row without KEEP), of their patterns at ip.  N32: the
+  // minimum and the word of its first chunk; P16: the minimal prefix and the mask of its chunks.
+  template <int E>
+  __device__ __forceinline__ void first_pass(const uint32_t (&gp)[E], const uint32_t (&ip)[E], uint32_t (&best)[E],
+                                             uint32_t (&at)[E]) const {
+    const uint32_t flip = (uint32_t)p.group.flip;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t h = lds_u32_volatile(gp + 4 * (c + k)) ^ lds_u32(ip + 4 * (c + k));
-          mn = min(mn, h);
-          if (INV) mx = max(mx, h);
+    for (int e = 0; e < E; ++e) {
+      best[e] = MODE == kModeN32 ? 0xffffffffu : 0x10000u;
+      at[e] = 0;
+    }
+    uint32_t bit = 1;
+    for (uint32_t c = 0; c < (uint32_t)L.words; c += 8, bit <<= 1) {
+      uint32_t a[8];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        if (KEEP || e == 0) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) a[k] = lds_u32_volatile(gp[e] + 4 * (c + k));
         }
-        const uint32_t m = INV ? min(mn, flip ^ mx) : mn;
-        if (m < best) {
-          best = m;
-          at = (uint32_t)c;
+        uint32_t h[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) h[k] = a[k] ^ lds_u32(ip[e] + 4 * (c + k));
+        if constexpr (MODE == kModeN32) {
+          uint32_t mn = h[0], mx = h[0];
+#pragma unroll
+          for (int k = 1; k < 8; ++k) {
+            mn = min(mn, h[k]);
+            if (INV) mx = max(mx, h[k]);
+          }
+          if (INV) mn = min(mn, flip ^ mx);
+          if (mn < best[e]) {
+            best[e] = mn;
+            at[e] = c;
+          }
+        } else {
+          uint32_t mn = h[0], mx = h[0];
+#pragma unroll
+          for (int k = 1; k < 8; ++k) {
+            mn = vmin2(mn, h[k]);
+            if (INV) mx = vmax2(mx, h[k]);
+          }
+          if (INV) mn = vmin2(mn, ~mx);
+          const uint32_t m = min(mn & 0xffffu, mn >> 16);
+          at[e] = m < best[e] ? bit : (m == best[e] ? at[e] | bit : at[e]);
+          best[e] = min(best[e], m);
         }
       }
+    }
+  }
+
+  // The representative of one element and its key 2 * group element + flipped, from pass 1.
+  __device__ __forceinline__ uint64_t second_pass(uint32_t gp, uint32_t ip, uint32_t best, uint32_t mask,
+                                                  uint64_t beta, uint32_t* key) const {
+    if constexpr (MODE == kModeN32) {
+      const uint32_t flip = (uint32_t)p.group.flip;
+      const uint32_t at = mask;
       uint32_t k0 = 0;
 #pragma unroll
       for (int k = 7; k >= 0; --k) {
@@ -280,58 +354,53 @@ struct RowGroup {
       *key = 2 * at + k0;
       return best;
     } else {
-      uint32_t best = 0x10000u, mask = 0, bit = 1;
-      for (int c = 0; c < L.words; c += 8, bit <<= 1) {
-        uint32_t mn = 0xffffffffu, mx = 0u;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t h = lds_u32_volatile(gp + 4 * (c + k)) ^ lds_u32(ip + 4 * (c + k));
-          mn = vmin2(mn, h);
-          if (INV) mx = vmax2(mx, h);
-        }
-        if (INV) mn = vmin2(mn, ~mx);
-        const uint32_t m = min(mn & 0xffffu, mn >> 16);
-        mask = m < best ? bit : (m == best ? mask | bit : mask);
-        best = min(best, m);
-      }
-      // the elements of the marked chunks that reach the prefix, compared by their low bits
-      const uint32_t two = best | (best << 16);
-      uint32_t found = 0;  // bit 4 k + 2 half + flipped of the chunk at `at`
+      // the elements of the marked chunks that reach the prefix, compared by their low bits (6x6
+      // torus: 1.08 elements per target reach it, the slowest of 32 lanes has 2.1)
+      const uint32_t two = best * 0x10001u;
+      uint32_t found = 0;  // words of the chunk at `at`: bit k its even element, bit 16 + k its odd one
       uint32_t at = 0, win = 0;
       uint64_t low = ~0ull;
-      const uint64_t low_ones = (1ull << L.nlow) - 1;
       const uint32_t perm_s = (uint32_t)__cvta_generic_to_shared(smem + L.off_perm);
       do {
         if (found == 0 && mask != 0) {
           at = (uint32_t)(__ffs(mask) - 1) * 8u;
           mask &= mask - 1;
+          uint32_t other = 0;  // halves that miss the prefix
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            const uint32_t d = lds_u32_volatile(gp + 4 * (at + k)) ^ lds_u32(ip + 4 * (at + k)) ^ two;
-            if ((d & 0xffffu) == 0u) found |= 1u << (4 * k);
-            if ((d >> 16) == 0u) found |= 4u << (4 * k);
-            if (INV) {
-              if ((d & 0xffffu) == 0xffffu) found |= 2u << (4 * k);
-              if ((d >> 16) == 0xffffu) found |= 8u << (4 * k);
-            }
+            uint32_t d = lds_u32_volatile(gp + 4 * (at + k)) ^ lds_u32(ip + 4 * (at + k)) ^ two;
+            if (INV) d = vmin2(d, ~d);
+            other += vmin2(d, 0x10001u) << k;
           }
+          found = ~other & 0xff00ffu;
         }
         if (found != 0) {
           const uint32_t f = (uint32_t)__ffs(found) - 1;
           found &= found - 1;
-          const uint32_t g = 2 * at + (f >> 1);
-          const uint32_t ps = perm_s + (g < (uint32_t)L.G ? g : 0u) * (uint32_t)L.perm_stride;
-          uint64_t v = 0;
-          for (int b = 0; b < L.nlow; b += 4) {
+          const uint32_t w = at + (f & 15u), half = f >> 4;
+          const uint32_t h = lds_u32_volatile(gp + 4 * w) ^ lds_u32(ip + 4 * w);
+          const bool flipped = INV && ((h >> (16 * half)) & 0xffffu) != best;
+          uint32_t g = 2 * w + half;
+          if (g >= (uint32_t)L.G) g = 0;  // padding repeats element 0
+          const uint32_t ps = perm_s + g * (uint32_t)L.perm_stride;
+          uint32_t hi = 0, lo = 0;  // the low bits, most significant first
+          int b = 0;
+          for (; b < L.nlow_pad - 32; b += 4) {
             const uint32_t src = lds_u32(ps + b);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (b + i < L.nlow) v = 2 * v + ((beta >> ((src >> (8 * i)) & 0xffu)) & 1ull);
+            for (int i = 0; i < 4; ++i) hi = 2 * hi + ((uint32_t)(beta >> __byte_perm(src, 0, 0x4440 + i)) & 1u);
           }
-          if (f & 1u) v ^= low_ones;
-          if (v < low) {
+          for (; b < L.nlow_pad; b += 4) {
+            const uint32_t src = lds_u32(ps + b);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) lo = 2 * lo + ((uint32_t)(beta >> __byte_perm(src, 0, 0x4440 + i)) & 1u);
+          }
+          uint64_t v = ((uint64_t)hi << 32) | lo;
+          if (flipped) v ^= (1ull << L.nlow) - 1;
+          const uint32_t mine = 2 * g + (flipped ? 1u : 0u);
+          if (v < low || (v == low && mine < win)) {
             low = v;
-            win = 2 * g + (f & 1u);
+            win = mine;
           }
         }
       } while (__any_sync(FULL, (found | mask) != 0));
@@ -340,37 +409,133 @@ struct RowGroup {
     }
   }
 
-  // Step 3 for the listed elements (total as returned by load_rows).
-  __device__ __forceinline__ void resolve(const DeviceIndex& ix, int total, int* __restrict__ err,
-                                          const uint64_t* __restrict__ binom) {
-    for (int w = 0; w < total; w += 32) {
-      const int at = order[min(w + lane, total - 1)];
-      const bool mine = w + lane < total;
-      const uint32_t e = entries[at].x;
-      const int t = (int)(e & 0xffffu), r = (int)(e >> 16);
-      const uint32_t info = tab<uint32_t>(L.off_ti)[t];
-      const uint32_t pat = info & 0xffffu;
-      const uint64_t beta = rows[r] ^ tab<uint64_t>(L.off_xm)[pat];
-      const uint32_t stride = 4u * (uint32_t)L.stride;
-      uint32_t key;
-      const uint64_t rep = scan(ga_s + (uint32_t)r * stride, img_s + pat * stride, beta, &key);
-      if (mine) {
-        bool ok = true;
-        if (info & kRowTermNeedsCheck) {
-          ok = constraint_ok(p.constraint, beta);
-          if (!ok) atomicOr(err, 1);
+  // Column indices of E representatives (kAbsent: not in the basis or !ok), the lookups side by side.
+  template <int E>
+  __device__ __forceinline__ void lookup(const DeviceIndex& ix, const uint64_t (&rep)[E], const bool (&ok)[E],
+                                         uint32_t (&j)[E], const uint64_t* __restrict__ binom) const {
+    if (ix.suffix16 != nullptr && !ix.identity && !ix.combinadic) {
+      uint32_t n[E];
+      uint32_t longest = 0;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const bool in = ok[e] && rep[e] <= ix.max_state;
+        const uint64_t b = in ? rep[e] >> ix.shift : 0ull;
+        j[e] = __ldg(ix.offsets + b);
+        n[e] = __ldg(ix.offsets + b + 1);
+        n[e] = in ? n[e] - j[e] : 0u;
+      }
+      const uint32_t low = (1u << ix.shift) - 1u;
+#pragma unroll
+      for (int e = 0; e < E; ++e) longest = max(longest, n[e]);
+      while (longest > 1) {
+        longest = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          if (n[e] > 1) {
+            const uint32_t half = n[e] >> 1;
+            if (__ldg(ix.suffix16 + (size_t)j[e] + half) <= ((uint32_t)rep[e] & low)) j[e] += half;
+            n[e] -= half;
+          }
+          longest = max(longest, n[e]);
         }
-        const int64_t j = ok ? mv_index_lookup(ix, rep, binom) : -1;
-        uint32_t g = key >> 1;
-        if (g >= (uint32_t)L.G) g = 0;  // padding repeats element 0
-        uint32_t neg = (uint32_t)__popcll(beta & tab<uint64_t>(L.off_ts)[t]) ^ (info >> 31);
-        if (INV && p.group.spin_inversion == -1) neg ^= key;
-        if constexpr (FERMI) neg ^= (uint32_t)fermion_parity(tab<uint64_t>(L.off_fs) + g, 32 * p.group.gpl, beta);
-        const uint32_t cls = (info >> 16) & 0xffu;
-        entries[at] = make_uint2(j >= 0 ? (uint32_t)j : kAbsent, (cls * (uint32_t)L.G + g) | (neg << 31));
+      }
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const bool there = n[e] != 0 && __ldg(ix.suffix16 + (size_t)(n[e] != 0 ? j[e] : 0u)) == ((uint32_t)rep[e] & low);
+        if (!there) j[e] = kAbsent;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int64_t i = ok[e] ? mv_index_lookup(ix, rep[e], binom) : -1;
+        j[e] = i >= 0 ? (uint32_t)i : kAbsent;
       }
     }
-    __syncwarp();
+  }
+
+  // Resolves E elements of this lane: terms term[e] of rows row[e] (one row without KEEP), where
+  // ok[e]; columns (kAbsent for elements outside the basis or !ok) and coefficient words in j and w.
+  template <int E>
+  __device__ __forceinline__ void resolve_some(const DeviceIndex& ix, const uint32_t (&row)[E],
+                                               const uint32_t (&term)[E], bool (&ok)[E], uint32_t (&j)[E],
+                                               uint32_t (&w)[E], int* __restrict__ err,
+                                               const uint64_t* __restrict__ binom) {
+    const uint32_t stride = 4u * (uint32_t)L.stride;
+    uint32_t gp[E], ip[E], best[E], at[E];
+    uint64_t rep[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      gp[e] = ga_s + row[e] * stride;
+      ip[e] = img_s + (tab<uint32_t>(L.off_ti)[term[e]] & 0xffffu) * stride;
+    }
+    first_pass<E>(gp, ip, best, at);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const uint32_t info = tab<uint32_t>(L.off_ti)[term[e]];
+      const State beta = rows[row[e]] ^ tab<State>(L.off_xm)[info & 0xffffu];
+      uint32_t key;
+      rep[e] = second_pass(gp[e], ip[e], best[e], at[e], beta, &key);
+      if (ok[e] && (info & kRowTermNeedsCheck) && !constraint_ok(p.constraint, beta)) {
+        ok[e] = false;
+        atomicOr(err, 1);
+      }
+      uint32_t g = key >> 1;
+      if (g >= (uint32_t)L.G) g = 0;  // padding repeats element 0
+      uint32_t neg = (uint32_t)popc_state((State)(beta & tab<State>(L.off_ts)[term[e]])) ^ (info >> 31);
+      if (INV && minus) neg ^= key;
+      if constexpr (FERMI) neg ^= fermion_sign(g, beta);
+      w[e] = (((info >> 16) & 0xffu) * (uint32_t)L.G + g) | (neg << 31);
+    }
+    lookup<E>(ix, rep, ok, j, binom);
+  }
+
+  // Step 3 without KEEP: take(columns, coefficient words) for the elements of this lane's row
+  // lane >> lane_shift.
+  template <typename Take>
+  __device__ __forceinline__ void resolve(const DeviceIndex& ix, int* __restrict__ err,
+                                          const uint64_t* __restrict__ binom, Take&& take) {
+    constexpr int E = kLaneElements<KEEP>;
+    const int r = lane >> L.lane_shift, sub = lane & (L.lanes_per_row - 1);
+    const int cnt = __shfl_sync(FULL, cnt_l, r);
+    const int most = (int)__reduce_max_sync(FULL, (unsigned)cnt);
+    for (int s = 0; s < most; s += E * L.lanes_per_row) {
+      uint32_t row[E], term[E], j[E], w[E];
+      bool ok[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int i = s + sub + e * L.lanes_per_row;
+        row[e] = (uint32_t)min(r, nr - 1);
+        ok[e] = i < cnt;
+        term[e] = ok[e] ? list[r * L.cap + i] : 0u;
+      }
+      resolve_some<E>(ix, row, term, ok, j, w, err, binom);
+      take(j, w);
+    }
+  }
+
+  // Step 3 with KEEP: the resolved elements replace the listed ones in entries.
+  __device__ __forceinline__ void resolve(const DeviceIndex& ix, int* __restrict__ err,
+                                          const uint64_t* __restrict__ binom) {
+    constexpr int E = kLaneElements<KEEP>;
+    for (int s = 0; s < total; s += 32 * E) {
+      uint32_t at[E], row[E], term[E], j[E], w[E];
+      bool ok[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int i = s + lane + 32 * e;
+        ok[e] = i < total;
+        at[e] = list[min(i, total - 1)];
+        const uint32_t v = entries[at[e]].x;
+        row[e] = v >> 16;
+        term[e] = v & 0xffffu;
+      }
+      __syncwarp();  // a clamped lane reads an element that its owner replaces
+      resolve_some<E>(ix, row, term, ok, j, w, err, binom);
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (ok[e] || s + lane + 32 * e < total) entries[at[e]] = make_uint2(j[e], w[e]);
+      __syncwarp();
+    }
   }
 
   // The diagonal elements: lane r < nr returns row r's.
@@ -378,20 +543,13 @@ struct RowGroup {
     double2 d = make_double2(0.0, 0.0);
     int n_l = 0;
     for (int b = 0; b < L.n_diag_blocks; ++b) {
-      const uint64_t m = tab<uint64_t>(L.off_dm)[32 * b + lane], k = tab<uint64_t>(L.off_dr)[32 * b + lane];
-      const uint64_t s = tab<uint64_t>(L.off_ds)[32 * b + lane];
+      const State m = tab<State>(L.off_dm)[32 * b + lane], k = tab<State>(L.off_dr)[32 * b + lane];
+      const State s = tab<State>(L.off_ds)[32 * b + lane];
       const uint2 info = tab<uint2>(L.off_db)[b];  // {signs of the 32 terms, class | last block of it << 31}
       for (int r = 0; r < nr; ++r) {
-        bool hit, odd;
-        if constexpr (MODE == kModeN32) {
-          const uint32_t a = __shfl_sync(FULL, (uint32_t)a_l, r);
-          hit = (a & (uint32_t)m) == (uint32_t)k && (k >> 32) == 0;
-          odd = __popc(a & (uint32_t)s) & 1;
-        } else {
-          const uint64_t a = shfl_u64(a_l, r);
-          hit = (a & m) == k;
-          odd = __popcll(a & s) & 1;
-        }
+        const State a = shfl_state(a_l, r);
+        const bool hit = (a & m) == k;
+        const bool odd = popc_state((State)(a & s)) & 1;
         const unsigned hits = __ballot_sync(FULL, hit);
         const unsigned minus = (__ballot_sync(FULL, odd) ^ info.x) & hits;
         if (lane == r) n_l += __popc(hits) - 2 * __popc(minus);
