@@ -969,8 +969,9 @@ struct DeviceTermSet {
 struct OperatorCache {
   TermTable off, diag;             // host copies (validated on every use)
   DeviceTermSet fwd_off, adj_off, fwd_diag, adj_diag;
-  std::vector<int32_t> coupling;   // optional, per term (off then diag)
-  int32_t* d_coupling = nullptr;
+  // forward terms with coupling ids (made by the first coupling product; ids per term, off then diag)
+  std::vector<int32_t> coupling;
+  DeviceTermSet cpl_off, cpl_diag;
 };
 
 std::unordered_map<const ls_hs_operator*, OperatorCache*> g_ops;
@@ -1026,26 +1027,31 @@ struct RowTables {
   std::vector<uint64_t> sm, sl1, sl2, xmask;
   std::vector<uint32_t> st, tinfo;
   std::vector<double> cval;  // interleaved
+  std::vector<uint32_t> coupling;  // per class
 };
 
-// The class of coefficient v (equal up to sign) in cval, appended when new; *neg: v = -class value.
-int coefficient_class(std::vector<double>* cval, double re, double im, bool* neg) {
-  const int n = (int)(cval->size() / 2);
+// The class of a term of coefficient v (equal up to sign) and coupling id, appended when new; *neg:
+// v = -class value.
+int coefficient_class(RowTables* R, double re, double im, int coupling, bool* neg) {
+  const int n = (int)R->coupling.size();
   for (int c = 0; c < n; ++c) {
-    const double a = (*cval)[2 * c], b = (*cval)[2 * c + 1];
+    const double a = R->cval[2 * c], b = R->cval[2 * c + 1];
+    if ((int)R->coupling[c] != coupling) continue;
     if (a == re && b == im) return *neg = false, c;
     if (a == -re && b == -im) return *neg = true, c;
   }
-  cval->push_back(re);
-  cval->push_back(im);
+  R->cval.push_back(re);
+  R->cval.push_back(im);
+  R->coupling.push_back((uint32_t)coupling);
   *neg = false;
   return n;
 }
 
 constexpr int kMaxRowClasses = 64;
 
-// Slots, patterns and classes of off-diagonal terms (matched through t.l).
-RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons) {
+// Slots, patterns and classes of off-diagonal terms (matched through t.l); coupling: an id per term,
+// or null (all 0).
+RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons, const int32_t* coupling) {
   RowTables R;
   if (t.n > 32767) return R;
   std::unordered_map<uint64_t, int> pattern;
@@ -1055,7 +1061,7 @@ RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons) {
     const auto it = pattern.emplace(t.x[k], (int)pattern.size());
     if (it.second) R.xmask.push_back(t.x[k]);
     bool neg = false;
-    const int cls = coefficient_class(&R.cval, t.v[2 * k], t.v[2 * k + 1], &neg);
+    const int cls = coefficient_class(&R, t.v[2 * k], t.v[2 * k + 1], coupling ? coupling[k] : 0, &neg);
     if (cls >= kMaxRowClasses) return R;
     R.tinfo[k] = (uint32_t)it.first->second | ((uint32_t)cls << 16) | (neg ? 1u << 31 : 0u) |
                  (term_breaks_constraint(cons, t.l[k], t.r[k]) ? kRowTermNeedsCheck : 0u);
@@ -1088,12 +1094,12 @@ RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons) {
 }
 
 // Blocks of 32 diagonal terms of one class each (matched through t.r).
-RowTables diag_rows(const TermTable& t) {
+RowTables diag_rows(const TermTable& t, const int32_t* coupling) {
   RowTables R;
   std::vector<std::vector<std::pair<int, bool>>> members;
   for (int k = 0; k < t.n; ++k) {
     bool neg = false;
-    const int cls = coefficient_class(&R.cval, t.v[2 * k], t.v[2 * k + 1], &neg);
+    const int cls = coefficient_class(&R, t.v[2 * k], t.v[2 * k + 1], coupling ? coupling[k] : 0, &neg);
     if (cls >= kMaxRowClasses) return R;
     if (cls >= (int)members.size()) members.resize(cls + 1);
     members[cls].push_back({k, neg});
@@ -1123,7 +1129,8 @@ RowTables diag_rows(const TermTable& t) {
 
 // Device layout: v (double2, 16-byte aligned) first, then m, l, r, x, s (uint64), xinfo (uint32),
 // then the row-group tables, each array on a 16-byte boundary.
-int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal, DeviceTermSet* out) {
+int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal, DeviceTermSet* out,
+                 const int32_t* coupling = nullptr) {
   std::vector<uint8_t> host;
   auto put = [&](const void* src, size_t sz) {
     const size_t at = (host.size() + 15) & ~(size_t)15;
@@ -1143,7 +1150,7 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal
     xinfo[k] = info;
     if (cnt != 2 || (info & kTermNeedsCheck)) all_two = 0;
   }
-  const RowTables R = diagonal ? diag_rows(t) : off_diag_rows(t, cons);
+  const RowTables R = diagonal ? diag_rows(t, coupling) : off_diag_rows(t, cons, coupling);
   const size_t n = (size_t)t.n;
   const size_t ov = put(t.v.data(), n * 16), om = put(t.m.data(), n * 8), ol = put(t.l.data(), n * 8);
   const size_t orr = put(t.r.data(), n * 8), ox = put(t.x.data(), n * 8), os = put(t.s.data(), n * 8);
@@ -1151,7 +1158,8 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal
   const size_t rsm = put(R.sm.data(), R.sm.size() * 8), rl1 = put(R.sl1.data(), R.sl1.size() * 8);
   const size_t rl2 = put(R.sl2.data(), R.sl2.size() * 8), rst = put(R.st.data(), R.st.size() * 4);
   const size_t rti = put(R.tinfo.data(), R.tinfo.size() * 4), rxm = put(R.xmask.data(), R.xmask.size() * 8);
-  const size_t rcv = put(R.cval.data(), R.cval.size() * 8);
+  const size_t rcv = put(R.cval.data(), R.cval.size() * 8), rcc = put(R.coupling.data(), R.coupling.size() * 4);
+  const size_t ocp = put(coupling, coupling ? n * 4 : 0);
   out->terms.all_two_site = all_two;
   if (!cuda_ok(cudaMalloc(&out->block, host.size()), "cudaMalloc(terms)")) return LS_GPU_ERR_CUDA;
   if (!cuda_ok(cudaMemcpy(out->block, host.data(), host.size(), cudaMemcpyHostToDevice), "upload terms"))
@@ -1174,13 +1182,14 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal
   r.tinfo = (const uint32_t*)(d + rti);
   r.xmask = (const uint64_t*)(d + rxm);
   r.cval = (const double2*)(d + rcv);
+  r.coupling = (const uint32_t*)(d + rcc);
+  out->terms.coupling = coupling ? (const int32_t*)(d + ocp) : nullptr;
   return 0;
 }
 
 void free_cache(OperatorCache* c) {
-  for (DeviceTermSet* s : {&c->fwd_off, &c->adj_off, &c->fwd_diag, &c->adj_diag})
+  for (DeviceTermSet* s : {&c->fwd_off, &c->adj_off, &c->fwd_diag, &c->adj_diag, &c->cpl_off, &c->cpl_diag})
     if (s->block) cudaFree(s->block);
-  if (c->d_coupling) cudaFree(c->d_coupling);
   delete c;
 }
 
@@ -1270,7 +1279,6 @@ int make_problem(ls_hs_operator const* op, bool adjoint, MatvecProblem* p) {
   p->constraint = basis_constraint(b);
   p->off = adjoint ? c->adj_off.terms : c->fwd_off.terms;
   p->diag = adjoint ? c->adj_diag.terms : c->fwd_diag.terms;
-  p->off.coupling = p->diag.coupling = c->d_coupling;
   p->n_rows = ix->n_states;
   // Real matrix elements: real term coefficients and real characters.  Characters are
   // cos/sin(-2 pi phi) in floating point (Group.hs:115-116), so sectors such as (pi, pi) carry
@@ -1671,20 +1679,20 @@ extern "C" int ls_gpu_coupling_inner_products(ls_hs_operator const* op, int n_co
   for (int t = 0; t < n_terms; ++t)
     if (term_coupling[t] < 0 || term_coupling[t] >= n_couplings)
       return fail(LS_GPU_ERR_INVALID, "term coupling id out of range");
-  if (c->d_coupling == nullptr || c->coupling.size() != (size_t)n_terms ||
-      memcmp(c->coupling.data(), term_coupling, (size_t)n_terms * 4) != 0) {
-    if (c->d_coupling) cudaFree(c->d_coupling);
-    c->d_coupling = nullptr;
-    c->coupling.assign(term_coupling, term_coupling + n_terms);
-    if (!cuda_ok(cudaMalloc((void**)&c->d_coupling, (size_t)std::max(n_terms, 1) * 4), "cudaMalloc(couplings)") ||
-        !cuda_ok(cudaMemcpy(c->d_coupling, c->coupling.data(), (size_t)n_terms * 4, cudaMemcpyHostToDevice),
-                 "upload couplings")) {
-      c->coupling.clear();
-      return LS_GPU_ERR_CUDA;
+  if (c->cpl_off.block == nullptr || c->cpl_diag.block == nullptr || c->coupling.size() != (size_t)n_terms ||
+      (n_terms > 0 && memcmp(c->coupling.data(), term_coupling, (size_t)n_terms * 4) != 0)) {
+    for (DeviceTermSet* s : {&c->cpl_off, &c->cpl_diag}) {
+      if (s->block) cudaFree(s->block);
+      s->block = nullptr;
     }
+    c->coupling.assign(term_coupling, term_coupling + n_terms);
+    const DeviceConstraint cons = basis_constraint(op->basis);
+    if (upload_terms(c->off, cons, false, &c->cpl_off, term_coupling) ||
+        upload_terms(c->diag, cons, true, &c->cpl_diag, term_coupling + c->off.n))
+      return LS_GPU_ERR_CUDA;
   }
-  p.off.coupling = c->d_coupling;
-  p.diag.coupling = c->d_coupling + c->off.n;
+  p.off = c->cpl_off.terms;
+  p.diag = c->cpl_diag.terms;
   return launch_coupling_products(p, n_couplings, d_g, d_x, d_out, device_error_word(), (cudaStream_t)stream);
 }
 

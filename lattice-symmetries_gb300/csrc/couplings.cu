@@ -8,7 +8,15 @@
 // the block partials by one more small kernel in a fixed order (deterministic).
 #include <type_traits>
 
+//
+// k_coupling_rows does the same on the row-group orbit scan (one lane per element, rowgroup.cuh),
+// wherever its tables fit: a lane keeps one sum per coupling over its row's elements, with
+// x_j n_j from a prescaled copy and coefficients from the (class, element) table, and multiplies by
+// conj(g_i) / n_i once per row.  28-site ladder, 1.43e6 rows, 3 couplings: 7.1 ms with one
+// warp per row (k_coupling_products), 2.3 ms with one lane per element; the scan and its
+// bookkeeping bound it.
 #include "matvec_launch.cuh"
+#include "rowsums.cuh"
 
 namespace lsg {
 
@@ -26,7 +34,8 @@ __global__ void __launch_bounds__(256, 2)
   const PackedTables T = stage_packed(p, L, smem, true);
   int32_t* cpl_off = (int32_t*)(smem + off_cpl);
   int32_t* cpl_diag = cpl_off + p.off.n;
-  for (int i = threadIdx.x; i < p.off.n + p.diag.n; i += blockDim.x) cpl_off[i] = p.off.coupling[i];
+  for (int i = threadIdx.x; i < p.off.n + p.diag.n; i += blockDim.x)
+    cpl_off[i] = i < p.off.n ? p.off.coupling[i] : p.diag.coupling[i - p.off.n];
   __syncthreads();
 
   const int lane = threadIdx.x & 31;
@@ -157,15 +166,147 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
+// out[c] = sum over the blocks' partials: a warp per coupling, lanes over the blocks, then a fixed
+// tree (deterministic).
 __global__ void k_sum_partials(const double2* __restrict__ partial, int n_blocks, int nc, double2* __restrict__ out) {
-  const int c = threadIdx.x;
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (c >= nc) return;
   double2 s = make_double2(0.0, 0.0);
-  for (int b = 0; b < n_blocks; ++b) {
-    s.x += partial[(size_t)b * nc + c].x;
-    s.y += partial[(size_t)b * nc + c].y;
+  for (int b = lane; b < n_blocks; b += 32) {
+    const double2 v = partial[(size_t)b * nc + c];
+    s.x += v.x;
+    s.y += v.y;
   }
-  out[c] = s;
+  s.x = warp_sum(s.x);
+  s.y = warp_sum(s.y);
+  if (lane == 0) out[c] = s;
+}
+
+constexpr int kCouplingThreads = 512;  // per-coupling sums in registers: up to 128 per thread
+
+template <int MODE, bool INV>
+__global__ void __launch_bounds__(kCouplingThreads, 1)
+    k_coupling_rows(const MatvecProblem p, const RowsLayout L, const RowsSums s, int nc, const double2* __restrict__ gv,
+                    double2* __restrict__ partial, int* __restrict__ err, const uint64_t* __restrict__ binom) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  using Group = RowGroup<MODE, INV, false, false>;
+  __shared__ uint8_t class_of_off[64], class_of_diag[64];  // coupling ids of the classes
+  if (threadIdx.x < 64) {
+    class_of_off[threadIdx.x] = threadIdx.x < p.off.rows.n_cls ? (uint8_t)p.off.rows.coupling[threadIdx.x] : 0;
+    class_of_diag[threadIdx.x] = threadIdx.x < p.diag.rows.n_cls ? (uint8_t)p.diag.rows.coupling[threadIdx.x] : 0;
+  }
+  Group::stage(L, p, smem);
+  double2* coef = reinterpret_cast<double2*>(smem + L.off_coef);
+  stage_coefficients<kColComplex>(L, p.off.rows, p.group.chars, coef);
+  __syncthreads();
+  Group g(L, p, smem);
+  const double2* __restrict__ xs = reinterpret_cast<const double2*>(s.xs);
+  const double2* __restrict__ x = reinterpret_cast<const double2*>(s.x);
+  const int lane = g.lane;
+  double2 tot[kMaxCouplings];
+#pragma unroll
+  for (int c = 0; c < kMaxCouplings; ++c) tot[c] = make_double2(0.0, 0.0);
+  const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t b = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; b < s.n_blocks; b += n_warps) {
+    const int64_t begin = b * s.rows_per_block, end = min(begin + s.rows_per_block, p.n_rows);
+    g.restart();
+    for (int64_t row0 = begin; row0 < end; row0 += L.R) {
+      g.load_rows(p.index, row0, (int)min((int64_t)L.R, end - row0));
+      double2 acc[kMaxCouplings];
+#pragma unroll
+      for (int c = 0; c < kMaxCouplings; ++c) acc[c] = make_double2(0.0, 0.0);
+      g.resolve(p.index, err, binom, [&](const auto& j, const auto& w, const auto& term) {
+        constexpr int E = sizeof(j) / sizeof(j[0]);
+        double2 xv[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) xv[e] = j[e] != Group::kAbsent ? __ldg(xs + j[e]) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const bool here = j[e] != Group::kAbsent;
+          const int cid = class_of_off[(g.template tab<uint32_t>(L.off_ti)[term[e]] >> 16) & 0xffu];
+          double2 v = make_double2(0.0, 0.0);
+          Column<kColComplex>::mac(v, flip_sign(coef[w[e] & 0x7fffffffu], w[e] & 0x80000000u), xv[e]);
+#pragma unroll
+          for (int c = 0; c < kMaxCouplings; ++c)
+            if (here && c == cid) acc[c] = add_v(acc[c], v);
+        }
+      });
+      // this lane's row: conj(g_i) / n_i times its sums
+      const int r = lane >> L.lane_shift;
+      const double inv = __shfl_sync(0xffffffffu, g.inv_l, r);
+      if (r < g.nr && inv != 0.0) {
+        const double2 gi = __ldg(gv + row0 + r);
+        const C2 wi{gi.x * inv, -gi.y * inv};
+#pragma unroll
+        for (int c = 0; c < kMaxCouplings; ++c) {
+          const C2 v = cmul(wi, C2{acc[c].x, acc[c].y});
+          tot[c] = add_v(tot[c], make_double2(v.re, v.im));
+        }
+      }
+      // the diagonal: lane r holds row r's counts
+      double2 d[kMaxCouplings];
+#pragma unroll
+      for (int c = 0; c < kMaxCouplings; ++c) d[c] = make_double2(0.0, 0.0);
+      g.diagonal_counts([&](uint32_t cls, int n) {
+        const double2 v = g.template tab<double2>(L.off_dv)[cls];
+        const int cid = class_of_diag[cls];
+#pragma unroll
+        for (int c = 0; c < kMaxCouplings; ++c)
+          if (c == cid) d[c] = make_double2(fma((double)n, v.x, d[c].x), fma((double)n, v.y, d[c].y));
+      });
+      if (lane < g.nr && g.inv_l != 0.0) {
+        const double2 gi = __ldg(gv + row0 + lane), xi = __ldg(x + row0 + lane);
+        const C2 gx = cmul_conj_b(C2{xi.x, xi.y}, C2{gi.x, gi.y});  // conj(g_i) x_i
+#pragma unroll
+        for (int c = 0; c < kMaxCouplings; ++c) {
+          const C2 v = cmul(C2{d[c].x, d[c].y}, gx);
+          tot[c] = add_v(tot[c], make_double2(v.re, v.im));
+        }
+      }
+    }
+  }
+  __shared__ double2 wsum[kCouplingThreads / 32][kMaxCouplings];
+  const int warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int c = 0; c < kMaxCouplings; ++c) {
+    const double re = warp_sum(tot[c].x), im = warp_sum(tot[c].y);
+    if (lane == 0) wsum[warp][c] = make_double2(re, im);
+  }
+  __syncthreads();
+  if (threadIdx.x < nc) {
+    double2 t = make_double2(0.0, 0.0);
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = add_v(t, wsum[w][threadIdx.x]);
+    partial[(size_t)blockIdx.x * nc + threadIdx.x] = t;
+  }
+}
+
+// Returns 1 when there is no memory for the prescaled copy of x or the tables do not fit (nothing launched).
+static int launch_coupling_rows(const MatvecProblem& p, int nc, const double* d_g, const double* d_x, double* d_out,
+                                int* d_err, const uint64_t* binom, cudaStream_t st) {
+  RowsLaunch q{};
+  if (!rows_plan(p, kColComplex, 1, p.n_rows, 0, &q, kCouplingThreads)) return 1;
+  double2* partial = (double2*)scratch((size_t)q.blocks * nc * sizeof(double2), 6);
+  if (partial == nullptr) return LS_GPU_ERR_CUDA;
+  double* d_xs = prescaled_copy(p, 2, 1, d_x, 1, 1, st);
+  if (d_xs == nullptr) return 1;
+  q.s.x = d_x;
+  q.s.xs = d_xs;
+  q.s.ldx = q.s.ldxs = 1;
+  auto go = [&](auto kern) -> int {
+    StageScope stage("couplings.kernel", st);
+    if (!ensure_smem_limit((const void*)kern, q.L.total)) return LS_GPU_ERR_CUDA;
+    kern<<<(unsigned)q.blocks, q.L.threads, q.L.total, st>>>(p, q.L, q.s, nc, reinterpret_cast<const double2*>(d_g),
+                                                             partial, d_err, binom);
+    if (!cuda_ok(cudaGetLastError(), "k_coupling_rows")) return LS_GPU_ERR_CUDA;
+    k_sum_partials<<<1, 32 * kMaxCouplings, 0, st>>>(partial, (int)q.blocks, nc, reinterpret_cast<double2*>(d_out));
+    return cuda_ok(cudaGetLastError(), "k_sum_partials") ? 0 : LS_GPU_ERR_CUDA;
+  };
+  const bool inv = p.group.spin_inversion != 0;
+  int rc;
+  if (q.mode == kModeN32) rc = inv ? go(k_coupling_rows<kModeN32, true>) : go(k_coupling_rows<kModeN32, false>);
+  else rc = inv ? go(k_coupling_rows<kModeP16, true>) : go(k_coupling_rows<kModeP16, false>);
+  cudaFreeAsync(d_xs, st);
+  return rc;
 }
 
 int launch_coupling_products(const MatvecProblem& p, int nc, const double* d_g, const double* d_x, double* d_out,
@@ -179,6 +320,10 @@ int launch_coupling_products(const MatvecProblem& p, int nc, const double* d_g, 
   if (p.off.coupling == nullptr) return fail(LS_GPU_ERR_INVALID, "operator terms carry no coupling ids");
   const uint64_t* binom = device_binomials();
   if (binom == nullptr) return LS_GPU_ERR_CUDA;
+  if (p.n_rows > 0 && p.index.norms != nullptr && rows_fit(p, 0)) {
+    const int rc = launch_coupling_rows(p, nc, d_g, d_x, d_out, d_err, binom, s);
+    if (rc != 1) return rc;
+  }
   const PackedLayout L = make_packed_layout(p, 0, 256);
   const size_t off_cpl = (L.total + 15) & ~(size_t)15;
   const size_t smem = off_cpl + (size_t)(p.off.n + p.diag.n) * 4;
@@ -191,7 +336,7 @@ int launch_coupling_products(const MatvecProblem& p, int nc, const double* d_g, 
     if (!ensure_smem_limit((const void*)kern, smem)) return LS_GPU_ERR_CUDA;
     kern<<<blocks, 256, smem, s>>>(p, L, off_cpl, nc, d_g, d_x, partial, d_err, binom);
     if (!cuda_ok(cudaGetLastError(), "k_coupling_products")) return LS_GPU_ERR_CUDA;
-    k_sum_partials<<<1, 32, 0, s>>>(partial, blocks, nc, reinterpret_cast<double2*>(d_out));
+    k_sum_partials<<<1, 32 * kMaxCouplings, 0, s>>>(partial, blocks, nc, reinterpret_cast<double2*>(d_out));
     return cuda_ok(cudaGetLastError(), "k_sum_partials") ? 0 : LS_GPU_ERR_CUDA;
   };
   const bool inv = p.group.spin_inversion != 0;

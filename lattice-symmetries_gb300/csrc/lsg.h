@@ -115,6 +115,7 @@ struct DeviceRowTerms {
   int n_pat = 0, n_cls = 0;
   const uint64_t* xmask = nullptr;  // [n_pat] flip masks
   const double2* cval = nullptr;    // [n_cls]
+  const uint32_t* coupling = nullptr;  // [n_cls] coupling id (terms of different couplings share no class)
 };
 constexpr uint32_t kRowTermNeedsCheck = 1u << 30;
 
@@ -127,7 +128,7 @@ struct DeviceTerms {
   const uint64_t* x = nullptr;
   const uint64_t* s = nullptr;
   const double2* v = nullptr;
-  const int32_t* coupling = nullptr;  // optional coupling id per term
+  const int32_t* coupling = nullptr;  // optional coupling id per term (tables of the coupling products)
   // Per term: bits 0-7 lowest flipped site, 8-15 highest flipped site, 16-23 number of flipped
   // sites, bit 24 set when the term can change a conserved particle number of the basis.
   const uint32_t* xinfo = nullptr;
@@ -260,6 +261,11 @@ struct MatvecProblem {
 bool rows_fit(const MatvecProblem& p, int n_sectors = 0);
 int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y, int64_t ldy,
                 int* d_err, const uint64_t* binom, cudaStream_t s);
+
+// A stream-ordered copy of x scaled by the orbit norms (k columns of `words` doubles per element, rows of
+// ldxs elements), to be freed with cudaFreeAsync; null without memory or on a launch error.
+double* prescaled_copy(const MatvecProblem& p, int words, int k, const double* d_x, int64_t ldx, int64_t ldxs,
+                       cudaStream_t s);
 
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,
                   double* d_y, int64_t ldy, int* d_err, cudaStream_t s);

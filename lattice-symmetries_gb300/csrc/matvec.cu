@@ -153,26 +153,34 @@ void rows_launch_config(int* max_threads, int* waves) {
   if (g_blocks_per_sm_override > 0) *waves = g_blocks_per_sm_override;
 }
 
+double* prescaled_copy(const MatvecProblem& p, int words, int k, const double* d_x, int64_t ldx, int64_t ldxs,
+                       cudaStream_t s) {
+  const int64_t elems = p.n_rows * ldxs * words;
+  double* d_xs = nullptr;
+  if (cudaMallocAsync((void**)&d_xs, (size_t)elems * sizeof(double), s) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  StageScope stage("matvec.prescale", s);
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((elems + 255) / 256, (int64_t)num_sms() * 16));
+  k_prescale<<<(unsigned)blocks, 256, 0, s>>>(d_x, ldx, p.index.norms, p.n_rows, k, words, d_xs, ldxs);
+  if (!cuda_ok(cudaGetLastError(), "k_prescale")) {
+    cudaFreeAsync(d_xs, s);
+    return nullptr;
+  }
+  return d_xs;
+}
+
 // y = H x by the row-group kernels, at most g_rhs_tile columns per launch.  Returns 1 when there
-// is no memory for the prescaled gather source (nothing has been launched).
+// is no memory for the prescaled gather source (no matvec kernel has been launched).
 static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y,
                               int64_t ldy, int* d_err, const uint64_t* binom, cudaStream_t s) {
   const int words = sc == Scalar::Complex ? 2 : 1;  // doubles per scalar
   MatvecProblem q = p;
   q.ldxs = words == 1 && k > 1 ? k + k % 2 : k;  // real columns are read in pairs
-  const int64_t elems = p.n_rows * q.ldxs * words;
-  double* d_xs = nullptr;
-  if (cudaMallocAsync((void**)&d_xs, (size_t)elems * sizeof(double), s) != cudaSuccess) {
-    cudaGetLastError();
-    return 1;
-  }
+  double* d_xs = prescaled_copy(p, words, k, d_x, ldx, q.ldxs, s);
+  if (d_xs == nullptr) return 1;
   int rc = 0;
-  {
-    StageScope stage("matvec.prescale", s);
-    const int64_t blocks = std::min<int64_t>((elems + 255) / 256, (int64_t)num_sms() * 16);
-    k_prescale<<<(unsigned)blocks, 256, 0, s>>>(d_x, ldx, p.index.norms, p.n_rows, k, words, d_xs, q.ldxs);
-    if (!cuda_ok(cudaGetLastError(), "k_prescale")) rc = LS_GPU_ERR_CUDA;
-  }
   for (int done = 0; rc == 0 && done < k; done += g_rhs_tile) {
     StageScope stage("matvec.kernel", s);
     const int chunk = std::min(k - done, g_rhs_tile);

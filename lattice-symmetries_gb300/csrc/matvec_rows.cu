@@ -37,6 +37,9 @@ __global__ void __launch_bounds__(kRowsThreads<KEEP>, 1)
   }
 }
 
+// Dynamic shared memory of a row-group kernel (the coupling products keep 1.2 KB more, statically).
+constexpr size_t kRowsSmem = kMaxDynamicSmem - 2048;
+
 // Layout for `warps` warps of R rows (keep: the resolved elements are kept in shared memory); false when it exceeds the shared memory of a CTA.
 static bool rows_layout(const MatvecProblem& p, int mode, bool complex_elements, bool keep, int n_sectors,
                         int warps, int R, RowsLayout* out) {
@@ -103,7 +106,7 @@ static bool rows_layout(const MatvecProblem& p, int mode, bool complex_elements,
   L.warp_bytes = o;
   L.total = L.off_warp + (uint32_t)warps * L.warp_bytes;
   *out = L;
-  return L.total <= kMaxDynamicSmem;
+  return L.total <= kRowsSmem;
 }
 
 // Modes that `p` can run in order of preference: N32 where the state fits 32 bits (whole states, no
@@ -136,7 +139,7 @@ static bool rows_shape(const MatvecProblem& p, bool complex_elements, bool keep,
     int warps[4];
     for (int i = 0; i < 4; ++i) {
       rows_layout(p, m, complex_elements, keep, n_sectors, 1, 8 >> i, &t[i]);
-      const int64_t room = (int64_t)kMaxDynamicSmem - t[i].off_warp;
+      const int64_t room = (int64_t)kRowsSmem - t[i].off_warp;
       warps[i] = t[i].warp_bytes == 0 || room < 0 ? 0 : (int)std::min<int64_t>(max_warps, room / t[i].warp_bytes);
     }
     for (const int enough : {24, 16, 8, kLeastWarps}) {
@@ -162,12 +165,14 @@ static bool rows_shape(const MatvecProblem& p, bool complex_elements, bool keep,
 
 void rows_launch_config(int* max_threads, int* waves);
 
-bool rows_plan(const MatvecProblem& p, int col, int k, int64_t n_rows, int n_sectors, RowsLaunch* out) {
+bool rows_plan(const MatvecProblem& p, int col, int k, int64_t n_rows, int n_sectors, RowsLaunch* out,
+               int most_threads) {
   const int units = col == kColPair && out->s.real_cols ? (k + 1) / 2 : k;  // columns of the lanes
   const bool keep = units > 1, complex_elements = n_sectors > 0 || col == kColComplex;
   // (the batched kernel holds the sector's description in registers, too)
   int max_threads = keep && n_sectors == 0 ? kRowsThreads<true> : kRowsThreads<false>, waves = 1;
-  rows_launch_config(&max_threads, &waves);
+  if (most_threads > 0) max_threads = most_threads;
+  else rows_launch_config(&max_threads, &waves);
   const int sms = num_sms();
   RowsLayout& L = out->L;
   if (!rows_shape(p, complex_elements, keep, n_rows, n_sectors, max_threads / 32, sms, &out->mode, &L)) return false;

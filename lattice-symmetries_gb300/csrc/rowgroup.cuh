@@ -489,7 +489,7 @@ struct RowGroup {
     lookup<E>(ix, rep, ok, j, binom);
   }
 
-  // Step 3 without KEEP: take(columns, coefficient words) for the elements of this lane's row
+  // Step 3 without KEEP: take(columns, coefficient words, terms) for the elements of this lane's row
   // lane >> lane_shift.
   template <typename Take>
   __device__ __forceinline__ void resolve(const DeviceIndex& ix, int* __restrict__ err,
@@ -509,7 +509,7 @@ struct RowGroup {
         term[e] = ok[e] ? list[r * L.cap + i] : 0u;
       }
       resolve_some<E>(ix, row, term, ok, j, w, err, binom);
-      take(j, w);
+      take(j, w, term);
     }
   }
 
@@ -538,9 +538,10 @@ struct RowGroup {
     }
   }
 
-  // The diagonal elements: lane r < nr returns row r's.
-  __device__ __forceinline__ double2 diagonal() const {
-    double2 d = make_double2(0.0, 0.0);
+  // Signed counts of the diagonal terms, class by class: each(class, count) with lane r < nr holding
+  // row r's count.
+  template <typename Each>
+  __device__ __forceinline__ void diagonal_counts(Each&& each) const {
     int n_l = 0;
     for (int b = 0; b < L.n_diag_blocks; ++b) {
       const State m = tab<State>(L.off_dm)[32 * b + lane], k = tab<State>(L.off_dr)[32 * b + lane];
@@ -551,16 +552,24 @@ struct RowGroup {
         const bool hit = (a & m) == k;
         const bool odd = popc_state((State)(a & s)) & 1;
         const unsigned hits = __ballot_sync(FULL, hit);
-        const unsigned minus = (__ballot_sync(FULL, odd) ^ info.x) & hits;
-        if (lane == r) n_l += __popc(hits) - 2 * __popc(minus);
+        const unsigned minus_hits = (__ballot_sync(FULL, odd) ^ info.x) & hits;
+        if (lane == r) n_l += __popc(hits) - 2 * __popc(minus_hits);
       }
       if (info.y >> 31) {
-        const double2 v = tab<double2>(L.off_dv)[info.y & 0xffffu];
-        d.x = fma((double)n_l, v.x, d.x);
-        d.y = fma((double)n_l, v.y, d.y);
+        each(info.y & 0xffffu, n_l);
         n_l = 0;
       }
     }
+  }
+
+  // The diagonal elements: lane r < nr returns row r's.
+  __device__ __forceinline__ double2 diagonal() const {
+    double2 d = make_double2(0.0, 0.0);
+    diagonal_counts([&](uint32_t cls, int n) {
+      const double2 v = tab<double2>(L.off_dv)[cls];
+      d.x = fma((double)n, v.x, d.x);
+      d.y = fma((double)n, v.y, d.y);
+    });
     return d;
   }
 };

@@ -115,7 +115,7 @@ __device__ __forceinline__ void resolve_and_sum(Group& g, const RowsSums& s, con
   const V* __restrict__ xs = reinterpret_cast<const V*>(s.xs);
   const int64_t ldv = COL == kColPair && s.real_cols ? s.ldxs / 2 : s.ldxs;
   V acc = Col::zero();
-  g.resolve(ix, err, binom, [&](const auto& j, const auto& w) {
+  g.resolve(ix, err, binom, [&](const auto& j, const auto& w, const auto&) {
     constexpr int E = sizeof(j) / sizeof(j[0]);
     V xv[E];
 #pragma unroll
@@ -202,6 +202,8 @@ struct RowsLaunch {
 };
 // Picks shape and layout for k columns over n_rows rows (n_sectors > 0: the batched kernel's
 // tables); false when the tables do not fit.
-bool rows_plan(const MatvecProblem& p, int col, int k, int64_t n_rows, int n_sectors, RowsLaunch* out);
+// max_threads 0: the matvec kernels' own.
+bool rows_plan(const MatvecProblem& p, int col, int k, int64_t n_rows, int n_sectors, RowsLaunch* out,
+               int max_threads = 0);
 
 }  // namespace lsg
