@@ -470,9 +470,14 @@ extern "C" void ls_hs_is_representative_halide_kernel(ptrdiff_t batch_size, uint
 // State index (indexing.c:94-125, :273-325)
 // =================================================================================================
 namespace {
-// Device copies of representatives produced by the GPU enumeration, keyed by the host array they
-// were copied to, so that building the index does not upload them again.
-std::unordered_map<const void*, uint64_t*> g_pending_device_reps;
+// Device copies of representatives (and their orbit norms) produced by the GPU enumeration, keyed by
+// the host array they were copied to, so that building the index does not upload them again.
+struct PendingStates {
+  uint64_t* reps;
+  double* norms;  // norms | inverse norms (projected bases), or null
+  const OrbitData* norms_for;
+};
+std::unordered_map<const void*, PendingStates> g_pending_device_reps;
 }
 
 struct ls_hs_state_index_binary_search_data : IndexData {};
@@ -492,7 +497,13 @@ extern "C" ls_hs_state_index_binary_search_data* ls_hs_create_state_index_binary
   cudaStream_t s = default_stream();
   auto it = g_pending_device_reps.find(representatives->elts);
   if (it != g_pending_device_reps.end()) {
-    ix->d_reps = it->second;
+    ix->d_reps = it->second.reps;
+    ix->d_norms = it->second.norms;
+    if (ix->d_norms != nullptr) {
+      ix->norms_for = it->second.norms_for;
+      ix->dev.norms = ix->d_norms;
+      ix->dev.inv_norms = ix->d_norms + std::max<int64_t>(ix->n_states, 1);
+    }
     g_pending_device_reps.erase(it);
   } else {
     if (!cuda_ok(cudaMalloc((void**)&ix->d_reps, std::max<int64_t>(ix->n_states, 1) * 8), "cudaMalloc(reps)") ||
@@ -512,6 +523,7 @@ extern "C" ls_hs_state_index_binary_search_data* ls_hs_create_state_index_binary
       !cuda_ok(cudaStreamSynchronize(s), "build index")) {
     report("ls_hs_create_state_index_binary_search_kernel_data");
     cudaFree(ix->d_reps);
+    cudaFree(ix->d_norms);
     delete ix;
     return nullptr;
   }
@@ -703,7 +715,7 @@ extern "C" int ls_gpu_set_enumeration_rule(int exact) {
   return previous;
 }
 
-static int enumerate_into(ls_hs_basis const* b, uint64_t** d_out, int64_t* count) {
+static int enumerate_into(ls_hs_basis const* b, uint64_t** d_out, double** d_norms, int64_t* count) {
   EnumerateRequest req{};
   uint64_t lo, hi;
   state_estimates(b, &lo, &hi);
@@ -737,7 +749,7 @@ static int enumerate_into(ls_hs_basis const* b, uint64_t** d_out, int64_t* count
     req.spin_inversion = 0;
   }
   if (req.mode == 1 && b->particle_type == LS_HS_SPINFUL_FERMION) req.number_sites = 2 * b->number_sites;
-  return enumerate_states(g, req, d_out, count, default_stream());
+  return enumerate_states(g, req, d_out, d_norms, count, default_stream());
 }
 
 // Allocation-free enumeration for callers that cannot allocate device memory; see
@@ -793,9 +805,10 @@ extern "C" void ls_chpl_enumerate_representatives(ls_hs_basis* p, uint64_t lower
     return;
   }
   uint64_t* d = nullptr;
+  double* norms = nullptr;
   int64_t n = 0;
   cudaStream_t s = default_stream();
-  if (enumerate_into(p, &d, &n) != 0) {
+  if (enumerate_into(p, &d, &norms, &n) != 0) {
     report("ls_chpl_enumerate_representatives");
     return;
   }
@@ -804,10 +817,11 @@ extern "C" void ls_chpl_enumerate_representatives(ls_hs_basis* p, uint64_t lower
       (n > 0 && !cuda_ok(cudaMemcpyAsync(h, d, (size_t)n * 8, cudaMemcpyDeviceToHost, s), "D2H reps")) ||
       !cuda_ok(cudaStreamSynchronize(s), "enumerate")) {
     cudaFree(d);
+    cudaFree(norms);
     report("ls_chpl_enumerate_representatives");
     return;
   }
-  g_pending_device_reps[h] = d;
+  g_pending_device_reps[h] = PendingStates{d, norms, basis_orbit(p)};
   dest->elts = h;
   dest->num_elts = (uint64_t)n;
   dest->freer = (void*)&free_pinned;

@@ -14,9 +14,10 @@
 //    and early exit (generator.cpp:181-253), so flags and norms are bit-identical to the
 //    reference built with lane width W.
 //  * enumeration: candidates in increasing order (combinadics unrank + Gosper steps,
-//    StatesEnumeration.chpl:29-32), one tile of blockDim*K candidates per block, flags kept
-//    as per-thread bit masks, block scan, a run per tile in an append buffer, an exclusive
-//    scan over tile counts, and a final ordered gather; the output is sorted.
+//    StatesEnumeration.chpl:29-32) in tiles; tiles whose common top bits already have a smaller
+//    image are dropped whole, the others tested against the group elements that those bits leave
+//    open; a run per tile in an append buffer, an exclusive scan over tile counts, and a final
+//    ordered gather; the output is sorted.
 //  * state index: the prefix-bucket table of kernels/indexing.c:45-117 built on the GPU and
 //    a branch-free window search (indexing.c:196-215).
 #include <algorithm>
@@ -103,18 +104,22 @@ __device__ inline uint64_t d_binom(int n, int k) {
 
 // Unrank with a downward scan: the bit positions decrease with i, so the total work is
 // O(n_bits + h) instead of O(n_bits * h).
-__device__ inline uint64_t d_unrank(int64_t index, int h, int n_bits) {
+template <typename Binomial>
+__device__ __forceinline__ uint64_t d_unrank(int64_t index, int h, int n_bits, Binomial&& binomial) {
   uint64_t state = 0;
   int c = n_bits - 1;
   for (int i = h; i > 0; --i) {
-    while (c >= i && (int64_t)d_binom(c, i) > index) --c;
+    while (c >= i && (int64_t)binomial(c, i) > index) --c;
     if (c < i - 1) c = i - 1;
-    uint64_t contribution = d_binom(c, i);
+    uint64_t contribution = binomial(c, i);
     state |= (uint64_t)1 << c;
     index -= (int64_t)contribution;
     --c;
   }
   return state;
+}
+__device__ inline uint64_t d_unrank(int64_t index, int h, int n_bits) {
+  return d_unrank(index, h, n_bits, [](int n, int k) { return d_binom(n, k); });
 }
 
 __device__ inline int64_t d_rank(uint64_t a) {
@@ -697,6 +702,7 @@ struct EnumArgs {
   int32_t* tile_count;
   int64_t* tile_start;
   uint64_t* append;
+  uint16_t* append_stab;  // stabiliser sizes (0: a non-trivial character); at most 2 * kMaxGroupElements
   int64_t capacity;
   unsigned long long* counter;
   // Spinful fermions (mode 3): candidate (iB, iA) = (idx / nA, idx % nA) is
@@ -707,12 +713,16 @@ struct EnumArgs {
   uint64_t minA, maxA;
 };
 
-__device__ inline uint64_t candidate_at(const EnumArgs& a, int64_t idx) {
+template <typename Binomial>
+__device__ __forceinline__ uint64_t candidate_at(const EnumArgs& a, int64_t idx, Binomial&& binomial) {
   if (a.spinful) {
     const int64_t iB = idx / a.nA, iA = idx - iB * a.nA;
-    return (d_unrank(a.rankB + iB, a.hB, a.ns) << a.ns) | d_unrank(a.rankA + iA, a.hA, a.ns);
+    return (d_unrank(a.rankB + iB, a.hB, a.ns, binomial) << a.ns) | d_unrank(a.rankA + iA, a.hA, a.ns, binomial);
   }
-  return a.h >= 0 ? d_unrank(a.first_rank + idx, a.h, a.n_bits) : (uint64_t)(a.first_rank + idx);
+  return a.h >= 0 ? d_unrank(a.first_rank + idx, a.h, a.n_bits, binomial) : (uint64_t)(a.first_rank + idx);
+}
+__device__ inline uint64_t candidate_at(const EnumArgs& a, int64_t idx) {
+  return candidate_at(a, idx, [](int n, int k) { return d_binom(n, k); });
 }
 // Successor of candidate v (only called while another candidate follows in the range).
 __device__ inline uint64_t candidate_next(const EnumArgs& a, uint64_t v) {
@@ -729,7 +739,7 @@ __device__ inline uint64_t candidate_next(const EnumArgs& a, uint64_t v) {
 // (mode 0), or the (N_up, N_down) product range of spinful fermions (mode 3).
 static void projected_candidates(const EnumerateRequest& req, int n_bits, EnumArgs* a) {
   a->n_bits = n_bits;
-  a->lane_width = 4;
+  a->lane_width = 4;  // kEnumLanes below
   a->reference_rule = req.reference_norm_rule;
   if (req.mode == 3) {
     const int ns = req.number_sites;
@@ -762,78 +772,360 @@ static void projected_candidates(const EnumerateRequest& req, int n_bits, EnumAr
   a->n_tiles = (a->n_candidates + kEnumTile - 1) / kEnumTile;
 }
 
-template <int DEPTH>
-__global__ void __launch_bounds__(kEnumThreads) k_enumerate_projected(DeviceGroup g, EnumArgs a) {
-  __shared__ int64_t warp_sums[32];
-  __shared__ int64_t total;
-  __shared__ unsigned long long base_slot;
-  for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
-    const int64_t first = tile * kEnumTile + (int64_t)threadIdx.x * kEnumPerThread;
-    uint32_t bits = 0;
-    int cnt = 0;
-    if (first < a.n_candidates) {
-      uint64_t v = candidate_at(a, first);
-      const int todo = (int)min((int64_t)kEnumPerThread, a.n_candidates - first);
-      for (int k = 0; k < todo; ++k) {
-        IsRepResult r = is_rep<DEPTH>(g, v, a.lane_width, true);
-        bool keep;
-        if (!r.ok) {
-          keep = false;
-        } else if (a.reference_rule) {
-          keep = r.sum > 0;
-        } else {
-          keep = r.trivial && r.exact_count > 0;
+// ------------------------------------------------------------------------------------------------
+// Projected enumeration by pruned blocks.
+//
+// The candidates of a block of consecutive ranks share their top bits: with F and L its first and
+// last state, every bit above the highest bit of F ^ L.  A group element whose image is decided by
+// those bits in some top part is compared with the block's states there once: smaller, and no
+// state of the block is a representative; larger, and the element needs no look at any of them.
+// Representatives crowd at small values, so most blocks die on that test (6x6 torus, 576 images:
+// 95 % of the blocks of 65536 candidates, 98 % of those of 4096) and the survivors are tested
+// against the undecided elements only.
+//
+// A CTA takes work items of `super` tiles of `tile` candidates from a counter (the surviving tiles
+// sit next to each other at small ranks), tests the item, then each tile: one thread per group
+// element, images from the one-hot table.  In a surviving tile the warps take runs of 32 candidates,
+// a run being tested as a block of its own once more: lanes on 32 undecided elements at a time, the
+// run's common bits first, then its remaining candidates one by one by the few bits that differ
+// within the run, each to its first smaller image.
+//
+// The stabiliser sum of a survivor is added in the reference's order (chunks of lane_width
+// elements, is_rep below): elements outside the stabiliser add 0.0 there, so only the members are
+// visited, in ascending order.
+//
+// The size of a survivor's stabiliser is its orbit norm, so the norms come with the states.
+//
+// Measured (GB300, 6x6 torus, (pi, pi), 4.5e9 candidates): a thread per candidate with a Benes
+// network per group element, bound by the slowest lane of each warp, 537 ms, and 22 ms for the
+// norms afterwards; pruned blocks 44 ms with the norms.  What is left is integer issue in the
+// runs (106e6 candidates reach them, 15.7e6 are kept) and the barriers between tiles.
+// ------------------------------------------------------------------------------------------------
+constexpr int kPruneThreads = 1024;
+constexpr int kPruneWarps = kPruneThreads / 32;
+constexpr int kEnumLanes = 4;      // lane width of the reference's is_representative
+constexpr int kPruneTile = 4096;   // most candidates per tile
+constexpr int kPruneSuper = 16;    // tiles per work item of large ranges
+
+struct PruneArgs {
+  int tile, super;
+  int64_t n_items;
+  unsigned long long* next;  // work counter
+  int binomials_at;          // shared-memory offset of the binomial table
+};
+
+// TABLE: the one-hot table is in shared memory (else read from global memory).
+template <bool TABLE>
+__global__ void __launch_bounds__(kPruneThreads, 1) k_enumerate_pruned(DeviceGroup g, EnumArgs a, PruneArgs q) {
+  extern __shared__ __align__(16) unsigned char prune_smem[];
+  const int G = g.n_elems, n = a.n_bits;
+  const uint64_t full = n >= 64 ? ~0ull : (1ull << n) - 1;
+  const bool inv = g.spin_inversion != 0;
+  uint64_t* kept = (uint64_t*)prune_smem;                        // [tile]
+  uint64_t* uy = kept + q.tile;                                  // undecided elements: image of the known bits
+  uint64_t* uk = uy + G;                                         // ... image of the known mask
+  uint64_t* buffers = uk + G;                                    // per warp: 64 undecided elements of a run
+  uint64_t* table = buffers + kPruneWarps * 64;                  // TABLE: one-hot images [n][G]
+  uint32_t* ue = (uint32_t*)(table + (TABLE ? (size_t)n * G : 0));  // ... element | plain << 30 | flipped << 31
+  uint32_t* buffers_e = ue + G;
+  uint16_t* kept_stab = (uint16_t*)(buffers_e + kPruneWarps * 64);  // [tile]
+  // binomials for the lanes' own ranks (divergent reads of constant memory are serialised)
+  const int weights = 1 + (a.spinful ? max(a.hA, a.hB) : max(a.h, 0)), lengths = a.spinful ? a.ns : n;
+  uint64_t* binomials = (uint64_t*)(prune_smem + q.binomials_at);
+  for (int i = threadIdx.x; i < lengths * weights; i += blockDim.x) binomials[i] = c_binom[i / weights][i % weights];
+  uint64_t* by = buffers + (threadIdx.x >> 5) * 64;
+  uint32_t* be = buffers_e + (threadIdx.x >> 5) * 64;
+  __shared__ uint64_t ends[2];
+  __shared__ int counts[(kMaxGroupElements + 31) / 32];
+  __shared__ uint32_t flags[kPruneTile / 32];  // kept candidates of the tile
+  __shared__ int next_run;
+  __shared__ unsigned long long item_s, base_s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr unsigned FULL = 0xffffffffu;
+  if (TABLE)
+    for (int i = tid; i < n * G; i += kPruneThreads) table[i] = __ldg(g.onehot + i);
+  const uint32_t table_s = (uint32_t)__cvta_generic_to_shared(table), row_bytes = 8u * (uint32_t)G;
+  auto image = [&](int b, int e) -> uint64_t {
+    if constexpr (TABLE) {
+      uint64_t v;
+      asm("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(table_s + (uint32_t)b * row_bytes + 8u * (uint32_t)e));
+      return v;
+    } else {
+      return __ldg(g.onehot + (size_t)b * G + e);
+    }
+  };
+  // How the images of an element compare with the states of a block, from the known bits of the
+  // states (F, known) and of the image (y, ky): bit 0 undecided, bit 1 smaller; bits 2 and 3 for
+  // the flipped image.
+  auto compare = [&](uint64_t F, uint64_t known, uint64_t y, uint64_t ky) -> uint32_t {
+    const uint64_t open = ~(known & ky) & full;  // positions not known on both sides
+    const int sh = open == 0 ? 0 : 64 - __clzll((long long)open);
+    const uint64_t as = sh >= 64 ? 0ull : F >> sh, ys = sh >= 64 ? 0ull : y >> sh;
+    uint32_t r = (ys == as ? 1u : 0u) | (ys < as ? 2u : 0u);
+    if (inv) {
+      const uint64_t fs = sh >= 64 ? 0ull : (~y & full) >> sh;
+      r |= (fs == as ? 4u : 0u) | (fs < as ? 8u : 0u);
+    }
+    return r;
+  };
+  uint64_t known = 0;  // the known bits of the block tested last
+
+  // Tests candidates [first, first + count): the number of undecided elements, -1 when an image is
+  // smaller for all of them.
+  auto prune = [&](int64_t first, int64_t count) -> int {
+    __syncthreads();  // the previous block's readers of uy / ue are done
+    if (tid == 0) ends[0] = candidate_at(a, first);
+    if (tid == 32) ends[1] = candidate_at(a, first + count - 1);
+    __syncthreads();
+    const uint64_t F = ends[0], d = F ^ ends[1];
+    const int low = d == 0 ? 0 : 64 - __clzll((long long)d);
+    known = low >= 64 ? 0ull : (full >> low) << low;
+    bool killed = false;
+    for (int e0 = 0; e0 < G; e0 += kPruneThreads) {
+      const int e = e0 + tid;
+      uint64_t y = 0, ky = 0;
+      uint32_t r = 0;
+      if (e < G) {
+        for (int b = low; b < n; ++b) {
+          const uint64_t img = image(b, e);
+          ky |= img;
+          if ((F >> b) & 1ull) y |= img;
         }
-        if (keep) {
-          bits |= 1u << k;
-          ++cnt;
-        }
-        if (k + 1 < todo) v = candidate_next(a, v);
+        r = compare(F, known, y, ky);
+        killed = killed || (r & 10u) != 0;
+      }
+      const bool plain = (r & 1u) != 0, flipped = (r & 4u) != 0;
+      const unsigned m = __ballot_sync(FULL, plain || flipped);
+      if (lane == 0 && e < G) counts[e >> 5] = __popc(m);
+      __syncthreads();
+      if (plain || flipped) {
+        int at = __popc(m & ((1u << lane) - 1u));
+        for (int c = 0; c < (e >> 5); ++c) at += counts[c];
+        uy[at] = y;
+        uk[at] = ky;
+        ue[at] = (uint32_t)e | (plain ? 1u << 30 : 0u) | (flipped ? 1u << 31 : 0u);
       }
     }
-    const int64_t excl = block_exclusive_scan((int64_t)cnt, warp_sums, &total);
-    if (threadIdx.x == 0) {
-      unsigned long long b = 0;
-      if (total > 0) b = atomicAdd(a.counter, (unsigned long long)total);
-      base_slot = b;
-      a.tile_count[tile] = (int32_t)total;
-      a.tile_start[tile] = (int64_t)b;
-    }
-    __syncthreads();
-    if (cnt > 0) {
-      int64_t pos = (int64_t)base_slot + excl;
-      uint64_t v = candidate_at(a, first);
-      for (int k = 0; bits != 0; ++k) {
-        if (bits & 1u) {
-          if (pos < a.capacity) a.append[pos] = v;
-          ++pos;
+    if (__syncthreads_or(killed)) return -1;
+    int u = 0;
+    for (int c = 0; c < (G + 31) / 32; ++c) u += counts[c];
+    return u;
+  };
+
+  // Which of the `todo` <= 32 consecutive candidates, lane i's in v, are kept (bits); u undecided
+  // elements of the block tested last.  *stabiliser: the size of candidate i's stabiliser, 0 where it
+  // has a non-trivial character.
+  auto kept_of = [&](uint64_t v, int todo, int u, int* stabiliser) -> uint32_t {
+    // the run as a block of its own: more bits are known
+    const uint64_t F = __shfl_sync(FULL, (unsigned long long)v, 0);
+    const uint64_t d = F ^ __shfl_sync(FULL, (unsigned long long)v, todo - 1);
+    const int low = d == 0 ? 0 : 64 - __clzll((long long)d);
+    const uint64_t run_known = low >= 64 ? 0ull : (full >> low) << low;
+    uint32_t alive = todo >= 32 ? ~0u : (1u << todo) - 1u;
+    // lane i: the stabiliser sum of candidate i so far, in the reference's order
+    double sum = 0.0, chunk_sum = 0.0;
+    int chunk = -1, members = 0;
+    bool trivial = true;
+    uint32_t noted = 0;  // the first member, while any_noted
+    bool any_noted = false, summed = false;
+    const int n_chunks = G / kEnumLanes;
+    auto add_member = [&](uint32_t member, uint64_t state) {
+      const int es = (int)(member & 0x3fffffffu);
+      const bool ps = (member >> 30) & 1u, fs = member >> 31;
+      const double cre = __ldg(&g.chars[es].x);
+      double s;
+      if (!inv) {
+        s = (g.fermionic && fermion_parity(g.fsign + (size_t)es * n, 1, state)) ? -cre : cre;
+        ++members;
+        if (s != 1.0) trivial = false;
+      } else {
+        s = (g.spin_inversion == 1 ? (double)ps + (double)fs : (double)ps - (double)fs) * cre;
+        members += (int)ps + (int)fs;
+        if (ps && cre != 1.0) trivial = false;
+        if (fs && (double)g.spin_inversion * cre != 1.0) trivial = false;
+      }
+      const int c = es / kEnumLanes;
+      if (c >= n_chunks) {  // the tail is added element by element
+        sum += chunk_sum;
+        chunk_sum = 0.0;
+        sum += s;
+      } else {
+        if (c != chunk) {
+          sum += chunk_sum;
+          chunk_sum = 0.0;
+          chunk = c;
         }
-        bits >>= 1;
-        if (bits) v = candidate_next(a, v);
+        chunk_sum += s;
+      }
+    };
+    // the alive candidates against the first `count` <= 32 elements of the warp's buffer
+    auto test = [&](int count) {
+      const uint32_t w = lane < count ? be[lane] : 0u;
+      const int e = (int)(w & 0x3fffffffu);
+      const bool plain = (w >> 30) & 1u, flipped = (w >> 31) & 1u;
+      const uint64_t y = lane < count ? by[lane] : 0ull;
+      for (uint32_t left = alive; left != 0; left &= left - 1) {
+        const int i = __ffs(left) - 1;
+        const uint64_t a_i = __shfl_sync(FULL, (unsigned long long)v, i);
+        const uint64_t varying = a_i & ~run_known;
+        uint64_t z = y;
+        for (uint32_t bits = (uint32_t)varying; bits != 0; bits &= bits - 1) z |= image(__ffs(bits) - 1, e);
+        for (uint32_t bits = (uint32_t)(varying >> 32); bits != 0; bits &= bits - 1) z |= image(__ffs(bits) + 31, e);
+        const uint64_t zf = z ^ full;
+        if (__any_sync(FULL, (plain && z < a_i) || (flipped && zf < a_i))) {
+          alive &= ~(1u << i);
+          continue;
+        }
+        const bool p = plain && z == a_i, f = flipped && zf == a_i;
+        for (unsigned m = __ballot_sync(FULL, p || f); m != 0; m &= m - 1) {
+          const int src = __ffs(m) - 1;
+          const int es = __shfl_sync(FULL, e, src);
+          const int ps = __shfl_sync(FULL, (int)p, src), fs = __shfl_sync(FULL, (int)f, src);
+          if (lane == i) {
+            // one member -- the identity, nearly always -- is only noted: its FP64 sum is done for
+            // all candidates at once below (the FP64 pipe was half busy with one lane at a time)
+            const uint32_t member = (uint32_t)es | (ps ? 1u << 30 : 0u) | (fs ? 1u << 31 : 0u);
+            if (!any_noted && !summed) {
+              noted = member;
+              any_noted = true;
+            } else {
+              if (any_noted) add_member(noted, a_i);
+              any_noted = false;
+              summed = true;
+              add_member(member, a_i);
+            }
+          }
+        }
+      }
+    };
+    int waiting = 0;  // elements in the buffer that the run's common bits leave open
+    for (int k0 = 0; k0 < u && alive != 0; k0 += 32) {
+      const bool valid = k0 + lane < u;
+      const uint32_t w = valid ? ue[k0 + lane] : 0u;
+      const int e = (int)(w & 0x3fffffffu);
+      uint64_t y = valid ? uy[k0 + lane] : 0ull, ky = valid ? uk[k0 + lane] : 0ull;
+      for (uint64_t bits = run_known & ~known; bits != 0; bits &= bits - 1) {
+        const int b = __ffsll((long long)bits) - 1;
+        const uint64_t img = image(b, e);
+        ky |= img;
+        if ((F >> b) & 1ull) y |= img;
+      }
+      const uint32_t r = valid ? compare(F, run_known, y, ky) : 0u;
+      const bool plain_ok = (w >> 30) & 1u, flipped_ok = (w >> 31) & 1u;
+      if (__any_sync(FULL, (plain_ok && (r & 2u)) || (flipped_ok && (r & 8u)))) return 0u;
+      const bool plain = plain_ok && (r & 1u), flipped = flipped_ok && (r & 4u);
+      const unsigned m = __ballot_sync(FULL, plain || flipped);
+      if (plain || flipped) {
+        const int at = waiting + __popc(m & ((1u << lane) - 1u));
+        by[at] = y;
+        be[at] = (uint32_t)e | (plain ? 1u << 30 : 0u) | (flipped ? 1u << 31 : 0u);
+      }
+      waiting += __popc(m);
+      __syncwarp();
+      if (waiting < 32) continue;
+      test(32);
+      waiting -= 32;
+      const uint64_t my = by[32 + lane];
+      const uint32_t me = be[32 + lane];
+      __syncwarp();
+      if (lane < waiting) {
+        by[lane] = my;
+        be[lane] = me;
+      }
+      __syncwarp();
+    }
+    if (alive != 0 && waiting > 0) test(waiting);
+    __syncwarp();  // the next run reuses the buffer
+    if (any_noted) add_member(noted, v);
+    sum += chunk_sum;
+    const bool keep = a.reference_rule ? sum > 0 : trivial && members > 0;
+    *stabiliser = trivial ? members : 0;
+    return alive & __ballot_sync(FULL, keep);
+  };
+
+  const int64_t item_size = (int64_t)q.tile * q.super;
+  const int segments = q.tile / 32;                                   // of 32 candidates: one word of flags
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) item_s = atomicAdd(q.next, 1ull);
+    __syncthreads();
+    const int64_t item = (int64_t)item_s;
+    if (item >= q.n_items) break;
+    const int64_t item_first = item * item_size;
+    const int64_t item_count = min(item_size, a.n_candidates - item_first);
+    if (q.super > 1 && prune(item_first, item_count) < 0) continue;
+    for (int64_t off = 0; off < item_count; off += q.tile) {
+      const int64_t first = item_first + off, count = min((int64_t)q.tile, item_count - off);
+      const int u = prune(first, count);  // its barriers end the previous tile's reads
+      if (u < 0) continue;
+      if (tid < segments) flags[tid] = 0;
+      if (tid == 0) next_run = 0;
+      __syncthreads();
+      for (;;) {
+        int r = 0;
+        if (lane == 0) r = atomicAdd(&next_run, 32);
+        r = __shfl_sync(FULL, r, 0);
+        if (r >= count) break;
+        const int todo = (int)min((int64_t)32, count - r);
+        const uint64_t v = candidate_at(a, first + r + min(lane, todo - 1), [&](int c, int k) -> uint64_t {
+          return c <= 0 || k > c ? 0ull : binomials[c * weights + k];
+        });
+        int stabiliser = 0;
+        const uint32_t keep = kept_of(v, todo, u, &stabiliser);
+        if ((keep >> lane) & 1u) {
+          kept[r + lane] = v;
+          kept_stab[r + lane] = (uint16_t)stabiliser;
+        }
+        if (lane == 0) flags[r >> 5] = keep;
+      }
+      __syncthreads();
+      int before = 0, total = 0;  // of this warp's first segment; of the tile
+      for (int w = 0; w < segments; ++w) {
+        const int c = __popc(flags[w]);
+        before += w < warp ? c : 0;
+        total += c;
+      }
+      if (tid == 0) {
+        const int64_t t = first / q.tile;
+        base_s = total > 0 ? atomicAdd(a.counter, (unsigned long long)total) : 0ull;
+        a.tile_count[t] = total;
+        a.tile_start[t] = (int64_t)base_s;
+      }
+      __syncthreads();
+      int64_t at = (int64_t)base_s + before;
+      for (int w = warp; w < segments; w += kPruneWarps) {
+        const uint32_t m = flags[w];
+        const int64_t to = at + __popc(m & ((1u << lane) - 1u));
+        if (((m >> lane) & 1u) && to < a.capacity) {
+          a.append[to] = kept[32 * w + lane];
+          a.append_stab[to] = kept_stab[32 * w + lane];
+        }
+        for (int i = w; i < min(w + kPruneWarps, segments); ++i) at += __popc(flags[i]);
       }
     }
-    __syncthreads();
   }
 }
 
-template <int D>
-struct RunEnumerate {
-  static void run(const DeviceGroup& g, const EnumArgs& a, cudaStream_t s) {
-    int64_t blocks = std::min<int64_t>(a.n_tiles, (int64_t)num_sms() * 8);
-    if (blocks < 1) blocks = 1;
-    k_enumerate_projected<D><<<(unsigned)blocks, kEnumThreads, 0, s>>>(g, a);
-  }
-};
-
+// Copies every tile's run to its place in the output, with the orbit norms sqrt(S / |G|) and their
+// inverses: a warp per tile.
 __global__ void k_gather_runs(int64_t n_tiles, const int32_t* __restrict__ tile_count,
                               const int64_t* __restrict__ tile_start,
                               const int64_t* __restrict__ tile_offset,
-                              const uint64_t* __restrict__ append, uint64_t* __restrict__ out) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_tiles;
-       t += (int64_t)gridDim.x * blockDim.x) {
+                              const uint64_t* __restrict__ append, const uint16_t* __restrict__ append_stab,
+                              double denominator, uint64_t* __restrict__ out, double* __restrict__ norms,
+                              double* __restrict__ inv_norms) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < n_tiles; t += warps) {
     const int c = tile_count[t];
+    if (c == 0) continue;
     const int64_t src = tile_start[t], dst = tile_offset[t];
-    for (int k = 0; k < c; ++k) out[dst + k] = append[src + k];
+    for (int k = lane; k < c; k += 32) {
+      out[dst + k] = append[src + k];
+      const double v = sqrt((double)append_stab[src + k] / denominator);  // as k_orbit_norms
+      norms[dst + k] = v;
+      inv_norms[dst + k] = v == 0.0 ? 0.0 : 1.0 / v;
+    }
   }
 }
 
@@ -871,8 +1163,9 @@ __global__ void k_enumerate_spinful(int64_t rankA, int64_t nA, int hA, int64_t r
 }
 
 int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_t** d_out,
-                     int64_t* count, cudaStream_t s) {
+                     double** d_norms, int64_t* count, cudaStream_t s) {
   *d_out = nullptr;
+  *d_norms = nullptr;
   *count = 0;
   if (ensure_binomials() != 0) return LS_GPU_ERR_CUDA;
   const int n_bits = (req.mode == 2 || req.mode == 3) ? 2 * req.number_sites : req.number_sites;
@@ -941,6 +1234,26 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
   DeviceGroup g = strip(*g0);
   EnumArgs a{};
   projected_candidates(req, n_bits, &a);
+  // tiles small enough that every SM gets several, work items of many tiles only for long ranges
+  const int sms = num_sms();
+  PruneArgs q{};
+  q.tile = kPruneTile;
+  while (q.tile > 256 && a.n_candidates < (int64_t)q.tile * sms * 8) q.tile /= 2;
+  a.n_tiles = (a.n_candidates + q.tile - 1) / q.tile;
+  q.super = a.n_tiles >= (int64_t)sms * 8 * kPruneSuper ? kPruneSuper : 1;
+  q.n_items = (a.n_tiles + q.super - 1) / q.super;
+  const size_t table_bytes = (size_t)n_bits * g.n_elems * 8;
+  size_t smem = (size_t)q.tile * 10 + (size_t)g.n_elems * 20 + (size_t)kPruneWarps * 64 * 12;
+  smem = (smem + 15) & ~(size_t)15;
+  const size_t binomial_bytes = (size_t)n_bits * (n_bits + 1) * 8;  // of at most n_bits lengths and weights
+  smem += binomial_bytes;
+  const bool table = smem + table_bytes <= 224 * 1024;  // 1.5 KB are static
+  if (table) smem += table_bytes;
+  q.binomials_at = (int)(smem - binomial_bytes);
+  const auto kernel = table ? k_enumerate_pruned<true> : k_enumerate_pruned<false>;
+  if (!cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+               "smem attribute"))
+    return LS_GPU_ERR_CUDA;
   // Capacity guess: candidates / |G| * 2 + slack; retried with the exact count on overflow.
   int64_t capacity = std::min<int64_t>(a.n_candidates,
                                        a.n_candidates / std::max(1, g.n_elems) * 2 + 1024 * 1024);
@@ -949,7 +1262,9 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
   int64_t* tile_offset = nullptr;
   unsigned long long* counter = nullptr;
   uint64_t* append = nullptr;
+  uint16_t* append_stab = nullptr;
   auto cleanup = [&]() {
+    cudaFree(append_stab);
     cudaFree(tile_count);
     cudaFree(tile_start);
     cudaFree(tile_offset);
@@ -959,27 +1274,31 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
   if (!cuda_ok(cudaMalloc((void**)&tile_count, a.n_tiles * 4), "alloc") ||
       !cuda_ok(cudaMalloc((void**)&tile_start, a.n_tiles * 8), "alloc") ||
       !cuda_ok(cudaMalloc((void**)&tile_offset, (a.n_tiles + 1) * 8), "alloc") ||
-      !cuda_ok(cudaMalloc((void**)&counter, 8), "alloc")) {
+      !cuda_ok(cudaMalloc((void**)&counter, 16), "alloc")) {
     cleanup();
     return LS_GPU_ERR_CUDA;
   }
+  q.next = counter + 1;
   unsigned long long total = 0;
   for (int attempt = 0; attempt < 2; ++attempt) {
-    if (!cuda_ok(cudaMalloc((void**)&append, std::max<int64_t>(capacity, 1) * 8), "alloc append")) {
+    if (!cuda_ok(cudaMalloc((void**)&append, std::max<int64_t>(capacity, 1) * 8), "alloc append") ||
+        !cuda_ok(cudaMalloc((void**)&append_stab, std::max<int64_t>(capacity, 1) * 2), "alloc append")) {
       cleanup();
       return LS_GPU_ERR_CUDA;
     }
     a.tile_count = tile_count;
     a.tile_start = tile_start;
     a.append = append;
+    a.append_stab = append_stab;
     a.capacity = capacity;
     a.counter = counter;
-    cudaMemsetAsync(counter, 0, 8, s);
+    cudaMemsetAsync(counter, 0, 16, s);
+    cudaMemsetAsync(tile_count, 0, (size_t)a.n_tiles * 4, s);  // pruned tiles write nothing
     {
       StageScope stage("basis.enumerate", s);
-      dispatch_depth<RunEnumerate>(g.depth, group_is_standard(*g0), g, a, s);
+      kernel<<<(unsigned)std::min<int64_t>(q.n_items, sms), kPruneThreads, smem, s>>>(g, a, q);
     }
-    if (!cuda_ok(cudaGetLastError(), "k_enumerate_projected") ||
+    if (!cuda_ok(cudaGetLastError(), "k_enumerate_pruned") ||
         !cuda_ok(cudaMemcpyAsync(&total, counter, 8, cudaMemcpyDeviceToHost, s), "read count") ||
         !cuda_ok(cudaStreamSynchronize(s), "enumerate")) {
       cleanup();
@@ -987,12 +1306,18 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
     }
     if ((int64_t)total <= capacity) break;
     cudaFree(append);
+    cudaFree(append_stab);
     append = nullptr;
+    append_stab = nullptr;
     capacity = (int64_t)total;
   }
   uint64_t* out = nullptr;
-  if (!cuda_ok(cudaMalloc((void**)&out, std::max<unsigned long long>(total, 1) * 8), "alloc out")) {
+  double* norms = nullptr;  // norms | inverse norms
+  const size_t n_out = (size_t)std::max<unsigned long long>(total, 1);
+  if (!cuda_ok(cudaMalloc((void**)&out, n_out * 8), "alloc out") ||
+      !cuda_ok(cudaMalloc((void**)&norms, n_out * 16), "alloc norms")) {
     cleanup();
+    cudaFree(out);
     return LS_GPU_ERR_CUDA;
   }
   int rc = 0;
@@ -1000,8 +1325,10 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
     StageScope stage("basis.enumerate_compact", s);
     rc = exclusive_scan<int32_t>(tile_count, a.n_tiles, tile_offset, s);
     if (rc == 0)
-      k_gather_runs<<<grid_for(a.n_tiles, 256), 256, 0, s>>>(a.n_tiles, tile_count, tile_start,
-                                                            tile_offset, append, out);
+      k_gather_runs<<<grid_for(a.n_tiles * 32, 256), 256, 0, s>>>(a.n_tiles, tile_count, tile_start,
+                                                                 tile_offset, append, append_stab,
+                                                                 (double)g.n_elems * (g.spin_inversion != 0 ? 2 : 1),
+                                                                 out, norms, norms + n_out);
   }
   if (rc == 0) {
     if (!cuda_ok(cudaGetLastError(), "k_gather_runs") || !cuda_ok(cudaStreamSynchronize(s), "gather"))
@@ -1010,9 +1337,11 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
   cleanup();
   if (rc != 0) {
     cudaFree(out);
+    cudaFree(norms);
     return rc;
   }
   *d_out = out;
+  *d_norms = norms;
   *count = (int64_t)total;
   return 0;
 }

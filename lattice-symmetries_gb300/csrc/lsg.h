@@ -207,9 +207,10 @@ struct EnumerateRequest {
   uint64_t lower, upper;
   int reference_norm_rule;  // 1: keep a state iff the reference's floating stabiliser sum > 0
 };
-// Enumerates into device memory; *d_out is allocated with cudaMalloc (caller frees).
+// Enumerates into device memory; *d_out is allocated with cudaMalloc (caller frees).  Projected
+// bases also get *d_norms (cudaMalloc): the orbit norms [n] and their inverses [n], n >= 1; else null.
 int enumerate_states(const DeviceGroup* g, const EnumerateRequest& req, uint64_t** d_out,
-                     int64_t* count, cudaStream_t s);
+                     double** d_norms, int64_t* count, cudaStream_t s);
 // Enumerates into the caller's d_out (capacity entries) without allocating: all scratch lives in
 // a static device array (see basis.cu).  *count receives the number of states.
 int enumerate_states_noalloc(const OrbitData* od, const EnumerateRequest& req, uint64_t* d_out,
