@@ -545,6 +545,7 @@ extern "C" void ls_hs_destroy_state_index_binary_search_kernel_data(
   cudaFree(cache->d_offsets);
   cudaFree(cache->d_suffix);
   cudaFree(cache->d_norms);
+  cudaFree(cache->d_ranks);
   cache->magic = 0;
   delete cache;
 }
@@ -1103,6 +1104,7 @@ RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons, const 
   R.st.resize(R.sm.size(), 0);
   R.shape.n_pat = (int)R.xmask.size();
   R.shape.n_cls = (int)(R.cval.size() / 2);
+  for (int k = 0; k < t.n; ++k) R.shape.any_sign |= t.s[k] != 0;
   R.shape.ok = 1;
   return R;
 }
@@ -1130,7 +1132,7 @@ RowTables diag_rows(const TermTable& t, const int32_t* coupling) {
         if (k >= 0 && members[c][b + i].second) signs |= 1u << i;
       }
       R.st.push_back(signs);
-      R.tinfo.push_back((uint32_t)c | (b + 32 >= members[c].size() ? 1u << 31 : 0u));
+      R.tinfo.push_back((uint32_t)c | ((uint32_t)n << 16) | (b + 32 >= members[c].size() ? 1u << 31 : 0u));
     }
   }
   R.shape.slot_blocks = (int)R.st.size();
@@ -1259,6 +1261,45 @@ int ensure_norms(IndexData* ix, const OrbitData* od) {
   return rc;
 }
 
+// Rank tables of a complete basis without a group: all states of a fixed weight (all below the
+// flipped maximum with spin inversion), or of fixed (N_up, N_down).  Other sets of states (installed
+// by the caller) and more than 40 bits keep the search.
+int ensure_ranks(IndexData* ix, ls_hs_basis const* b) {
+  if (ix->d_ranks != nullptr || ix->n_states == 0) return 0;
+  const int n = basis_number_bits(b);
+  if (n > 40) return 0;
+  int split = (n + 1) / 2, h = 0, species = 0;
+  int64_t n_lo = 0, expected = 0;
+  if (b->particle_type == LS_HS_SPINFUL_FERMION && b->number_up >= 0) {
+    species = 1;
+    split = b->number_sites;
+    h = b->number_particles - b->number_up;
+    n_lo = fixed_hamming_state_to_index(low_ones(b->number_up) << (split - b->number_up)) + 1;
+    expected = n_lo * (fixed_hamming_state_to_index(low_ones(h) << (split - h)) + 1);
+  } else {
+    if (!hamming_fixed(b)) return 0;
+    h = b->particle_type == LS_HS_SPIN ? b->number_up : b->number_particles;
+    expected = fixed_hamming_state_to_index(low_ones(h) << (n - h)) + 1;
+    if (b->particle_type == LS_HS_SPIN && b->spin_inversion != 0) expected /= 2;
+  }
+  if (ix->n_states != expected) return 0;
+  cudaStream_t s = default_stream();
+  const size_t lo = (size_t)1 << split, hi = (size_t)1 << (n - split);
+  if (!cuda_ok(cudaMalloc((void**)&ix->d_ranks, (lo + hi) * 4), "cudaMalloc(ranks)")) return LS_GPU_ERR_CUDA;
+  int rc = launch_rank_tables(split, n - split, h, species, n_lo, ix->d_ranks, ix->d_ranks + lo, s);
+  // read by kernels on the caller's stream
+  if (rc == 0) rc = cuda_ok(cudaStreamSynchronize(s), "rank tables") ? 0 : LS_GPU_ERR_CUDA;
+  if (rc != 0) {
+    cudaFree(ix->d_ranks);
+    ix->d_ranks = nullptr;
+    return rc;
+  }
+  ix->dev.rank_lo = ix->d_ranks;
+  ix->dev.rank_hi = ix->d_ranks + lo;
+  ix->dev.rank_split = split;
+  return 0;
+}
+
 // Builds the kernel-side description of y = op x (adjoint: y = op^dagger x).
 int make_problem(ls_hs_operator const* op, bool adjoint, MatvecProblem* p) {
   ls_hs_basis const* b = op->basis;
@@ -1272,6 +1313,7 @@ int make_problem(ls_hs_operator const* op, bool adjoint, MatvecProblem* p) {
   p->projection = !b->requires_projection ? 0 : (has_permutations(b) ? 2 : 1);
   if (p->projection == 1 && b->spin_inversion == 0) return fail(LS_GPU_ERR_INVALID, "projection without symmetries");
   if (ensure_norms(ix, p->projection == 2 ? od : nullptr) != 0) return LS_GPU_ERR_CUDA;
+  if (p->projection != 2 && !b->state_index_is_identity && ensure_ranks(ix, b) != 0) return LS_GPU_ERR_CUDA;
   p->group = DeviceGroup{};
   if (p->projection == 2) {
     const DeviceGroup* dg = orbit_device(od);

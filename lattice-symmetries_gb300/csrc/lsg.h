@@ -88,6 +88,10 @@ struct DeviceIndex {
   // combinadics ranking (fixed Hamming weight, no projection): index = rank(state) - rank_base
   int combinadic = 0;
   int64_t rank_base = 0;
+  // Complete bases without a group: index = rank_hi[state >> rank_split] + rank_lo[low bits], or null.
+  const uint32_t* rank_lo = nullptr;
+  const uint32_t* rank_hi = nullptr;
+  int rank_split = 0;
 };
 
 // Basis-level constraints checked on every generated state (fixed particle numbers).
@@ -111,8 +115,10 @@ struct DeviceRowTerms {
   const uint32_t* st = nullptr;    // terms of the patterns, first | second << 16 (diagonal: per
                                    // block, the signs of its 32 terms)
   const uint32_t* tinfo = nullptr;  // [terms] pattern | class << 16 | check << 30 | sign << 31
-                                    // (diagonal: per block, class | last block of the class << 31)
+                                    // (diagonal: per block, class | terms << 16 | last block of the
+                                    // class << 31)
   int n_pat = 0, n_cls = 0;
+  int any_sign = 0;                // some off-diagonal term has a sign mask
   const uint64_t* xmask = nullptr;  // [n_pat] flip masks
   const double2* cval = nullptr;    // [n_cls]
   const uint32_t* coupling = nullptr;  // [n_cls] coupling id (terms of different couplings share no class)
@@ -171,6 +177,7 @@ struct IndexData {
   uint16_t* d_suffix = nullptr;       // 2-byte key suffixes (shift <= 16)
   double* d_norms = nullptr;          // filled lazily when a projected matvec needs them
   const OrbitData* norms_for = nullptr;
+  uint32_t* d_ranks = nullptr;        // rank_lo | rank_hi of DeviceIndex, filled by the first matvec without a group
 };
 
 constexpr uint32_t kOrbitMagic = 0x4f524249u;  // "ORBI"
@@ -266,6 +273,13 @@ int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int
 // A stream-ordered copy of x scaled by the orbit norms (k columns of `words` doubles per element, rows of
 // ldxs elements), to be freed with cudaFreeAsync; null without memory or on a launch error.
 double* prescaled_copy(const MatvecProblem& p, int words, int k, const double* d_x, int64_t ldx, int64_t ldxs,
+                       cudaStream_t s);
+
+// Kernels of bases without a group (matvec_free.cu); rank tables of their states (see k_rank_tables).
+bool free_fits(const MatvecProblem& p);
+int launch_free(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y, int64_t ldy,
+                int* d_err, cudaStream_t s);
+int launch_rank_tables(int split, int high_bits, int h, int species, int64_t n_lo, uint32_t* d_lo, uint32_t* d_hi,
                        cudaStream_t s);
 
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,

@@ -307,6 +307,11 @@ int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, i
     }
     return 0;
   }
+  // counting elements, incomplete bases and more than 40 bits of a constrained basis keep the search kernel
+  if (free_fits(p)) {
+    StageScope stage("matvec.kernel", s);
+    return launch_free(p, sc, k, d_x, ldx, d_y, ldy, d_err, s);
+  }
   const SmemLayout L = make_layout(p, false);
   if (L.total > kMaxDynamicSmem) return fail(LS_GPU_ERR_INVALID, "term tables too large for shared memory");
   const int threads = 256;
