@@ -129,8 +129,8 @@ bool rows_fit(const MatvecProblem& p, int n_sectors) {
   return false;
 }
 
-// Shape for p (rows_fit): as many rows per warp as leave enough warps their area, fewer where the
-// last round of row groups over all warps would be a large part of the work.
+// Shape for p (rows_fit): the cheapest number of rows per warp among those that leave enough warps
+// their area.
 static bool rows_shape(const MatvecProblem& p, bool complex_elements, bool keep, int64_t n_rows, int n_sectors,
                        int max_warps, int sms, int* mode, RowsLayout* L) {
   for (const int m : {kModeN32, kModeP16}) {
@@ -147,13 +147,15 @@ static bool rows_shape(const MatvecProblem& p, bool complex_elements, bool keep,
       double least = 0.0;
       for (int i = 0; i < 4; ++i) {
         if (warps[i] < std::min(enough, max_warps) || warps[i] < 1) continue;
+        // rounds of row groups over all warps x steps of a group: images and lists row by row, the
+        // scan of 64 elements (about half the slots match) over all words
         const int64_t R = 8 >> i, all = (int64_t)sms * warps[i], groups = (n_rows + R - 1) / R;
-        const double waste = (double)((groups + all - 1) / all * all * R) / (double)std::max<int64_t>(1, n_rows);
-        if (pick < 0 || waste < least) {
+        const double scans = (double)((t[i].n_slots * R / 2 + 63) / 64) * (2.0 + t[i].words / 16.0);
+        const double cost = (double)((groups + all - 1) / all) * (4.0 + (double)R + scans);
+        if (pick < 0 || cost < least) {
           pick = i;
-          least = waste;
+          least = cost;
         }
-        if (waste <= 1.3) break;
       }
       if (pick < 0) continue;
       *mode = m;
@@ -207,10 +209,11 @@ int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int
   if (!rows_plan(p, col, k, p.n_rows, 0, &q))
     return fail(LS_GPU_ERR_INVALID, "row-group tables do not fit in shared memory");
   s.x = d_x;
-  s.xs = p.xs;
+  s.xs = p.xs != nullptr ? p.xs : d_x;
+  s.norms = p.xs != nullptr ? nullptr : p.index.norms;
   s.y = d_y;
   s.ldx = ldx;
-  s.ldxs = p.ldxs;
+  s.ldxs = p.xs != nullptr ? p.ldxs : ldx;
   s.ldy = ldy;
   const RowsLayout& L = q.L;
   const bool keep = s.cols > 1;

@@ -24,7 +24,8 @@ constexpr int kColReal = 0, kColPair = 1, kColComplex = 2;
 
 struct RowsSums {
   const double* x;   // the caller's vectors (diagonal), leading dimension ldx in scalars
-  const double* xs;  // x_j n_j, leading dimension ldxs in scalars
+  const double* xs;  // x_j n_j, leading dimension ldxs in scalars; x itself where norms != null
+  const double* norms;  // the orbit norms n_j where xs is not scaled (small problems), else null
   double* y;
   int64_t ldx, ldxs, ldy;
   int64_t rows_per_block, n_blocks;  // consecutive rows of one warp
@@ -70,6 +71,8 @@ __device__ __forceinline__ double flip_sign(double v, uint32_t sign) {
 __device__ __forceinline__ double2 flip_sign(double2 v, uint32_t sign) {
   return make_double2(flip_sign(v.x, sign), flip_sign(v.y, sign));
 }
+__device__ __forceinline__ double scaled(double v, double n) { return v * n; }
+__device__ __forceinline__ double2 scaled(double2 v, double n) { return make_double2(v.x * n, v.y * n); }
 __device__ __forceinline__ double shfl_down_v(double v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
 __device__ __forceinline__ double2 shfl_down_v(double2 v, int d) {
   return make_double2(__shfl_down_sync(0xffffffffu, v.x, d), __shfl_down_sync(0xffffffffu, v.y, d));
@@ -120,6 +123,10 @@ __device__ __forceinline__ void resolve_and_sum(Group& g, const RowsSums& s, con
     V xv[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) xv[e] = j[e] != Group::kAbsent ? __ldg(xs + (int64_t)j[e] * ldv) : Col::zero();
+    if (s.norms != nullptr) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) xv[e] = scaled(xv[e], j[e] != Group::kAbsent ? __ldg(s.norms + j[e]) : 0.0);
+    }
 #pragma unroll
     for (int e = 0; e < E; ++e)
       if (j[e] != Group::kAbsent) Col::mac(acc, flip_sign(coef[w[e] & 0x7fffffffu], w[e] & 0x80000000u), xv[e]);
@@ -168,6 +175,10 @@ __device__ __forceinline__ void sum_rows(const Group& g, const RowsSums& s, cons
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) xv[u] = w[u].x != Group::kAbsent ? __ldg(xs + (int64_t)w[u].x * ldv) : Col::zero();
+      if (s.norms != nullptr) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) xv[u] = scaled(xv[u], w[u].x != Group::kAbsent ? __ldg(s.norms + w[u].x) : 0.0);
+      }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (w[u].x != Group::kAbsent) Col::mac(acc, flip_sign(coef[w[u].y & 0x7fffffffu], w[u].y & 0x80000000u), xv[u]);
