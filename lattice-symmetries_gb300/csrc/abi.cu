@@ -2,12 +2,14 @@
 // ls_gpu_* symbols declared in include/ls_gb300.h.  Host logic only; kernels live in basis.cu
 // and matvec*.cu.
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -986,6 +988,7 @@ struct OperatorCache {
   DeviceTermSet fwd_off, adj_off, fwd_diag, adj_diag;
   // forward terms with coupling ids (made by the first coupling product; ids per term, off then diag)
   std::vector<int32_t> coupling;
+  int n_couplings = 0;
   DeviceTermSet cpl_off, cpl_diag;
 };
 
@@ -1043,6 +1046,7 @@ struct RowTables {
   std::vector<uint32_t> st, tinfo;
   std::vector<double> cval;  // interleaved
   std::vector<uint32_t> coupling;  // per class
+  std::vector<double> cvec;        // merged: [class][coupling] interleaved
 };
 
 // The class of a term of coefficient v (equal up to sign) and coupling id, appended when new; *neg:
@@ -1063,22 +1067,89 @@ int coefficient_class(RowTables* R, double re, double im, int coupling, bool* ne
 }
 
 constexpr int kMaxRowClasses = 64;
+constexpr int kMaxMergedClasses = 4;  // sums per lane of the coupling products
 
-// Slots, patterns and classes of off-diagonal terms (matched through t.l); coupling: an id per term,
-// or null (all 0).
-RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons, const int32_t* coupling) {
+// Which earlier term every term acts like (the same pattern, flip and sign masks), or itself.
+std::vector<int> alike_terms(const TermTable& t) {
+  std::vector<int> same(t.n);
+  std::map<std::array<uint64_t, 5>, int> seen;
+  for (int k = 0; k < t.n; ++k) same[k] = seen.emplace(std::array<uint64_t, 5>{t.m[k], t.l[k], t.r[k], t.x[k], t.s[k]}, k).first->second;
+  return same;
+}
+
+// Slots, patterns and classes of off-diagonal terms (matched through t.l).  Terms that act alike are
+// one element with the sum of their coefficients.  coupling: an id per term, or null.  With ids,
+// alike terms of different couplings are still one element where few classes result: a class is
+// then a vector of coefficients, one per coupling (cvec); else every coupling has its own terms.
+RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons, const int32_t* coupling, int n_couplings) {
   RowTables R;
   if (t.n > 32767) return R;
+  std::vector<int> same = alike_terms(t);
+  std::vector<double> v = t.v;  // per term: the sum over the terms alike
+  std::vector<int> cls(t.n, 0);
+  std::vector<bool> neg(t.n, false);
+  bool merged = coupling != nullptr;
+  if (merged) {
+    const size_t row = 2 * (size_t)n_couplings;
+    std::vector<double> vec(row * t.n, 0.0);
+    for (int k = 0; k < t.n; ++k) {
+      vec[row * same[k] + 2 * coupling[k]] += t.v[2 * k];
+      vec[row * same[k] + 2 * coupling[k] + 1] += t.v[2 * k + 1];
+    }
+    for (int k = 0; k < t.n && merged; ++k) {
+      if (same[k] != k) continue;
+      const double* mine = vec.data() + row * k;
+      const int n = (int)(R.cvec.size() / row);
+      int c = 0;
+      for (; c < n; ++c) {
+        const double* other = R.cvec.data() + row * c;
+        bool plus = true, minus = true;
+        for (size_t i = 0; i < row; ++i) {
+          plus = plus && mine[i] == other[i];
+          minus = minus && mine[i] == -other[i];
+        }
+        if (plus || minus) {
+          neg[k] = !plus;
+          break;
+        }
+      }
+      if (c == n) R.cvec.insert(R.cvec.end(), mine, mine + row);
+      cls[k] = c;
+      merged = c < kMaxMergedClasses;
+    }
+  }
+  if (merged) {
+    R.shape.n_cls = (int)(R.cvec.size() / (2 * (size_t)n_couplings));
+    R.shape.merged = 1;
+    R.cval.assign(2 * (size_t)R.shape.n_cls, 0.0);
+    for (int c = 0; c < R.shape.n_cls; ++c) R.cval[2 * c] = 1.0;  // the vectors come in at the end
+    R.coupling.resize(R.shape.n_cls);
+    for (int c = 0; c < R.shape.n_cls; ++c) R.coupling[c] = (uint32_t)c;
+  } else {
+    R.cvec.clear();
+    for (int k = 0; k < t.n; ++k) {
+      if (coupling != nullptr) same[k] = k;  // every coupling keeps its own terms
+      if (same[k] == k) continue;
+      v[2 * same[k]] += t.v[2 * k];
+      v[2 * same[k] + 1] += t.v[2 * k + 1];
+    }
+    for (int k = 0; k < t.n; ++k) {
+      if (same[k] != k) continue;
+      bool minus = false;
+      cls[k] = coefficient_class(&R, v[2 * k], v[2 * k + 1], coupling ? coupling[k] : 0, &minus);
+      neg[k] = minus;
+      if (cls[k] >= kMaxRowClasses) return R;
+    }
+    R.shape.n_cls = (int)(R.cval.size() / 2);
+  }
   std::unordered_map<uint64_t, int> pattern;
   std::unordered_map<uint64_t, std::vector<int>> open;  // mask -> slots with a free second pattern
   R.tinfo.assign((size_t)std::max(t.n, 1), 0);
   for (int k = 0; k < t.n; ++k) {
+    if (same[k] != k) continue;
     const auto it = pattern.emplace(t.x[k], (int)pattern.size());
     if (it.second) R.xmask.push_back(t.x[k]);
-    bool neg = false;
-    const int cls = coefficient_class(&R, t.v[2 * k], t.v[2 * k + 1], coupling ? coupling[k] : 0, &neg);
-    if (cls >= kMaxRowClasses) return R;
-    R.tinfo[k] = (uint32_t)it.first->second | ((uint32_t)cls << 16) | (neg ? 1u << 31 : 0u) |
+    R.tinfo[k] = (uint32_t)it.first->second | ((uint32_t)cls[k] << 16) | (neg[k] ? 1u << 31 : 0u) |
                  (term_breaks_constraint(cons, t.l[k], t.r[k]) ? kRowTermNeedsCheck : 0u);
     std::vector<int>& free_slots = open[t.m[k]];
     size_t f = 0;
@@ -1103,7 +1174,6 @@ RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons, const 
   R.sl2.resize(R.sm.size(), 1);
   R.st.resize(R.sm.size(), 0);
   R.shape.n_pat = (int)R.xmask.size();
-  R.shape.n_cls = (int)(R.cval.size() / 2);
   for (int k = 0; k < t.n; ++k) R.shape.any_sign |= t.s[k] != 0;
   R.shape.ok = 1;
   return R;
@@ -1146,7 +1216,7 @@ RowTables diag_rows(const TermTable& t, const int32_t* coupling) {
 // Device layout: v (double2, 16-byte aligned) first, then m, l, r, x, s (uint64), xinfo (uint32),
 // then the row-group tables, each array on a 16-byte boundary.
 int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal, DeviceTermSet* out,
-                 const int32_t* coupling = nullptr) {
+                 const int32_t* coupling = nullptr, int n_couplings = 0) {
   std::vector<uint8_t> host;
   auto put = [&](const void* src, size_t sz) {
     const size_t at = (host.size() + 15) & ~(size_t)15;
@@ -1166,7 +1236,7 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal
     xinfo[k] = info;
     if (cnt != 2 || (info & kTermNeedsCheck)) all_two = 0;
   }
-  const RowTables R = diagonal ? diag_rows(t, coupling) : off_diag_rows(t, cons, coupling);
+  const RowTables R = diagonal ? diag_rows(t, coupling) : off_diag_rows(t, cons, coupling, n_couplings);
   const size_t n = (size_t)t.n;
   const size_t ov = put(t.v.data(), n * 16), om = put(t.m.data(), n * 8), ol = put(t.l.data(), n * 8);
   const size_t orr = put(t.r.data(), n * 8), ox = put(t.x.data(), n * 8), os = put(t.s.data(), n * 8);
@@ -1175,6 +1245,7 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal
   const size_t rl2 = put(R.sl2.data(), R.sl2.size() * 8), rst = put(R.st.data(), R.st.size() * 4);
   const size_t rti = put(R.tinfo.data(), R.tinfo.size() * 4), rxm = put(R.xmask.data(), R.xmask.size() * 8);
   const size_t rcv = put(R.cval.data(), R.cval.size() * 8), rcc = put(R.coupling.data(), R.coupling.size() * 4);
+  const size_t rcm = put(R.cvec.data(), R.cvec.size() * 8);
   const size_t ocp = put(coupling, coupling ? n * 4 : 0);
   out->terms.all_two_site = all_two;
   if (!cuda_ok(cudaMalloc(&out->block, host.size()), "cudaMalloc(terms)")) return LS_GPU_ERR_CUDA;
@@ -1199,6 +1270,7 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal
   r.xmask = (const uint64_t*)(d + rxm);
   r.cval = (const double2*)(d + rcv);
   r.coupling = (const uint32_t*)(d + rcc);
+  r.cvec = (const double2*)(d + rcm);
   out->terms.coupling = coupling ? (const int32_t*)(d + ocp) : nullptr;
   return 0;
 }
@@ -1735,15 +1807,16 @@ extern "C" int ls_gpu_coupling_inner_products(ls_hs_operator const* op, int n_co
   for (int t = 0; t < n_terms; ++t)
     if (term_coupling[t] < 0 || term_coupling[t] >= n_couplings)
       return fail(LS_GPU_ERR_INVALID, "term coupling id out of range");
-  if (c->cpl_off.block == nullptr || c->cpl_diag.block == nullptr || c->coupling.size() != (size_t)n_terms ||
+  if (c->cpl_off.block == nullptr || c->cpl_diag.block == nullptr || c->coupling.size() != (size_t)n_terms || c->n_couplings != n_couplings ||
       (n_terms > 0 && memcmp(c->coupling.data(), term_coupling, (size_t)n_terms * 4) != 0)) {
     for (DeviceTermSet* s : {&c->cpl_off, &c->cpl_diag}) {
       if (s->block) cudaFree(s->block);
       s->block = nullptr;
     }
     c->coupling.assign(term_coupling, term_coupling + n_terms);
+    c->n_couplings = n_couplings;
     const DeviceConstraint cons = basis_constraint(op->basis);
-    if (upload_terms(c->off, cons, false, &c->cpl_off, term_coupling) ||
+    if (upload_terms(c->off, cons, false, &c->cpl_off, term_coupling, n_couplings) ||
         upload_terms(c->diag, cons, true, &c->cpl_diag, term_coupling + c->off.n))
       return LS_GPU_ERR_CUDA;
   }

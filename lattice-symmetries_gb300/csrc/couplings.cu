@@ -12,7 +12,9 @@
 // k_coupling_rows does the same on the row-group orbit scan (one lane per element, rowgroup.cuh),
 // wherever its tables fit: a lane keeps one sum per coupling over its row's elements, with
 // x_j n_j from a prescaled copy and coefficients from the (class, element) table, and multiplies by
-// conj(g_i) / n_i once per row.  28-site ladder, 1.43e6 rows, 3 couplings: 7.1 ms with one
+// conj(g_i) / n_i once per row.  Alike terms of different couplings (Heisenberg and DM on a bond)
+// are one element: the lane then sums per class, and the class sums count for each coupling with the
+// class' coefficient at the very end.  28-site ladder, 1.43e6 rows, 3 couplings: 7.1 ms with one
 // warp per row (k_coupling_products), 2.3 ms with one lane per element; the scan and its
 // bookkeeping bound it.
 #include "matvec_launch.cuh"
@@ -190,7 +192,7 @@ __global__ void __launch_bounds__(kCouplingThreads, 1)
                     double2* __restrict__ partial, int* __restrict__ err, const uint64_t* __restrict__ binom) {
   extern __shared__ __align__(16) unsigned char smem[];
   using Group = RowGroup<MODE, INV, false, false>;
-  __shared__ uint8_t class_of_off[64], class_of_diag[64];  // coupling ids of the classes
+  __shared__ uint8_t class_of_off[64], class_of_diag[64];  // the sums that the classes go to
   if (threadIdx.x < 64) {
     class_of_off[threadIdx.x] = threadIdx.x < p.off.rows.n_cls ? (uint8_t)p.off.rows.coupling[threadIdx.x] : 0;
     class_of_diag[threadIdx.x] = threadIdx.x < p.diag.rows.n_cls ? (uint8_t)p.diag.rows.coupling[threadIdx.x] : 0;
@@ -203,9 +205,9 @@ __global__ void __launch_bounds__(kCouplingThreads, 1)
   const double2* __restrict__ xs = reinterpret_cast<const double2*>(s.xs);
   const double2* __restrict__ x = reinterpret_cast<const double2*>(s.x);
   const int lane = g.lane;
-  double2 tot[kMaxCouplings];
+  double2 tot[kMaxCouplings], dtot[kMaxCouplings];
 #pragma unroll
-  for (int c = 0; c < kMaxCouplings; ++c) tot[c] = make_double2(0.0, 0.0);
+  for (int c = 0; c < kMaxCouplings; ++c) tot[c] = dtot[c] = make_double2(0.0, 0.0);
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t b = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; b < s.n_blocks; b += n_warps) {
     const int64_t begin = b * s.rows_per_block, end = min(begin + s.rows_per_block, p.n_rows);
@@ -260,23 +262,42 @@ __global__ void __launch_bounds__(kCouplingThreads, 1)
 #pragma unroll
         for (int c = 0; c < kMaxCouplings; ++c) {
           const C2 v = cmul(C2{d[c].x, d[c].y}, gx);
-          tot[c] = add_v(tot[c], make_double2(v.re, v.im));
+          dtot[c] = add_v(dtot[c], make_double2(v.re, v.im));
         }
       }
     }
   }
-  __shared__ double2 wsum[kCouplingThreads / 32][kMaxCouplings];
+  // off-diagonal sums per class or coupling, diagonal sums per coupling
+  __shared__ double2 wsum[kCouplingThreads / 32][kMaxCouplings], dsum[kCouplingThreads / 32][kMaxCouplings];
   const int warp = threadIdx.x >> 5;
 #pragma unroll
   for (int c = 0; c < kMaxCouplings; ++c) {
     const double re = warp_sum(tot[c].x), im = warp_sum(tot[c].y);
-    if (lane == 0) wsum[warp][c] = make_double2(re, im);
+    const double dre = warp_sum(dtot[c].x), dim = warp_sum(dtot[c].y);
+    if (lane == 0) {
+      wsum[warp][c] = make_double2(re, im);
+      dsum[warp][c] = make_double2(dre, dim);
+    }
   }
   __syncthreads();
   if (threadIdx.x < nc) {
-    double2 t = make_double2(0.0, 0.0);
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = add_v(t, wsum[w][threadIdx.x]);
-    partial[(size_t)blockIdx.x * nc + threadIdx.x] = t;
+    C2 t{0.0, 0.0};
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+      if (!p.off.rows.merged) {
+        t.re += wsum[w][threadIdx.x].x;
+        t.im += wsum[w][threadIdx.x].y;
+      } else {
+        for (int c = 0; c < p.off.rows.n_cls; ++c) {
+          const double2 v = p.off.rows.cvec[c * nc + threadIdx.x];
+          const C2 f = cmul(C2{v.x, v.y}, C2{wsum[w][c].x, wsum[w][c].y});
+          t.re += f.re;
+          t.im += f.im;
+        }
+      }
+      t.re += dsum[w][threadIdx.x].x;
+      t.im += dsum[w][threadIdx.x].y;
+    }
+    partial[(size_t)blockIdx.x * nc + threadIdx.x] = make_double2(t.re, t.im);
   }
 }
 

@@ -121,7 +121,11 @@ struct DeviceRowTerms {
   int any_sign = 0;                // some off-diagonal term has a sign mask
   const uint64_t* xmask = nullptr;  // [n_pat] flip masks
   const double2* cval = nullptr;    // [n_cls]
-  const uint32_t* coupling = nullptr;  // [n_cls] coupling id (terms of different couplings share no class)
+  // Coupling products: [n_cls] the sum that a class goes to -- its coupling, or, merged, the class
+  // itself, whose sum counts cvec[class][coupling] times for each coupling.
+  const uint32_t* coupling = nullptr;
+  int merged = 0;
+  const double2* cvec = nullptr;
 };
 constexpr uint32_t kRowTermNeedsCheck = 1u << 30;
 

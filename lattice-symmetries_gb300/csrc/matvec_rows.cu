@@ -37,8 +37,8 @@ __global__ void __launch_bounds__(kRowsThreads<KEEP>, 1)
   }
 }
 
-// Dynamic shared memory of a row-group kernel (the coupling products keep 1.2 KB more, statically).
-constexpr size_t kRowsSmem = kMaxDynamicSmem - 2048;
+// Dynamic shared memory of a row-group kernel (the coupling products keep 2.2 KB more, statically).
+constexpr size_t kRowsSmem = kMaxDynamicSmem - 4096;
 
 // Layout for `warps` warps of R rows (keep: the resolved elements are kept in shared memory); false when it exceeds the shared memory of a CTA.
 static bool rows_layout(const MatvecProblem& p, int mode, bool complex_elements, bool keep, int n_sectors,

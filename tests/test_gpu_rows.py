@@ -117,3 +117,34 @@ def test_non_finite_input_reaches_its_rows_only(cases, bad):
     y = c.op.apply_device(torch.from_numpy(x).cuda()).cpu().numpy()
     reached[j] = True
     assert np.array_equal(~np.isfinite(y), reached)
+
+
+@pytest.mark.parametrize("many", [False, True])
+def test_alike_terms_of_several_couplings(many):
+    """Couplings that share bonds: their alike terms are one element, summed per class (up to four
+    classes) or per coupling (more).  Every coupling's product against the oracle's matvec of it."""
+    import importlib
+    import torch
+    ag = importlib.import_module("lattice-symmetries_gb300.autograd")
+    n = 7
+    legs, rungs = LAT.ladder(n)
+    parts = [LAT.heisenberg(legs), LAT.dm_z(legs, 0.6), LAT.heisenberg(rungs),
+             LAT.heisenberg(rungs, 0.5) + LAT.dm_z(legs, 0.3) + LAT.heisenberg(legs, -0.7)]
+    if many:  # five classes: both directions of the legs and of the second neighbours, and the rungs
+        second = [(leg + i, leg + (i + 2) % n) for leg in (0, n) for i in range(n)]
+        parts[2] = parts[2] + LAT.heisenberg(second, 0.2) + LAT.dm_z(second, 0.35)
+    b = ls.SpinBasis(2 * n, n, None, ls.Symmetries(LAT.ladder_symmetries(n, 2)))
+    b.build(exact_norms=True)
+    pop = ag.ParametrizedOperator(b, parts, [0.4, 1.1, -0.7, 0.3])
+    D = b.number_states
+    rng = np.random.default_rng(8)
+    g, x = (rng.normal(size=D) + 1j * rng.normal(size=D) for _ in range(2))
+    out = pop.coupling_products(torch.from_numpy(g).cuda(), torch.from_numpy(x).cuda()).cpu().numpy()
+    y = pop.operator.apply_device(torch.from_numpy(x).cuda()).cpu().numpy()
+    total = np.zeros(D, dtype=np.complex128)
+    for c, part in enumerate(parts):
+        hx = Case(b, part).oracle_matvec(b.states, x, complex_=True)
+        total += pop.theta[c] * hx
+        # a sum of D products: FP64 rounding below D * 2^-53 * |g| |H x|
+        assert abs(out[c] - np.vdot(g, hx)) <= RTOL * np.linalg.norm(g) * np.linalg.norm(hx)
+    assert np.linalg.norm(y - total) <= RTOL * np.linalg.norm(total)
