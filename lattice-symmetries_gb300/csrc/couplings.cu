@@ -324,8 +324,12 @@ static int launch_coupling_rows(const MatvecProblem& p, int nc, const double* d_
   };
   const bool inv = p.group.spin_inversion != 0;
   int rc;
-  if (q.mode == kModeN32) rc = inv ? go(k_coupling_rows<kModeN32, true>) : go(k_coupling_rows<kModeN32, false>);
-  else rc = inv ? go(k_coupling_rows<kModeP16, true>) : go(k_coupling_rows<kModeP16, false>);
+  switch (q.mode) {  // groups of at most 128 elements
+    case kModeN32: rc = inv ? go(k_coupling_rows<kModeN32, true>) : go(k_coupling_rows<kModeN32, false>); break;
+    case 2: rc = inv ? go(k_coupling_rows<2, true>) : go(k_coupling_rows<2, false>); break;
+    case 5: rc = inv ? go(k_coupling_rows<5, true>) : go(k_coupling_rows<5, false>); break;
+    default: rc = fail(LS_GPU_ERR_INVALID, "coupling products: at most 128 group elements");
+  }
   cudaFreeAsync(d_xs, st);
   return rc;
 }

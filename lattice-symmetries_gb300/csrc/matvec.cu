@@ -201,7 +201,7 @@ static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const do
 }
 
 // Row-group kernels wherever their tables fit (faster than the packed kernels at every measured size
-// and group: 2.0x at 576 images, 2.3x at 56 with 16 columns, 9.7x at 150 with five; level at 257
+// and group: 2.3x at 576 images, 2.3x at 56 with 16 columns, 10.6x at 150 with five; 1.2x at 257
 // rows, where launches count); otherwise splits k right-hand sides into launches of
 // 16, 8, 4 and 1 columns of the packed kernels.
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,

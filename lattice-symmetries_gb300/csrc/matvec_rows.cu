@@ -1,44 +1,32 @@
 // matvec_rows.cu -- y = H x from the row-group orbit scan (rowgroup.cuh, rowsums.cuh): projected bases, real
-// or complex vectors, up to 16 complex or 32 real columns per launch.
+// or complex vectors, up to 16 complex or 32 real columns per launch.  The choice of mode and shape,
+// and the kernels of the N32 mode; those of the bit planes are in matvec_rows_w*.cu.
 #include <algorithm>
+#include <cmath>
 
-#include "matvec_launch.cuh"
-#include "rowsums.cuh"
+#include "rowkernel.cuh"
 
 namespace lsg {
 
-template <int MODE, bool INV, bool FERMI, int COL, bool KEEP>
-__global__ void __launch_bounds__(kRowsThreads<KEEP>, 1)
-    k_matvec_rows(const MatvecProblem p, const RowsLayout L, const RowsSums s, int* __restrict__ err,
-                  const uint64_t* __restrict__ binom) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  using Group = RowGroup<MODE, INV, FERMI, KEEP>;
-  Group::stage(L, p, smem);
-  auto* coef = reinterpret_cast<typename Column<COL>::C*>(smem + L.off_coef);
-  stage_coefficients<COL>(L, p.off.rows, p.group.chars, coef);
-  __syncthreads();
-  Group g(L, p, smem);
-  // blocks of rows are dealt across the CTAs first: a last round that does not fill the grid
-  // leaves a few warps on every SM instead of whole SMs without work (28-site chain, 16 columns:
-  // the busiest SM had 17 % more FP64 work than the mean)
-  const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t b = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; b < s.n_blocks; b += n_warps) {
-    const int64_t begin = b * s.rows_per_block, end = min(begin + s.rows_per_block, p.n_rows);
-    g.restart();
-    for (int64_t row = begin; row < end; row += L.R) {
-      g.load_rows(p.index, row, (int)min((int64_t)L.R, end - row));
-      if constexpr (KEEP) {
-        g.resolve(p.index, err, binom);
-        sum_rows<COL>(g, s, coef, row);
-      } else {
-        resolve_and_sum<COL>(g, s, p.index, coef, row, err, binom);
-      }
-    }
-  }
+// Planes of the bit-plane scan: enough for about 2^-4 ties per target, log2 |G| + 4 bits at half
+// filling, more where the particle number leaves less than a bit per site.
+static int rows_planes(const MatvecProblem& p) {
+  const int n = p.group.n_bits, inv = p.group.spin_inversion != 0 ? 1 : 0;
+  double f = 0.5;
+  if (p.constraint.kind == 1) f = (double)p.constraint.w0 / n;
+  if (p.constraint.kind == 2) f = (double)(p.constraint.w0 + p.constraint.w1) / n;
+  const double entropy = f <= 0.0 || f >= 1.0 ? 0.0 : -(f * std::log2(f) + (1.0 - f) * std::log2(1.0 - f));
+  const double want = std::log2((double)std::max(p.group.n_elems, 1)) / std::max(entropy, 0.2) + 4.0;
+  return std::max(1, std::min({(int)std::ceil(want), n - inv, 32}));
 }
 
 // Dynamic shared memory of a row-group kernel (the coupling products keep 2.2 KB more, statically).
 constexpr size_t kRowsSmem = kMaxDynamicSmem - 4096;
+
+// Shared memory that leaves 60 KB of L1 for the gathers instead of 28 KB.  One column scatters its
+// reads of x and of the index: 6x6 torus, 4 rows per warp, 20 warps within this 73.5 ms, 24 warps
+// beyond it 80.5 ms (18 and 22 warps, which load the schedulers unevenly, 80.8 and 83.3 ms).
+constexpr size_t kRowsSmemL1 = 194 * 1024;
 
 // Layout for `warps` warps of R rows (keep: the resolved elements are kept in shared memory); false when it exceeds the shared memory of a CTA.
 static bool rows_layout(const MatvecProblem& p, int mode, bool complex_elements, bool keep, int n_sectors,
@@ -64,13 +52,19 @@ static bool rows_layout(const MatvecProblem& p, int mode, bool complex_elements,
   L.n_pat = t.n_pat;
   L.n_diag_blocks = d.slot_blocks;
   L.G = p.group.n_elems;
-  L.words = mode == kModeN32 ? (L.G + 7) / 8 * 8 : (L.G + 15) / 16 * 8;
-  L.stride = L.words + 1;  // odd: patterns (and rows) next to each other fall into different banks
+  const int n = p.group.n_bits, inv = p.group.spin_inversion != 0 ? 1 : 0;
+  if (mode == kModeN32) {
+    L.words = (L.G + 7) / 8 * 8;
+  } else {
+    L.planes = rows_planes(p);
+    L.nlow = n - inv - L.planes;
+    L.nlow_pad = (L.nlow + 3) / 4 * 4;
+    const int pw = L.nlow_pad / 4 + 1;  // and the top bit's source
+    L.perm_stride = 4 * (pw % 2 ? pw : pw + 1);
+    L.words = L.planes * mode;
+  }
+  L.stride = L.words | 1;  // odd: patterns (and rows) next to each other fall into different banks
   L.site_words = (L.words + 31) / 32 * 32;
-  L.nlow = mode == kModeP16 ? p.group.n_bits - 16 : 0;
-  const int pw = (L.nlow + 3) / 4;
-  L.nlow_pad = 4 * pw;
-  L.perm_stride = 4 * (pw % 2 ? pw : pw + 1);
   // a table beyond the shared memory of a CTA cannot fit (and would overflow the 32-bit offsets)
   const size_t big = (size_t)L.n_pat * L.stride * 4 + (size_t)t.n_cls * L.G * 16 * std::max(n_sectors, 1) +
                      (size_t)R * L.cap * 10;
@@ -81,7 +75,7 @@ static bool rows_layout(const MatvecProblem& p, int mode, bool complex_elements,
   L.off_coef = take((size_t)t.n_cls * L.G * (complex_elements ? 16 : 8) * std::max(n_sectors, 1));
   L.off_site = take((size_t)p.group.n_bits * L.site_words * 4);
   L.off_img = take((size_t)L.n_pat * L.stride * 4);
-  L.off_perm = take(mode == kModeP16 ? (size_t)L.G * L.perm_stride : 0);
+  L.off_perm = take((size_t)L.G * L.perm_stride);
   L.off_sm = take((size_t)32 * L.slot_blocks * state);
   L.off_sl1 = take((size_t)32 * L.slot_blocks * state);
   L.off_sl2 = take((size_t)32 * L.slot_blocks * state);
@@ -103,20 +97,36 @@ static bool rows_layout(const MatvecProblem& p, int mode, bool complex_elements,
   L.w_list = take((size_t)R * L.cap * 2);
   L.w_ent = take(keep ? (size_t)R * L.cap * 8 : 0);
   L.w_a = take((size_t)R * state);
+  L.w_sets = take(mode == kModeN32 ? 0 : (size_t)mode * 128);
   L.warp_bytes = o;
   L.total = L.off_warp + (uint32_t)warps * L.warp_bytes;
   *out = L;
   return L.total <= kRowsSmem;
 }
 
-// Modes that `p` can run in order of preference: N32 where the state fits 32 bits (whole states, no
-// second comparison), else, or when its pattern images do not fit, P16 (half the table, two
-// elements per word; at most 32 chunks of 16 elements in the scan's mask).
+// The scan modes, and which of them `p` can run.
+constexpr int kRowModes[] = {kModeN32, 2, 5, 9, 16};
 static bool rows_mode_allowed(const MatvecProblem& p, int mode) {
-  const int n = p.group.n_bits;
+  const int n = p.group.n_bits, W = (p.group.n_elems + 31) / 32;
   if (p.group.n_elems < 1 || !p.off.rows.ok || !p.diag.rows.ok) return false;
   if (p.group.fermionic && (p.group.gpl < 1 || p.group.gpl > 4)) return false;  // as the packed kernels
-  return mode == kModeN32 ? n <= 32 : n >= 17 && n <= 63 && p.group.n_elems <= 512;
+  if (mode == kModeN32) return n <= 32;
+  if (n < 2 || n > 63 || W > mode) return false;
+  for (const int m : kRowModes)
+    if (m != kModeN32 && m >= W) return m == mode;  // the smallest that holds the group
+  return false;
+}
+
+// About the instructions of one target's scan (32 targets at a time): the line between N32 and bit
+// planes.  150 elements on 25 sites: 137 us by N32, 125 by planes; 128 elements of the 4x4 Hubbard
+// model 2362 and 2764 us; 56 images of the 28-site chain 1544 and 1581 us; 28 elements of the ladder
+// 4.4 and 6.2 ms a training step.  Two species make many ties
+// among the top bits, which cost bit planes a round each.
+static double rows_scan_cost(const MatvecProblem& p, int mode) {
+  const int inv = p.group.spin_inversion != 0 ? 1 : 0;
+  if (mode == kModeN32) return (p.group.n_elems + 7) / 8 * 8 * (3.5 + inv) + 60.0;
+  const int planes = rows_planes(p);
+  return planes * (4.5 * mode + 5.0) + (p.constraint.kind == 2 ? 8.0 : 2.5) * (30.0 + 4.0 * (p.group.n_bits - planes));
 }
 
 constexpr int kLeastWarps = 4;
@@ -124,7 +134,7 @@ constexpr int kLeastWarps = 4;
 bool rows_fit(const MatvecProblem& p, int n_sectors) {
   RowsLayout L;
   if (p.projection != 2) return false;
-  for (const int m : {kModeN32, kModeP16})
+  for (const int m : kRowModes)
     if (rows_mode_allowed(p, m) && rows_layout(p, m, n_sectors > 0 || p.real_elements == 0, true, n_sectors, kLeastWarps, 1, &L)) return true;
   return false;
 }
@@ -133,16 +143,25 @@ bool rows_fit(const MatvecProblem& p, int n_sectors) {
 // their area.
 static bool rows_shape(const MatvecProblem& p, bool complex_elements, bool keep, int64_t n_rows, int n_sectors,
                        int max_warps, int sms, int* mode, RowsLayout* L) {
-  for (const int m : {kModeN32, kModeP16}) {
-    if (!rows_mode_allowed(p, m)) continue;
+  int modes[2], n_modes = 0;  // N32 and the group's bit planes, the cheaper scan first
+  for (const int m : kRowModes)
+    if (rows_mode_allowed(p, m)) modes[n_modes++] = m;
+  if (n_modes == 2 && rows_scan_cost(p, modes[1]) < rows_scan_cost(p, modes[0])) std::swap(modes[0], modes[1]);
+  for (int k = 0; k < n_modes; ++k) {
+    const int m = modes[k];
     RowsLayout t[4];
     int warps[4];
     for (int i = 0; i < 4; ++i) {
       rows_layout(p, m, complex_elements, keep, n_sectors, 1, 8 >> i, &t[i]);
-      const int64_t room = (int64_t)kRowsSmem - t[i].off_warp;
-      warps[i] = t[i].warp_bytes == 0 || room < 0 ? 0 : (int)std::min<int64_t>(max_warps, room / t[i].warp_bytes);
+      auto fit = [&](size_t limit) -> int {
+        const int64_t room = (int64_t)limit - t[i].off_warp;
+        const int w = t[i].warp_bytes == 0 || room < 0 ? 0 : (int)std::min<int64_t>(max_warps, room / t[i].warp_bytes);
+        return w >= 8 ? w / 4 * 4 : w;  // whole warps per scheduler
+      };
+      warps[i] = fit(kRowsSmem);
+      if (!keep && fit(kRowsSmemL1) >= 20) warps[i] = fit(kRowsSmemL1);
     }
-    for (const int enough : {24, 16, 8, kLeastWarps}) {
+    for (const int enough : {keep ? 24 : 20, 16, 8, kLeastWarps}) {
       int pick = -1;
       double least = 0.0;
       for (int i = 0; i < 4; ++i) {
@@ -215,32 +234,15 @@ int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int
   s.ldx = ldx;
   s.ldxs = p.xs != nullptr ? p.ldxs : ldx;
   s.ldy = ldy;
-  const RowsLayout& L = q.L;
-  const bool keep = s.cols > 1;
-  auto go = [&](auto kern) -> int {
-    if (!ensure_smem_limit((const void*)kern, L.total)) return LS_GPU_ERR_CUDA;
-    kern<<<(unsigned)q.blocks, L.threads, L.total, st>>>(p, L, s, d_err, binom);
-    return cuda_ok(cudaGetLastError(), "k_matvec_rows") ? 0 : LS_GPU_ERR_CUDA;
-  };
-  const bool inv = p.group.spin_inversion != 0;
-  auto with_col = [&](auto mtag, auto itag, auto ftag) -> int {
-    constexpr int M = decltype(mtag)::value;
-    constexpr bool I = decltype(itag)::value, F = decltype(ftag)::value;
-    if (col == kColReal) return go(k_matvec_rows<M, I, F, kColReal, false>);
-    if (col == kColPair)
-      return keep ? go(k_matvec_rows<M, I, F, kColPair, true>) : go(k_matvec_rows<M, I, F, kColPair, false>);
-    return keep ? go(k_matvec_rows<M, I, F, kColComplex, true>) : go(k_matvec_rows<M, I, F, kColComplex, false>);
-  };
-  auto with_mode = [&](auto mtag) -> int {
-    if (p.group.fermionic) {
-      if (inv) return fail(LS_GPU_ERR_INVALID, "fermionic groups have no spin inversion");
-      return with_col(mtag, std::false_type{}, std::true_type{});
-    }
-    return inv ? with_col(mtag, std::true_type{}, std::false_type{})
-               : with_col(mtag, std::false_type{}, std::false_type{});
-  };
-  return q.mode == kModeN32 ? with_mode(std::integral_constant<int, kModeN32>{})
-                          : with_mode(std::integral_constant<int, kModeP16>{});
+  switch (q.mode) {
+    case kModeN32: return launch_rows_mode<kModeN32>(p, q, col, d_err, binom, st);
+    case 2: return launch_rows_mode<2>(p, q, col, d_err, binom, st);
+    case 5: return launch_rows_mode<5>(p, q, col, d_err, binom, st);
+    case 9: return launch_rows_mode<9>(p, q, col, d_err, binom, st);
+    default: return launch_rows_mode<16>(p, q, col, d_err, binom, st);
+  }
 }
+
+template int launch_rows_mode<kModeN32>(const MatvecProblem&, const RowsLaunch&, int, int*, const uint64_t*, cudaStream_t);
 
 }  // namespace lsg

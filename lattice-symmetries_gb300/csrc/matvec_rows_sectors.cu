@@ -105,8 +105,12 @@ int launch_rows_sectors(const MatvecProblem& p, int k, int col, const SectorDesc
   auto with_inv = [&](auto mtag) -> int {
     return inv ? with_keep(mtag, std::true_type{}) : with_keep(mtag, std::false_type{});
   };
-  return q.mode == kModeN32 ? with_inv(std::integral_constant<int, kModeN32>{})
-                            : with_inv(std::integral_constant<int, kModeP16>{});
+  switch (q.mode) {  // groups of at most 128 elements
+    case kModeN32: return with_inv(std::integral_constant<int, kModeN32>{});
+    case 2: return with_inv(std::integral_constant<int, 2>{});
+    case 5: return with_inv(std::integral_constant<int, 5>{});
+    default: return fail(LS_GPU_ERR_INVALID, "sector batches: at most 128 group elements");
+  }
 }
 
 }  // namespace lsg

@@ -23,17 +23,23 @@
 // and neighbouring lanes read neighbouring patterns (few bank conflicts), and go to shared memory.
 //
 // Measured (GB300, warp per row -> lane per element): T x C6 on 25 sites, 150 elements, 34.7e3 rows, 5
-// complex columns 1328 -> 137 us (the ragged block also scans once instead of twice); 28-site
-// chain, 56 images, 16 columns 3609 -> 1538 us; 4x4 Hubbard, 128 elements, 8 columns 6724 ->
-// 2351 us; 6x6 torus, 576 images, one column 169.3 -> 85.2 ms.
+// complex columns 1328 -> 125 us (the ragged block also scans once instead of twice; 137 us with N32);
+// 28-site chain, 56 images, 16 columns 3609 -> 1540 us; 4x4 Hubbard, 128 elements, 8 columns 6724 ->
+// 2358 us; 6x6 torus, 576 images, one column 169.1 -> 73.5 ms (85.2 ms with prefix minima instead of
+// bit planes).
 //
 // Modes.  N32 (states of at most 32 bits): candidates are whole states, so their minimum is the
 // representative; the scan remembers the chunk of 8 elements that first reached it and a second
-// look at that chunk finds the element.  P16 (any width from 17 bits; used when the N32 tables do
-// not fit or the group is large): candidates are the top 16 bits of the states, two elements per
-// 32-bit word, so that loads, XORs and minima cover two elements each; the chunks of 16 elements
-// that reach the minimal prefix are kept as a bit mask and their matching elements (usually one)
-// are compared by their remaining bits, gathered through a byte table of source positions.
+// look at that chunk finds the element.
+// Bit planes (any width; large groups): for each of the top positions of the image one bit per
+// group element, 32 elements to a word -- linear over XOR like the images themselves, so the same
+// row and pattern tables hold them.  A lane keeps the set of elements that can still be minimal (W
+// words in registers) and goes down the positions: where some of them have a 0 there, those stay.
+// With spin inversion the planes are taken relative to the top position's, which flips every image
+// to its smaller form.  That is one XOR-AND, half an OR and a select per word and position, for about
+// log2 |G| + 4 positions (13 x 9 words for 288 elements, where a minimum over 16-bit prefixes
+// took 144 words at three operations and half-word bookkeeping); the one or two elements left are
+// compared by their remaining bits, gathered through a byte table of source positions.
 //
 // The order of the tie-break (lowest element, unflipped first) is that of the packed kernels.
 #pragma once
@@ -42,34 +48,27 @@
 
 namespace lsg {
 
-constexpr int kModeN32 = 0, kModeP16 = 1;
-// Elements that a lane takes at a time (6x6 torus, one column: 1 / 2 / 4 at a time 86.4 / 85.2 / 98 ms;
-// 4x4 Hubbard, 8 columns: 1 / 2 / 4 at a time 2444 / 2534 / 3600 us).
-template <bool KEEP>
-constexpr int kLaneElements = KEEP ? 1 : 2;
+// Scan modes: N32, or bit planes of W words per position (W the mode's value).
+constexpr int kModeN32 = 0;
+// Elements that a lane takes at a time (6x6 torus, one column: 2 against 1 is 85.2 against 86.4 ms; 4x4
+// Hubbard, 8 columns: 1 / 2 / 4 at a time 2444 / 2534 / 3600 us); the sets of two elements on planes
+// of 16 words do not fit the registers.
+template <int MODE, bool KEEP>
+constexpr int kLaneElements = KEEP || MODE > 9 ? 1 : 2;
 
 // Shared-memory layout and shape of a row-group kernel (bytes from the start of dynamic shared
 // memory; w_* relative to a warp's area).
 struct RowsLayout {
   int threads, R, lanes_per_row, lane_shift, cap, T, n_slots, slot_blocks, n_pat, n_diag_blocks;
   int G, words, stride, site_words;  // words of g-images per row / pattern, their padded strides
-  int nlow, nlow_pad, perm_stride;   // P16: bits below the 16-bit prefix, rounded up to 4, bytes per element
+  int planes, nlow, nlow_pad, perm_stride;  // bit planes: positions, bits below them, rounded up to 4, bytes
+                                            // of an element's source positions
   uint32_t off_site, off_img, off_perm, off_coef, off_sm, off_sl1, off_sl2, off_st, off_ti, off_ts, off_xm;
   uint32_t off_dm, off_dr, off_ds, off_db, off_dv, off_fs, off_sectors, off_first, off_warp;
-  uint32_t warp_bytes, w_ent, w_list, w_a;  // w_list: KEEP the elements' positions in scan order
+  uint32_t warp_bytes, w_ent, w_list, w_a, w_sets;  // w_list: KEEP the elements' positions in scan order
   uint32_t total;
 };
 
-__device__ __forceinline__ uint32_t vmin2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-__device__ __forceinline__ uint32_t vmax2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
 __device__ __forceinline__ uint64_t shfl_u64(uint64_t v, int src) {
   return ((uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(v >> 32), src) << 32) |
          __shfl_sync(0xffffffffu, (uint32_t)v, src);
@@ -105,6 +104,7 @@ struct RowGroup {
   uint16_t* list;     // [R][cap]: the terms of each row's elements; KEEP: positions in entries, in scan order
   uint2* entries;     // KEEP: [R][cap], {term | row << 16, -} when listed, {column, coefficient word} resolved
   State* rows;        // [R] row states
+  uint32_t* sets;     // bit planes: [W][32] the lanes' sets of minimal elements
   uint32_t img_s, ga_s;
   int lane;
   State prev;         // state whose images are in row `prev_row` of ga
@@ -124,6 +124,7 @@ struct RowGroup {
     entries = (uint2*)(w + L.w_ent);
     list = (uint16_t*)(w + L.w_list);
     rows = (State*)(w + L.w_a);
+    sets = (uint32_t*)(w + L.w_sets) + (threadIdx.x & 31);
     img_s = (uint32_t)__cvta_generic_to_shared(s + L.off_img);
     ga_s = (uint32_t)__cvta_generic_to_shared(ga);
     lane = threadIdx.x & 31;
@@ -149,20 +150,31 @@ struct RowGroup {
       if constexpr (MODE == kModeN32) {
         site[i] = w < L.words ? (uint32_t)__ldg(r + (w < G ? w : 0)) : 0u;
       } else {
-        const uint64_t v0 = __ldg(r + (2 * w < G ? 2 * w : 0)), v1 = __ldg(r + (2 * w + 1 < G ? 2 * w + 1 : 0));
-        site[i] = w < L.words ? (uint32_t)(v0 >> (nb - 16)) | ((uint32_t)(v1 >> (nb - 16)) << 16) : 0u;
+        // which of the word's 32 elements move site b to the plane's position (or, with spin
+        // inversion, to the top)
+        const int top = nb - 1, pos = top - w / MODE - (INV ? 1 : 0), g0 = 32 * (w % MODE);
+        uint32_t v = 0;
+        if (w < L.words)
+          for (int i32 = 0; i32 < 32 && g0 + i32 < G; ++i32) {
+            const uint64_t image = __ldg(r + g0 + i32);
+            const uint32_t bit = (uint32_t)(image >> pos) ^ (INV ? (uint32_t)(image >> top) : 0u);
+            v |= (bit & 1u) << i32;
+          }
+        site[i] = v;
       }
     }
-    if constexpr (MODE == kModeP16) {
+    if constexpr (MODE != kModeN32) {
       // source positions of an element's low bits, most significant first, after bits that are zero
       // in every state (position 63)
       unsigned char* perm = smem + L.off_perm;
+      // and, last, of its top bit
       const int pad = L.nlow_pad - L.nlow;
       for (int i = tid; i < G * pad; i += nt) perm[(i / pad) * L.perm_stride + i % pad] = 63;
       for (int i = tid; i < nb * G; i += nt) {
         const int b = i / G, g = i - b * G;
         const int to = __ffsll((long long)__ldg(p.group.onehot + i)) - 1;
         if (to < L.nlow) perm[g * L.perm_stride + (L.nlow_pad - 1 - to)] = (unsigned char)b;
+        if (to == nb - 1) perm[g * L.perm_stride + L.nlow_pad] = (unsigned char)b;
       }
     }
     auto states = [&](uint32_t off, const uint64_t* src, int n) {
@@ -224,6 +236,7 @@ struct RowGroup {
     if (lane < nr) rows[lane] = a_l;
     const uint32_t site_s = (uint32_t)__cvta_generic_to_shared(smem + L.off_site) + 4u * (uint32_t)lane;
     const uint32_t row_bytes = 4u * (uint32_t)L.site_words;
+#pragma unroll 1
     for (int r = 0; r < nr; ++r) {
       const State a = shfl_state(a_l, r);
       const State diff = a ^ prev;
@@ -238,6 +251,8 @@ struct RowGroup {
           for (int k = 0; k < 4; ++k) v[k] = lane + 32 * k < left ? g[32 * k] : 0u;
         }
         const uint32_t base = site_s + 4u * (uint32_t)w0;
+        
+#pragma unroll 1
         for (State d = diff; d != 0;) {
           const uint32_t s0 = base + (uint32_t)low_bit(d) * row_bytes;
           d &= d - 1;
@@ -264,6 +279,7 @@ struct RowGroup {
       const State m = tab<State>(L.off_sm)[32 * b + lane];
       const State l1 = tab<State>(L.off_sl1)[32 * b + lane], l2 = tab<State>(L.off_sl2)[32 * b + lane];
       const uint32_t t12 = tab<uint32_t>(L.off_st)[32 * b + lane];
+#pragma unroll 1
       for (int r = 0; r < nr; ++r) {
         const State x = shfl_state(a_l, r) & m;
         const bool h1 = x == l1, h2 = x == l2;
@@ -287,30 +303,34 @@ struct RowGroup {
     __syncwarp();
   }
 
-  // Pass 1 for E elements: images of their rows at gp (one row without KEEP), of their patterns at ip.  N32: the
-  // minimum and the word of its first chunk; P16: the minimal prefix and the mask of its chunks.
+  // What pass 1 leaves for pass 2 of an element.  N32: the minimum and the word of its first chunk;
+  // bit planes: the top bits of the minimum and the elements that have them.
+  struct Found {
+    uint32_t best, at;
+    uint32_t set[MODE == kModeN32 ? 1 : MODE];
+  };
+
+  // Pass 1 for E elements: images of their rows at gp (one row without KEEP), of their patterns at ip.
   template <int E>
-  __device__ __forceinline__ void first_pass(const uint32_t (&gp)[E], const uint32_t (&ip)[E], uint32_t (&best)[E],
-                                             uint32_t (&at)[E]) const {
-    const uint32_t flip = (uint32_t)p.group.flip;
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      best[e] = MODE == kModeN32 ? 0xffffffffu : 0x10000u;
-      at[e] = 0;
-    }
-    uint32_t bit = 1;
-    for (uint32_t c = 0; c < (uint32_t)L.words; c += 8, bit <<= 1) {
-      uint32_t a[8];
+  __device__ __forceinline__ void first_pass(const uint32_t (&gp)[E], const uint32_t (&ip)[E], Found (&found)[E]) const {
+    if constexpr (MODE == kModeN32) {
+      const uint32_t flip = (uint32_t)p.group.flip;
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        if (KEEP || e == 0) {
+        found[e].best = 0xffffffffu;
+        found[e].at = 0;
+      }
+      for (uint32_t c = 0; c < (uint32_t)L.words; c += 8) {
+        uint32_t a[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) a[k] = lds_u32_volatile(gp[e] + 4 * (c + k));
-        }
-        uint32_t h[8];
+        for (int e = 0; e < E; ++e) {
+          if (KEEP || e == 0) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) h[k] = a[k] ^ lds_u32(ip[e] + 4 * (c + k));
-        if constexpr (MODE == kModeN32) {
+            for (int k = 0; k < 8; ++k) a[k] = lds_u32_volatile(gp[e] + 4 * (c + k));
+          }
+          uint32_t h[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) h[k] = a[k] ^ lds_u32(ip[e] + 4 * (c + k));
           uint32_t mn = h[0], mx = h[0];
 #pragma unroll
           for (int k = 1; k < 8; ++k) {
@@ -318,94 +338,113 @@ struct RowGroup {
             if (INV) mx = max(mx, h[k]);
           }
           if (INV) mn = min(mn, flip ^ mx);
-          if (mn < best[e]) {
-            best[e] = mn;
-            at[e] = c;
+          if (mn < found[e].best) {
+            found[e].best = mn;
+            found[e].at = c;
           }
-        } else {
-          uint32_t mn = h[0], mx = h[0];
+        }
+      }
+    } else {
+      constexpr int W = MODE;
 #pragma unroll
-          for (int k = 1; k < 8; ++k) {
-            mn = vmin2(mn, h[k]);
-            if (INV) mx = vmax2(mx, h[k]);
+      for (int e = 0; e < E; ++e) {
+        found[e].best = 0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const int left = L.G - 32 * w;
+          found[e].set[w] = left >= 32 ? ~0u : (left > 0 ? (1u << left) - 1u : 0u);
+        }
+      }
+#pragma unroll 1  // (the instruction cache)
+      for (int q = 0; q < L.planes; ++q) {
+        uint32_t a[W];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          if (KEEP || e == 0) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) a[w] = lds_u32_volatile(gp[e] + 4 * (q * W + w));
           }
-          if (INV) mn = vmin2(mn, ~mx);
-          const uint32_t m = min(mn & 0xffffu, mn >> 16);
-          at[e] = m < best[e] ? bit : (m == best[e] ? at[e] | bit : at[e]);
-          best[e] = min(best[e], m);
+          uint32_t z[W], any = 0;  // the elements with a 0 here
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            z[w] = found[e].set[w] & ~(a[w] ^ lds_u32(ip[e] + 4 * (q * W + w)));
+            any |= z[w];
+          }
+#pragma unroll
+          for (int w = 0; w < W; ++w) found[e].set[w] = any != 0 ? z[w] : found[e].set[w];
+          found[e].best = 2 * found[e].best + (any != 0 ? 0u : 1u);
         }
       }
     }
   }
 
   // The representative of one element and its key 2 * group element + flipped, from pass 1.
-  __device__ __forceinline__ uint64_t second_pass(uint32_t gp, uint32_t ip, uint32_t best, uint32_t mask,
-                                                  uint64_t beta, uint32_t* key) const {
+  __device__ __forceinline__ uint64_t second_pass(uint32_t gp, uint32_t ip, const Found& found, uint64_t beta,
+                                                  uint32_t* key) const {
     if constexpr (MODE == kModeN32) {
       const uint32_t flip = (uint32_t)p.group.flip;
-      const uint32_t at = mask;
+      const uint32_t at = found.at;
       uint32_t k0 = 0;
 #pragma unroll
       for (int k = 7; k >= 0; --k) {
         const uint32_t h = lds_u32_volatile(gp + 4 * (at + k)) ^ lds_u32(ip + 4 * (at + k));
-        if (INV && (h ^ flip) == best) k0 = 2 * k + 1;
-        if (h == best) k0 = 2 * k;
+        if (INV && (h ^ flip) == found.best) k0 = 2 * k + 1;
+        if (h == found.best) k0 = 2 * k;
       }
       *key = 2 * at + k0;
-      return best;
+      return found.best;
     } else {
-      // the elements of the marked chunks that reach the prefix, compared by their low bits (6x6
-      // torus: 1.08 elements per target reach it, the slowest of 32 lanes has 2.1)
-      const uint32_t two = best * 0x10001u;
-      uint32_t found = 0;  // words of the chunk at `at`: bit k its even element, bit 16 + k its odd one
-      uint32_t at = 0, win = 0;
+      // the remaining elements compared by their low bits (6x6 torus, 13 planes: 1.15 per target,
+      // the slowest of 32 lanes has 2.5)
+      uint32_t words = 0;  // of the set that are not empty
+#pragma unroll
+      for (int w = 0; w < MODE; ++w) {
+        sets[32 * w] = found.set[w];
+        if (found.set[w] != 0) words |= 1u << w;
+      }
+      uint32_t word = 0, base = 0, win = 0;
       uint64_t low = ~0ull;
       const uint32_t perm_s = (uint32_t)__cvta_generic_to_shared(smem + L.off_perm);
+#pragma unroll 1
       do {
-        if (found == 0 && mask != 0) {
-          at = (uint32_t)(__ffs(mask) - 1) * 8u;
-          mask &= mask - 1;
-          uint32_t other = 0;  // halves that miss the prefix
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            uint32_t d = lds_u32_volatile(gp + 4 * (at + k)) ^ lds_u32(ip + 4 * (at + k)) ^ two;
-            if (INV) d = vmin2(d, ~d);
-            other += vmin2(d, 0x10001u) << k;
-          }
-          found = ~other & 0xff00ffu;
+        if (word == 0 && words != 0) {
+          base = (uint32_t)__ffs(words) - 1;
+          words &= words - 1;
+          word = sets[32 * base];
         }
-        if (found != 0) {
-          const uint32_t f = (uint32_t)__ffs(found) - 1;
-          found &= found - 1;
-          const uint32_t w = at + (f & 15u), half = f >> 4;
-          const uint32_t h = lds_u32_volatile(gp + 4 * w) ^ lds_u32(ip + 4 * w);
-          const bool flipped = INV && ((h >> (16 * half)) & 0xffffu) != best;
-          uint32_t g = 2 * w + half;
-          if (g >= (uint32_t)L.G) g = 0;  // padding repeats element 0
+        if (word != 0) {
+          const uint32_t g = 32 * base + (uint32_t)__ffs(word) - 1;
+          word &= word - 1;
           const uint32_t ps = perm_s + g * (uint32_t)L.perm_stride;
           uint32_t hi = 0, lo = 0;  // the low bits, most significant first
           int b = 0;
+#pragma unroll 1
           for (; b < L.nlow_pad - 32; b += 4) {
             const uint32_t src = lds_u32(ps + b);
 #pragma unroll
             for (int i = 0; i < 4; ++i) hi = 2 * hi + ((uint32_t)(beta >> __byte_perm(src, 0, 0x4440 + i)) & 1u);
           }
+#pragma unroll 1
           for (; b < L.nlow_pad; b += 4) {
             const uint32_t src = lds_u32(ps + b);
 #pragma unroll
             for (int i = 0; i < 4; ++i) lo = 2 * lo + ((uint32_t)(beta >> __byte_perm(src, 0, 0x4440 + i)) & 1u);
           }
           uint64_t v = ((uint64_t)hi << 32) | lo;
-          if (flipped) v ^= (1ull << L.nlow) - 1;
-          const uint32_t mine = 2 * g + (flipped ? 1u : 0u);
-          if (v < low || (v == low && mine < win)) {
+          uint32_t flipped = 0;
+          if (INV) {
+            flipped = (uint32_t)(beta >> (lds_u32(ps + L.nlow_pad) & 0xffu)) & 1u;
+            if (flipped) v ^= (1ull << L.nlow) - 1;
+          }
+          // elements ascend: the first of equal images stays
+          if (v < low) {
             low = v;
-            win = mine;
+            win = 2 * g + flipped;
           }
         }
-      } while (__any_sync(FULL, (found | mask) != 0));
+      } while (__any_sync(FULL, (word | words) != 0));
       *key = win;
-      return ((uint64_t)best << L.nlow) | low;
+      return ((uint64_t)found.best << L.nlow) | low;
     }
   }
 
@@ -427,6 +466,7 @@ struct RowGroup {
       const uint32_t low = (1u << ix.shift) - 1u;
 #pragma unroll
       for (int e = 0; e < E; ++e) longest = max(longest, n[e]);
+#pragma unroll 1
       while (longest > 1) {
         longest = 0;
 #pragma unroll
@@ -461,20 +501,21 @@ struct RowGroup {
                                                uint32_t (&w)[E], int* __restrict__ err,
                                                const uint64_t* __restrict__ binom) {
     const uint32_t stride = 4u * (uint32_t)L.stride;
-    uint32_t gp[E], ip[E], best[E], at[E];
+    uint32_t gp[E], ip[E];
+    Found found[E];
     uint64_t rep[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       gp[e] = ga_s + row[e] * stride;
       ip[e] = img_s + (tab<uint32_t>(L.off_ti)[term[e]] & 0xffffu) * stride;
     }
-    first_pass<E>(gp, ip, best, at);
+    first_pass<E>(gp, ip, found);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const uint32_t info = tab<uint32_t>(L.off_ti)[term[e]];
       const State beta = rows[row[e]] ^ tab<State>(L.off_xm)[info & 0xffffu];
       uint32_t key;
-      rep[e] = second_pass(gp[e], ip[e], best[e], at[e], beta, &key);
+      rep[e] = second_pass(gp[e], ip[e], found[e], beta, &key);
       if (ok[e] && (info & kRowTermNeedsCheck) && !constraint_ok(p.constraint, beta)) {
         ok[e] = false;
         atomicOr(err, 1);
@@ -494,7 +535,7 @@ struct RowGroup {
   template <typename Take>
   __device__ __forceinline__ void resolve(const DeviceIndex& ix, int* __restrict__ err,
                                           const uint64_t* __restrict__ binom, Take&& take) {
-    constexpr int E = kLaneElements<KEEP>;
+    constexpr int E = kLaneElements<MODE, KEEP>;
     const int r = lane >> L.lane_shift, sub = lane & (L.lanes_per_row - 1);
     const int cnt = __shfl_sync(FULL, cnt_l, r);
     const int most = (int)__reduce_max_sync(FULL, (unsigned)cnt);
@@ -516,7 +557,7 @@ struct RowGroup {
   // Step 3 with KEEP: the resolved elements replace the listed ones in entries.
   __device__ __forceinline__ void resolve(const DeviceIndex& ix, int* __restrict__ err,
                                           const uint64_t* __restrict__ binom) {
-    constexpr int E = kLaneElements<KEEP>;
+    constexpr int E = kLaneElements<MODE, KEEP>;
     for (int s = 0; s < total; s += 32 * E) {
       uint32_t at[E], row[E], term[E], j[E], w[E];
       bool ok[E];
@@ -547,6 +588,7 @@ struct RowGroup {
       const State m = tab<State>(L.off_dm)[32 * b + lane], k = tab<State>(L.off_dr)[32 * b + lane];
       const State s = tab<State>(L.off_ds)[32 * b + lane];
       const uint2 info = tab<uint2>(L.off_db)[b];  // {signs of the 32 terms, class | last block of it << 31}
+#pragma unroll 1
       for (int r = 0; r < nr; ++r) {
         const State a = shfl_state(a_l, r);
         const bool hit = (a & m) == k;

@@ -216,5 +216,9 @@ struct RowsLaunch {
 // max_threads 0: the matvec kernels' own.
 bool rows_plan(const MatvecProblem& p, int col, int k, int64_t n_rows, int n_sectors, RowsLaunch* out,
                int max_threads = 0);
+// Launches a plan of this scan mode (rowkernel.cuh).
+template <int MODE>
+int launch_rows_mode(const MatvecProblem& p, const RowsLaunch& q, int col, int* d_err, const uint64_t* binom,
+                     cudaStream_t st);
 
 }  // namespace lsg
