@@ -1174,7 +1174,16 @@ RowTables off_diag_rows(const TermTable& t, const DeviceConstraint& cons, const 
   R.sl2.resize(R.sm.size(), 1);
   R.st.resize(R.sm.size(), 0);
   R.shape.n_pat = (int)R.xmask.size();
-  for (int k = 0; k < t.n; ++k) R.shape.any_sign |= t.s[k] != 0;
+  for (int k = 0; k < t.n; ++k) {
+    R.shape.any_sign |= t.s[k] != 0;
+    R.shape.any_check |= (R.tinfo[k] & kRowTermNeedsCheck) != 0;
+  }
+  R.shape.two_site = 1;
+  for (int k = 0; k < R.shape.n_slots; ++k) {
+    const int sites = __builtin_popcountll(R.sm[k]);
+    // (a pattern with bits outside its mask never matches: one by one)
+    if (sites < 1 || sites > 2 || ((R.sl1[k] | R.sl2[k]) & ~R.sm[k])) R.shape.two_site = 0;
+  }
   R.shape.ok = 1;
   return R;
 }
@@ -1202,7 +1211,12 @@ RowTables diag_rows(const TermTable& t, const int32_t* coupling) {
         if (k >= 0 && members[c][b + i].second) signs |= 1u << i;
       }
       R.st.push_back(signs);
-      R.tinfo.push_back((uint32_t)c | ((uint32_t)n << 16) | (b + 32 >= members[c].size() ? 1u << 31 : 0u));
+      bool free_of_masks = true;
+      for (size_t i = 0; i < n; ++i) {
+        const int k = members[c][b + i].first;
+        free_of_masks = free_of_masks && t.m[k] == 0 && t.r[k] == 0;
+      }
+      R.tinfo.push_back((uint32_t)c | ((uint32_t)n << 16) | (free_of_masks ? 1u << 30 : 0u) | (b + 32 >= members[c].size() ? 1u << 31 : 0u));
     }
   }
   R.shape.slot_blocks = (int)R.st.size();
@@ -1420,12 +1434,17 @@ int make_problem(ls_hs_operator const* op, bool adjoint, MatvecProblem* p) {
   return 0;
 }
 
+// One pinned read and one synchronisation; the word is cleared only when it is set.
 int read_and_clear_error(cudaStream_t s) {
-  int h[4] = {0, 0, 0, 0};
+  int* h = (int*)pinned_scratch(4 * sizeof(int), 11);
   int* d = device_error_word();
-  if (!cuda_ok(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s), "read error word") ||
-      !cuda_ok(cudaMemsetAsync(d, 0, sizeof(h), s), "clear error word") ||
+  if (h == nullptr) return LS_GPU_ERR_CUDA;
+  if (!cuda_ok(cudaMemcpyAsync(h, d, 4 * sizeof(int), cudaMemcpyDeviceToHost, s), "read error word") ||
       !cuda_ok(cudaStreamSynchronize(s), "matvec"))
+    return LS_GPU_ERR_CUDA;
+  if ((h[0] | h[1] | h[2] | h[3]) != 0 &&
+      (!cuda_ok(cudaMemsetAsync(d, 0, 4 * sizeof(int), s), "clear error word") ||
+       !cuda_ok(cudaStreamSynchronize(s), "matvec")))
     return LS_GPU_ERR_CUDA;
   if (h[0] != 0)
     return fail(LS_GPU_ERR_BASIS,

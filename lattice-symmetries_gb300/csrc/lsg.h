@@ -115,10 +115,11 @@ struct DeviceRowTerms {
   const uint32_t* st = nullptr;    // terms of the patterns, first | second << 16 (diagonal: per
                                    // block, the signs of its 32 terms)
   const uint32_t* tinfo = nullptr;  // [terms] pattern | class << 16 | check << 30 | sign << 31
-                                    // (diagonal: per block, class | terms << 16 | last block of the
-                                    // class << 31)
+                                    // (diagonal: per block, class | terms << 16 | no masks << 30 | last
+                                    // block of the class << 31)
   int n_pat = 0, n_cls = 0;
-  int any_sign = 0;                // some off-diagonal term has a sign mask
+  int any_sign = 0, any_check = 0;  // some off-diagonal term has a sign mask / may leave the basis
+  int two_site = 0;                // every off-diagonal slot's mask has one or two sites
   const uint64_t* xmask = nullptr;  // [n_pat] flip masks
   const double2* cval = nullptr;    // [n_cls]
   // Coupling products: [n_cls] the sum that a class goes to -- its coupling, or, merged, the class

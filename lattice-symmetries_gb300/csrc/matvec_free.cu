@@ -7,15 +7,20 @@
 // reads (in shared memory up to 26 bits) in place of a walk over the set bits through a binomial
 // table or a search.  (N_up, N_down) has the same form with one table per species.
 //
-// Rows.  One thread per row and column.  A thread first tests the term slots (two exclusive patterns
-// per slot, DeviceRowTerms) into a bit mask and then takes its set bits, four gathers at a time, so
-// that lanes with other matches do not idle on a term that is not theirs; all columns of a row
-// share a warp.
+// Rows.  One thread per row and column.  A thread first matches the term slots (two exclusive patterns
+// per slot, DeviceRowTerms) into a bit mask, 32 slots at once: the state's bit at the first (second)
+// site of every slot is an XOR of table words over the state's nibbles, and so are the parities of
+// 32 diagonal terms.  (Slots on more than two sites are tested one by one.)  It then takes the mask's
+// set bits, four gathers at a time, so that lanes with other matches do not idle on a term that is
+// not theirs.  The bits are taken from
+// the top: neighbouring rows agree in their high sites, so their lanes meet the same terms there and
+// read neighbouring entries of x.  All columns of a row share a warp.
 //
 // The FP64 pipe (1 FMA per element for real vectors, 2 or 4 per complex column) and the loads bound
 // it.  Measured (GB300, one thread per row with a binomial walk or a search per element, every column on
-// its own -> here): 24 spins, weight 12 (2.7e6 rows), one real vector 1345 -> 178 us; 12-site
-// Hubbard, 6 + 6 fermions (8.5e5 rows), 4 complex columns 1380 -> 261 us.
+// its own -> here): 24 spins, weight 12 (2.7e6 rows), one real vector 1345 -> 122 us (178 us
+// with slots and diagonal terms tested one by one); 12-site Hubbard, 6 + 6 fermions (8.5e5 rows), 4
+// complex columns 1380 -> 250 us.
 #include <algorithm>
 
 #include "matvec_launch.cuh"
@@ -28,10 +33,28 @@ extern const uint64_t* device_binomials();
 constexpr int kFreeThreads = 512;
 constexpr size_t kFreeSmem = 112 * 1024;  // two CTAs per SM
 
+// A slot as the kernel reads it: mask, the two patterns, their terms (first | second << 16).
+template <typename State>
+struct alignas(sizeof(State) == 4 ? 16 : 32) FreeSlot {
+  State m, l1, l2;
+  uint32_t terms;
+};
+template <typename State>
+struct alignas(2 * sizeof(State)) FreeTerm {
+  State x;
+  uint32_t info;
+};
+
+// 32 slots at once: the bits that the two patterns want at the slots' first and second sites.
+struct FreeWant {
+  uint32_t first1, second1, first2, second2;  // pattern 1, pattern 2
+  uint32_t valid;
+};
+
 struct FreeLayout {
-  int T, n_slots, n_diag_blocks, signs, tables_in_smem;
-  uint32_t off_tlo, off_thi, off_coef, off_sm, off_sl1, off_sl2, off_st, off_ti, off_ts, off_tx, off_dm, off_dr, off_ds,
-      off_db, off_dv;
+  int T, n_slots, n_diag_blocks, signs, checks, planes, tables_in_smem;
+  int nibbles;
+  uint32_t off_tlo, off_thi, off_coef, off_slots, off_terms, off_ts, off_want, off_first, off_second, off_parity, off_dm, off_dr, off_ds, off_db, off_dv;
   uint32_t total;
   int cols, rows_per_warp;
 };
@@ -93,13 +116,19 @@ __global__ void __launch_bounds__(kFreeThreads, 2)
     words(L.off_tlo, p.index.rank_lo, 1 << split);
     words(L.off_thi, p.index.rank_hi, 1 << high_bits);
   }
-  states(L.off_sm, p.off.rows.sm, L.n_slots);
-  states(L.off_sl1, p.off.rows.sl1, L.n_slots);
-  states(L.off_sl2, p.off.rows.sl2, L.n_slots);
-  words(L.off_st, p.off.rows.st, L.n_slots);
-  words(L.off_ti, p.off.rows.tinfo, L.T);
+  FreeSlot<State>* slots = (FreeSlot<State>*)(smem + L.off_slots);
+  for (int i = tid; i < L.n_slots; i += nt)
+    slots[i] = {(State)__ldg(p.off.rows.sm + i), (State)__ldg(p.off.rows.sl1 + i), (State)__ldg(p.off.rows.sl2 + i),
+                __ldg(p.off.rows.st + i)};
+  FreeTerm<State>* terms = (FreeTerm<State>*)(smem + L.off_terms);
+  for (int i = tid; i < L.T; i += nt) terms[i] = {(State)__ldg(p.off.x + i), __ldg(p.off.rows.tinfo + i)};
   states(L.off_ts, p.off.s, L.T);
-  states(L.off_tx, p.off.x, L.T);
+  const int slot_blocks = (L.n_slots + 31) / 32;
+  uint32_t* first_lut = (uint32_t*)(smem + L.off_first);    // [block][nibble][16]
+  uint32_t* second_lut = (uint32_t*)(smem + L.off_second);
+  uint32_t* parity_lut = (uint32_t*)(smem + L.off_parity);  // [diagonal block][nibble][16]
+  FreeWant* want = (FreeWant*)(smem + L.off_want);
+  const int per_block = 16 * L.nibbles;
   states(L.off_dm, p.diag.rows.sm, 32 * L.n_diag_blocks);
   states(L.off_dr, p.diag.rows.sl1, 32 * L.n_diag_blocks);
   states(L.off_ds, p.diag.rows.sl2, 32 * L.n_diag_blocks);
@@ -107,20 +136,55 @@ __global__ void __launch_bounds__(kFreeThreads, 2)
   for (int i = tid; i < L.n_diag_blocks; i += nt)
     db[i] = make_uint2(__ldg(p.diag.rows.st + i), __ldg(p.diag.rows.tinfo + i));
   stage_d2((double2*)(smem + L.off_dv), p.diag.rows.cval, p.diag.rows.n_cls);
-  C* coef = (C*)(smem + L.off_coef);
-  for (int i = tid; i < p.off.rows.n_cls; i += nt) {
-    const double2 v = __ldg(p.off.rows.cval + i);
+  C* coef = (C*)(smem + L.off_coef);  // per term, with its sign
+  for (int i = tid; i < L.T; i += nt) {
+    const uint32_t info = __ldg(p.off.rows.tinfo + i);
+    const double2 v = flip_sign(__ldg(p.off.rows.cval + ((info >> 16) & 0xffu)), info & 0x80000000u);
     if constexpr (COL == kColComplex) coef[i] = v;
     else coef[i] = v.x;
   }
   __syncthreads();
-  const State* sm = (const State*)(smem + L.off_sm);
-  const State* sl1 = (const State*)(smem + L.off_sl1);
-  const State* sl2 = (const State*)(smem + L.off_sl2);
-  const uint32_t* st = (const uint32_t*)(smem + L.off_st);
-  const uint32_t* ti = (const uint32_t*)(smem + L.off_ti);
+  const State* ds = (const State*)(smem + L.off_ds);
+  if (L.planes) {
+    for (int i = tid; i < slot_blocks * per_block; i += nt) {
+      const int blk = i / per_block, at = (i - blk * per_block) >> 4;
+      const State v = (State)((uint64_t)(i & 15) << (4 * at));
+      uint32_t f = 0, g = 0;
+      for (int k = 32 * blk; k < min(32 * blk + 32, L.n_slots); ++k) {
+        const State m = slots[k].m;
+        const State lowest = m & (0 - m);
+        if (v & lowest) f |= 1u << (k & 31);
+        const State highest = m ^ lowest ? m ^ lowest : m;  // one-site slots: the same site
+        if (v & highest) g |= 1u << (k & 31);
+      }
+      first_lut[i] = f;
+      second_lut[i] = g;
+    }
+    for (int blk = tid; blk < slot_blocks; blk += nt) {
+      FreeWant w{0, 0, 0, 0, 0};
+      for (int k = 32 * blk; k < min(32 * blk + 32, L.n_slots); ++k) {
+        const State m = slots[k].m, l1 = slots[k].l1, l2 = slots[k].l2;
+        const State lowest = m & (0 - m), highest = m ^ lowest ? m ^ lowest : m;
+        const uint32_t bit = 1u << (k & 31);
+        w.valid |= bit;
+        if (l1 & lowest) w.first1 |= bit;
+        if (l1 & highest) w.second1 |= bit;
+        if (l2 & lowest) w.first2 |= bit;
+        if (l2 & highest) w.second2 |= bit;
+      }
+      want[blk] = w;
+    }
+  }
+  for (int i = tid; i < L.n_diag_blocks * per_block; i += nt) {
+    const int blk = i / per_block, at = (i - blk * per_block) >> 4;
+    const State v = (State)((uint64_t)(i & 15) << (4 * at));
+    uint32_t f = 0;
+    for (int k = 0; k < 32; ++k)
+      if (popc_state((State)(v & ds[32 * blk + k])) & 1) f |= 1u << k;
+    parity_lut[i] = f;
+  }
+  __syncthreads();
   const State* ts = (const State*)(smem + L.off_ts);
-  const State* tx = (const State*)(smem + L.off_tx);
   const uint32_t* lo = L.tables_in_smem ? (const uint32_t*)(smem + L.off_tlo) : p.index.rank_lo;
   const uint32_t* hi = L.tables_in_smem ? (const uint32_t*)(smem + L.off_thi) : p.index.rank_hi;
   const State low_mask = (State)(((uint64_t)1 << split) - 1), flip = (State)p.group.flip;
@@ -136,13 +200,28 @@ __global__ void __launch_bounds__(kFreeThreads, 2)
        row += warps * L.rows_per_warp) {
     const State a = identity ? (State)row : (State)__ldg(p.index.reps + row);
     V acc = Col::zero();
-    for (int s0 = 0; s0 < L.n_slots; s0 += 32) {
-      const int n = min(32, L.n_slots - s0);
+    for (int s0 = (L.n_slots - 1) / 32 * 32; s0 >= 0; s0 -= 32) {
       uint32_t first = 0, any = 0;  // slots whose first / some pattern matches
-      for (int i = 0; i < n; ++i) {
-        const State v = a & sm[s0 + i];
-        if (v == sl1[s0 + i]) first |= 1u << i;
-        if (v == sl2[s0 + i]) any |= 1u << i;
+      if (L.planes) {
+        const uint32_t* fl = first_lut + (s0 >> 5) * per_block;
+        const uint32_t* sl = second_lut + (s0 >> 5) * per_block;
+        uint32_t f = 0, g = 0;
+        State left = a;
+        for (int k = 0; k < L.nibbles; ++k, left >>= 4) {
+          f ^= fl[16 * k + (int)(left & 15)];
+          g ^= sl[16 * k + (int)(left & 15)];
+        }
+        const FreeWant w = want[s0 >> 5];
+        first = ~(f ^ w.first1) & ~(g ^ w.second1) & w.valid;
+        any = ~(f ^ w.first2) & ~(g ^ w.second2) & w.valid;
+      } else {
+        const int n = min(32, L.n_slots - s0);
+        for (int i = 0; i < n; ++i) {
+          const FreeSlot<State> q = slots[s0 + i];
+          const State v = a & q.m;
+          if (v == q.l1) first |= 1u << i;
+          if (v == q.l2) any |= 1u << i;
+        }
       }
       any |= first;
       while (any != 0) {
@@ -153,15 +232,15 @@ __global__ void __launch_bounds__(kFreeThreads, 2)
         for (int u = 0; u < 4; ++u) {
           xv[u] = Col::zero();
           if (any != 0) {
-            const int i = __ffs(any) - 1;
-            any &= any - 1;
-            const uint32_t t12 = st[s0 + i];
+            const int i = 31 - __clz(any);
+            any ^= 1u << i;
+            const uint32_t t12 = slots[s0 + i].terms;
             const uint32_t t = ((first >> i) & 1u) ? t12 & 0xffffu : t12 >> 16;
-            const uint32_t info = ti[t];
-            State b = a ^ tx[t];
-            uint32_t neg = info >> 31;
-            if (L.signs) neg ^= (uint32_t)popc_state((State)(b & ts[t]));
-            if ((info & kRowTermNeedsCheck) && !constraint_ok(p.constraint, b)) {
+            const FreeTerm<State> term = terms[t];
+            State b = a ^ term.x;
+            uint32_t neg = 0;
+            if (L.signs) neg = (uint32_t)popc_state((State)(b & ts[t]));
+            if (L.checks && (term.info & kRowTermNeedsCheck) && !constraint_ok(p.constraint, b)) {
               atomicOr(err, 1);
               continue;
             }
@@ -174,7 +253,8 @@ __global__ void __launch_bounds__(kFreeThreads, 2)
             }
             const uint64_t j = identity ? (uint64_t)b : (uint64_t)(hi[b >> split] + lo[b & low_mask]);
             xv[u] = __ldg(x + j * (uint64_t)ldx + c);
-            cf[u] = flip_sign(coef[(info >> 16) & 0xffu], neg << 31);
+            cf[u] = coef[t];
+            if (L.signs || INV) cf[u] = flip_sign(cf[u], neg << 31);
             ok |= 1u << u;
           }
         }
@@ -187,13 +267,18 @@ __global__ void __launch_bounds__(kFreeThreads, 2)
     int count = 0;
     for (int b = 0; b < L.n_diag_blocks; ++b) {
       const uint2 info = db[b];  // {signs, class | last block of it << 31}
-      const State* m = (const State*)(smem + L.off_dm) + 32 * b;
-      const State* r = (const State*)(smem + L.off_dr) + 32 * b;
-      const State* s = (const State*)(smem + L.off_ds) + 32 * b;
-      for (int i = 0; i < (int)((info.y >> 16) & 0x3fu); ++i) {
-        const int odd = (popc_state((State)(a & s[i])) ^ (int)(info.x >> i)) & 1;
-        if ((a & m[i]) == r[i]) count += 1 - 2 * odd;
+      const uint32_t valid = 0xffffffffu >> (32 - ((info.y >> 16) & 0x3fu));
+      uint32_t odd = info.x;
+      State left = a;
+      for (int k = 0; k < L.nibbles; ++k, left >>= 4) odd ^= parity_lut[b * per_block + 16 * k + (int)(left & 15)];
+      uint32_t hit = valid;
+      if (!((info.y >> 30) & 1u)) {  // some term of the block has a mask
+        const State* m = (const State*)(smem + L.off_dm) + 32 * b;
+        const State* r = (const State*)(smem + L.off_dr) + 32 * b;
+        for (int i = 0; i < 32; ++i)
+          if ((a & m[i]) != r[i]) hit &= ~(1u << i);
       }
+      count += __popc(hit) - 2 * __popc(hit & odd);
       if (info.y >> 31) {
         const double2 v = ((const double2*)(smem + L.off_dv))[info.y & 0xffffu];
         dre = fma((double)count, v.x, dre);
@@ -221,7 +306,7 @@ static bool free_layout(const MatvecProblem& p, FreeLayout* out) {
   const DeviceRowTerms &t = p.off.rows, &d = p.diag.rows;
   if (!t.ok || !d.ok || p.group.n_bits > 63) return false;
   if (!p.index.identity && p.index.rank_lo == nullptr) return false;
-  if ((size_t)p.off.n * 20 > kFreeSmem || (size_t)d.slot_blocks * 32 * 12 > kFreeSmem) return false;
+  if ((size_t)p.off.n * 40 > 2 * kFreeSmem || (size_t)t.slot_blocks * 32 * 40 > 2 * kFreeSmem || (size_t)d.slot_blocks * 32 * 12 > kFreeSmem) return false;
   const size_t state = p.group.n_bits <= 32 ? 4 : 8;
   uint32_t o = 0;
   auto take = [&](size_t bytes) {
@@ -233,14 +318,18 @@ static bool free_layout(const MatvecProblem& p, FreeLayout* out) {
   L.n_slots = t.n_slots;
   L.n_diag_blocks = d.slot_blocks;
   L.signs = t.any_sign;
-  L.off_coef = take((size_t)t.n_cls * 16);
-  L.off_sm = take(L.n_slots * state);
-  L.off_sl1 = take(L.n_slots * state);
-  L.off_sl2 = take(L.n_slots * state);
-  L.off_st = take((size_t)L.n_slots * 4);
-  L.off_ti = take((size_t)L.T * 4);
+  L.off_coef = take((size_t)L.T * 16);
+  L.off_slots = take((size_t)L.n_slots * state * 4);
+  L.off_terms = take((size_t)L.T * state * 2);
   L.off_ts = take(L.T * state);
-  L.off_tx = take(L.T * state);
+  L.nibbles = (p.group.n_bits + 3) / 4;
+  L.planes = t.two_site;
+  L.checks = t.any_check;
+  const size_t lut = L.planes ? (size_t)t.slot_blocks * L.nibbles * 64 : 0;
+  L.off_want = take((size_t)t.slot_blocks * sizeof(FreeWant));
+  L.off_first = take(lut);
+  L.off_second = take(lut);
+  L.off_parity = take((size_t)L.n_diag_blocks * L.nibbles * 64);
   L.off_dm = take(32 * L.n_diag_blocks * state);
   L.off_dr = take(32 * L.n_diag_blocks * state);
   L.off_ds = take(32 * L.n_diag_blocks * state);
