@@ -129,13 +129,13 @@ static double rows_scan_cost(const MatvecProblem& p, int mode) {
   return planes * (4.5 * mode + 5.0) + (p.constraint.kind == 2 ? 8.0 : 2.5) * (30.0 + 4.0 * (p.group.n_bits - planes));
 }
 
-constexpr int kLeastWarps = 4;
+constexpr int64_t kLeastWarps = 4;
 
 bool rows_fit(const MatvecProblem& p, int n_sectors) {
   RowsLayout L;
   if (p.projection != 2) return false;
   for (const int m : kRowModes)
-    if (rows_mode_allowed(p, m) && rows_layout(p, m, n_sectors > 0 || p.real_elements == 0, true, n_sectors, kLeastWarps, 1, &L)) return true;
+    if (rows_mode_allowed(p, m) && rows_layout(p, m, n_sectors > 0 || p.real_elements == 0, true, n_sectors, (int)kLeastWarps, 1, &L)) return true;
   return false;
 }
 
@@ -161,7 +161,7 @@ static bool rows_shape(const MatvecProblem& p, bool complex_elements, bool keep,
       warps[i] = fit(kRowsSmem);
       if (!keep && fit(kRowsSmemL1) >= 20) warps[i] = fit(kRowsSmemL1);
     }
-    for (const int enough : {keep ? 24 : 20, 16, 8, kLeastWarps}) {
+    for (const int enough : {keep ? 24 : 20, 16, 8, (int)kLeastWarps}) {
       int pick = -1;
       double least = 0.0;
       for (int i = 0; i < 4; ++i) {
@@ -200,7 +200,9 @@ bool rows_plan(const MatvecProblem& p, int col, int k, int64_t n_rows, int n_sec
   int warps = L.threads / 32;
   // few rows: one group of rows per warp, the warps spread over the SMs
   const int64_t groups = (n_rows + L.R - 1) / L.R;
-  const int64_t per_sm = std::max<int64_t>(kLeastWarps, (groups + sms - 1) / sms);
+  // ... and enough of them to fill the tables in a few passes
+  const int64_t staged = (int64_t)L.n_pat * L.words + (int64_t)p.group.n_bits * L.G;
+  const int64_t per_sm = std::max<int64_t>({kLeastWarps, (groups + sms - 1) / sms, staged / 256});
   if (per_sm < warps) {
     warps = (int)per_sm;
     if (!rows_layout(p, out->mode, complex_elements, keep, n_sectors, warps, L.R, &L)) return false;

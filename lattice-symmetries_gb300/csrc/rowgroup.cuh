@@ -143,24 +143,29 @@ struct RowGroup {
     const int G = L.G, nb = p.group.n_bits;
     const int tid = threadIdx.x, nt = blockDim.x;
     uint32_t* site = (uint32_t*)(smem + L.off_site);
+    if constexpr (MODE == kModeN32) {
 #pragma unroll 4
-    for (int i = tid; i < nb * L.site_words; i += nt) {
-      const int b = i / L.site_words, w = i - b * L.site_words;
-      const uint64_t* r = p.group.onehot + b * G;
-      if constexpr (MODE == kModeN32) {
-        site[i] = w < L.words ? (uint32_t)__ldg(r + (w < G ? w : 0)) : 0u;
-      } else {
-        // which of the word's 32 elements move site b to the plane's position (or, with spin
-        // inversion, to the top)
-        const int top = nb - 1, pos = top - w / MODE - (INV ? 1 : 0), g0 = 32 * (w % MODE);
-        uint32_t v = 0;
-        if (w < L.words)
-          for (int i32 = 0; i32 < 32 && g0 + i32 < G; ++i32) {
-            const uint64_t image = __ldg(r + g0 + i32);
-            const uint32_t bit = (uint32_t)(image >> pos) ^ (INV ? (uint32_t)(image >> top) : 0u);
-            v |= (bit & 1u) << i32;
-          }
-        site[i] = v;
+      for (int i = tid; i < nb * L.site_words; i += nt) {
+        const int b = i / L.site_words, w = i - b * L.site_words;
+        site[i] = w < L.words ? (uint32_t)__ldg(p.group.onehot + b * G + (w < G ? w : 0)) : 0u;
+      }
+    } else {
+      // word w of plane q: which of 32 elements move site b to the plane's position (or, with spin
+      // inversion, to the top).  A warp reads the 32 images once and ballots plane by plane.
+      const int ln = tid & 31, top = nb - 1;
+#pragma unroll 2
+      for (int i = tid >> 5; i < nb * MODE; i += nt >> 5) {
+        const int b = i / MODE, w = i - b * MODE, g = 32 * w + ln;
+        const uint64_t image = g < G ? __ldg(p.group.onehot + b * G + g) : 0ull;
+        for (int q = 0; q < L.planes; ++q) {
+          const uint32_t bit = (uint32_t)(image >> (top - q - (INV ? 1 : 0))) ^ (INV ? (uint32_t)(image >> top) : 0u);
+          const unsigned v = __ballot_sync(FULL, bit & 1u);
+          if (ln == 0) site[b * L.site_words + q * MODE + w] = v;
+        }
+      }
+      for (int i = tid; i < nb * (L.site_words - L.words); i += nt) {
+        const int pad = L.site_words - L.words, b = i / pad;
+        site[b * L.site_words + L.words + i - b * pad] = 0u;
       }
     }
     if constexpr (MODE != kModeN32) {
