@@ -609,11 +609,10 @@ __device__ __forceinline__ void gram_epilogue(uint32_t tmem_buf, const int (*col
   }
 }
 
-// Reduces the per-thread sums over lane blocks and complex pairs into partial[s][blockIdx.x]
-// (k x k complex), then clears them.
+// Reduces the per-thread sums over lane blocks and complex pairs into `partial` (k x k complex: this
+// CTA's share of the sector), then clears them.
 template <int KP>
-__device__ __forceinline__ void gram_flush(double (&acc)[GramShape<KP>::DC], double* P, int k, int64_t s,
-                                           double2* partial) {
+__device__ __forceinline__ void gram_flush(double (&acc)[GramShape<KP>::DC], double* P, int k, double2* partial) {
   using Sh = GramShape<KP>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int quarter = warp & 3, part = warp >> 2;
@@ -634,7 +633,7 @@ __device__ __forceinline__ void gram_flush(double (&acc)[GramShape<KP>::DC], dou
       re += Pq[(2 * a) * Sh::NR + 2 * b] + Pq[(2 * a + 1) * Sh::NR + 2 * b + 1];
       im += Pq[(2 * a) * Sh::NR + 2 * b + 1] - Pq[(2 * a + 1) * Sh::NR + 2 * b];
     }
-    partial[((size_t)s * gridDim.x + blockIdx.x) * nout + o] = make_double2(re, im);
+    partial[o] = make_double2(re, im);
   }
   __syncthreads();
 }
@@ -642,7 +641,7 @@ __device__ __forceinline__ void gram_flush(double (&acc)[GramShape<KP>::DC], dou
 template <int KP>
 __global__ void __launch_bounds__(kThreads, 1)
     k_block_gram_tc(int64_t D, int k, int64_t tiles_per_sector, int64_t total_tiles, const double* X,
-                    const double* Y, bool same, double2* partial, int* err) {
+                    const double* Y, bool same, double2* partials, int slots, int* err) {
   using Sh = GramShape<KP>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* XD = smem;
@@ -654,6 +653,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int tid = threadIdx.x, warp = tid >> 5;
   const int64_t t_begin = (int64_t)blockIdx.x * total_tiles / gridDim.x;
   const int64_t t_end = (int64_t)(blockIdx.x + 1) * total_tiles / gridDim.x;
+  // the partial Gram of the CTA's share of sector s (one slot per sector that it touches)
+  auto partial = [&](int64_t s) {
+    return partials + ((size_t)blockIdx.x * slots + (size_t)(s - t_begin / tiles_per_sector)) * (size_t)(k * k);
+  };
   // zero planes of X (never written again)
   for (uint32_t g = 0; g < kRows / 8; ++g)
     for (uint32_t e = tid; e < (uint32_t)(Sh::Z * Sh::NR * 16 / 16); e += kThreads)
@@ -726,7 +729,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     same);
     if (it >= 1) {
       gram_epilogue<KP>(tmem + (buf ^ 1) * Sh::buf_cols, colmax[(it - 1) % 3], same, acc);
-      if ((tile - 1) / tiles_per_sector != s) gram_flush<KP>(acc, P, k, (tile - 1) / tiles_per_sector, partial);
+      if ((tile - 1) / tiles_per_sector != s) gram_flush<KP>(acc, P, k, partial((tile - 1) / tiles_per_sector));
     }
     tc::fence_before_sync();
   }
@@ -739,13 +742,45 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else {
       tc::fence_after_sync();
       gram_epilogue<KP>(tmem + lb * Sh::buf_cols, colmax[(n - 1) % 3], same, acc);
-      gram_flush<KP>(acc, P, k, (t_end - 1) / tiles_per_sector, partial);
+      gram_flush<KP>(acc, P, k, partial((t_end - 1) / tiles_per_sector));
     }
   }
   if (failed && threadIdx.x == 0) atomicExch(err, 1);
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, Sh::tmem_cols);
+}
+
+// G[s] = the partials of the CTAs whose tiles touch sector s, added in a fixed order.  (Partials for
+// every CTA and sector, cleared and summed in full, took 22 us per Gram of 44 sectors.)
+__global__ void __launch_bounds__(256) k_gram_tc_sum(const double2* __restrict__ partials, int ctas, int slots, int nout,
+                                                     int64_t tiles_per_sector, int64_t total_tiles,
+                                                     double2* __restrict__ G) {
+  __shared__ double2 warp_sums[8][32];
+  const int64_t s = blockIdx.x, begin = s * tiles_per_sector, end = begin + tiles_per_sector;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o = blockIdx.y * 32 + lane;
+  auto first_tile = [&](int64_t c) { return c * total_tiles / ctas; };
+  int64_t c0 = begin * ctas / total_tiles;  // the CTA that holds the sector's first tile
+  while (c0 > 0 && first_tile(c0) > begin) --c0;
+  while (first_tile(c0 + 1) <= begin) ++c0;
+  double2 t = make_double2(0.0, 0.0);
+  if (o < nout)
+    for (int64_t c = c0 + warp; c < ctas && first_tile(c) < end; c += 8) {
+      if (first_tile(c) == first_tile(c + 1)) continue;  // no tiles
+      const double2 v = partials[((size_t)c * slots + (size_t)(s - first_tile(c) / tiles_per_sector)) * nout + o];
+      t.x += v.x;
+      t.y += v.y;
+    }
+  warp_sums[warp][lane] = t;
+  __syncthreads();
+  if (warp == 0 && o < nout) {
+    t = make_double2(0.0, 0.0);
+    for (int w = 0; w < 8; ++w) {
+      t.x += warp_sums[w][lane].x;
+      t.y += warp_sums[w][lane].y;
+    }
+    G[s * nout + o] = t;
+  }
 }
 
 template <int KP>
@@ -756,17 +791,21 @@ int run_gram_tc(int64_t S, int64_t D, int k, const double* d_x, const double* d_
   const int64_t total = S * tiles_per_sector;
   const int grid = (int)std::min<int64_t>(total, (int64_t)num_sms());
   const int nout = k * k;
-  const size_t pbytes = (size_t)S * grid * nout * sizeof(double2);
+  // a CTA's tiles are consecutive: it keeps one partial per sector that they touch, at most `slots`
+  const int64_t most_tiles = (total + grid - 1) / grid;
+  const int slots = (int)((most_tiles + tiles_per_sector - 2) / tiles_per_sector + 1);
   double2* partial = nullptr;
-  if (!cuda_ok(cudaMallocAsync((void**)&partial, pbytes, st), "cudaMallocAsync(Gram partials)")) return LS_GPU_ERR_CUDA;
-  // a CTA writes the partials of the sectors its rows touch; the others stay zero
-  bool ok = cuda_ok(cudaMemsetAsync(partial, 0, pbytes, st), "cudaMemsetAsync(Gram partials)");
+  if (!cuda_ok(cudaMallocAsync((void**)&partial, (size_t)grid * slots * nout * sizeof(double2), st),
+               "cudaMallocAsync(Gram partials)"))
+    return LS_GPU_ERR_CUDA;
+  k_block_gram_tc<KP><<<grid, kThreads, Sh::smem, st>>>(D, k, tiles_per_sector, total, d_x, d_y, d_x == d_y, partial,
+                                                        slots, device_error_word() + 1);
+  bool ok = cuda_ok(cudaGetLastError(), "k_block_gram_tc");
   if (ok) {
-    k_block_gram_tc<KP><<<grid, kThreads, Sh::smem, st>>>(D, k, tiles_per_sector, total, d_x, d_y, d_x == d_y,
-                                                          partial, device_error_word() + 1);
-    ok = cuda_ok(cudaGetLastError(), "k_block_gram_tc");
+    k_gram_tc_sum<<<dim3((unsigned)S, (unsigned)((nout + 31) / 32)), 256, 0, st>>>(
+        partial, grid, slots, nout, tiles_per_sector, total, reinterpret_cast<double2*>(d_g));
+    ok = cuda_ok(cudaGetLastError(), "k_gram_tc_sum");
   }
-  if (ok) ok = launch_gram_partial_sum(partial, grid, nout, S, reinterpret_cast<double2*>(d_g), st) == 0;
   ok = cuda_ok(cudaFreeAsync(partial, st), "cudaFreeAsync(Gram partials)") && ok;
   return ok ? 0 : LS_GPU_ERR_CUDA;
 }
