@@ -184,9 +184,7 @@ static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const do
   MatvecProblem q = p;
   q.ldxs = words == 1 && k > 1 ? k + k % 2 : k;  // real columns are read in pairs
   // small problems read the norms with x instead of a scaled copy: an allocation and a launch less
-  // (pairs of real columns need the copy's alignment)
-  const bool unscaled =
-      k == 1 ? p.n_rows <= kUnscaledRows : words == 2 && p.n_rows * k <= kUnscaledElements;
+  const bool unscaled = k == 1 ? p.n_rows <= kUnscaledRows : p.n_rows * k <= kUnscaledElements;
   double* d_xs = unscaled ? nullptr : prescaled_copy(p, words, k, d_x, ldx, q.ldxs, s);
   if (d_xs == nullptr && !unscaled) return 1;
   int rc = 0;

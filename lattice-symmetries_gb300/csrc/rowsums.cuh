@@ -80,6 +80,21 @@ __device__ __forceinline__ double2 shfl_down_v(double2 v, int d) {
 __device__ __forceinline__ double add_v(double a, double b) { return a + b; }
 __device__ __forceinline__ double2 add_v(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
+// x_j (n_j) of column unit c: a vector load from a scaled copy or of complex columns; pairs of the
+// caller's real columns are only 8-byte aligned and may lack the second.
+template <int COL>
+__device__ __forceinline__ typename Column<COL>::V load_x(const RowsSums& s, uint32_t j, int c) {
+  using V = typename Column<COL>::V;
+  if constexpr (COL == kColPair) {
+    if (s.norms != nullptr && s.real_cols) {
+      const double* q = s.xs + (int64_t)j * s.ldxs + 2 * c;
+      return make_double2(__ldg(q), 2 * c + 1 < s.real_cols ? __ldg(q + 1) : 0.0);
+    }
+  }
+  const int64_t ldv = COL == kColPair && s.real_cols ? s.ldxs / 2 : s.ldxs;
+  return __ldg(reinterpret_cast<const V*>(s.xs) + (int64_t)j * ldv + c);
+}
+
 // y of one row and column: the sum over n_i plus the diagonal (zero for a zero-norm row).
 template <int COL>
 __device__ __forceinline__ void write_output(const RowsSums& s, int64_t row, int c, typename Column<COL>::V acc,
@@ -115,14 +130,12 @@ __device__ __forceinline__ void resolve_and_sum(Group& g, const RowsSums& s, con
   using V = typename Col::V;
   constexpr unsigned FULL = 0xffffffffu;
   const RowsLayout& L = g.L;
-  const V* __restrict__ xs = reinterpret_cast<const V*>(s.xs);
-  const int64_t ldv = COL == kColPair && s.real_cols ? s.ldxs / 2 : s.ldxs;
   V acc = Col::zero();
   g.resolve(ix, err, binom, [&](const auto& j, const auto& w, const auto&) {
     constexpr int E = sizeof(j) / sizeof(j[0]);
     V xv[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) xv[e] = j[e] != Group::kAbsent ? __ldg(xs + (int64_t)j[e] * ldv) : Col::zero();
+    for (int e = 0; e < E; ++e) xv[e] = j[e] != Group::kAbsent ? load_x<COL>(s, j[e], 0) : Col::zero();
     if (s.norms != nullptr) {
 #pragma unroll
       for (int e = 0; e < E; ++e) xv[e] = scaled(xv[e], j[e] != Group::kAbsent ? __ldg(s.norms + j[e]) : 0.0);
@@ -153,8 +166,6 @@ __device__ __forceinline__ void sum_rows(const Group& g, const RowsSums& s, cons
   const int c = lane % s.cols, rest = lane / s.cols;
   const int q = rest & (s.q - 1), rl = rest / s.q;
   const bool active = rl < s.rp;
-  const V* __restrict__ xs = reinterpret_cast<const V*>(s.xs) + c;
-  const int64_t ldv = COL == kColPair && s.real_cols ? s.ldxs / 2 : s.ldxs;
   const double2 diag = g.diagonal();
   for (int r0 = 0; r0 < g.nr; r0 += s.rp) {
     const int r = r0 + rl;
@@ -174,7 +185,7 @@ __device__ __forceinline__ void sum_rows(const Group& g, const RowsSums& s, cons
         w[u] = at + q < n ? e[at] : make_uint2(Group::kAbsent, 0u);
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) xv[u] = w[u].x != Group::kAbsent ? __ldg(xs + (int64_t)w[u].x * ldv) : Col::zero();
+      for (int u = 0; u < 4; ++u) xv[u] = w[u].x != Group::kAbsent ? load_x<COL>(s, w[u].x, c) : Col::zero();
       if (s.norms != nullptr) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) xv[u] = scaled(xv[u], w[u].x != Group::kAbsent ? __ldg(s.norms + w[u].x) : 0.0);
