@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kFreeThreads, 2)
        row += warps * L.rows_per_warp) {
     const State a = identity ? (State)row : (State)__ldg(p.index.reps + row);
     V acc = Col::zero();
-    for (int s0 = (L.n_slots - 1) / 32 * 32; s0 >= 0; s0 -= 32) {
+    for (int s0 = 32 * (slot_blocks - 1); s0 >= 0; s0 -= 32) {  // none without off-diagonal terms
       uint32_t first = 0, any = 0;  // slots whose first / some pattern matches
       if (L.planes) {
         const uint32_t* fl = first_lut + (s0 >> 5) * per_block;

@@ -50,13 +50,15 @@ def _case(name):
         return Case(ls.SpinfulFermionBasis(5, 4), LAT.hubbard(LAT.chain_bonds(5), 1.0, 3.0))
     if name == "hubbard_all":
         return Case(ls.SpinfulFermionBasis(4), LAT.hubbard(LAT.chain_bonds(4), 1.0, 3.0))
+    if name == "diagonal":  # no off-diagonal terms at all
+        return Case(ls.SpinBasis(9, 4), ls.Expr("σᶻ₀ σᶻ₁", sites=[list(b) for b in LAT.chain_bonds(9)]))
     if name == "all_pairs":  # more than 32 term slots
         return Case(ls.SpinBasis(12, 5), LAT.heisenberg([(i, j) for i in range(12) for j in range(i)]))
     raise KeyError(name)
 
 
 NAMES = ["all_states", "odd_weight", "one_site", "no_particles", "inversion", "bits26", "bits32", "bits33", "bits40",
-         "bits41", "spinless", "hubbard", "hubbard_total", "hubbard_all", "all_pairs"]
+         "bits41", "spinless", "hubbard", "hubbard_total", "hubbard_all", "all_pairs", "diagonal"]
 
 
 @pytest.mark.parametrize("name", NAMES)

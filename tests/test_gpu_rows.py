@@ -43,13 +43,16 @@ def _case(name):
         e = e + ls.Expr("σᶻ₀ σᶻ₁", sites=[list(b) for b in LAT.chain_bonds(10)]) + \
             ls.Expr("σᶻ₀", sites=[[i] for i in range(10)]).scale(0.4)
         return Case(ls.SpinBasis(10, None, None, S(LAT.chain_symmetries(10, 3))), e)
+    if name == "diagonal":  # no off-diagonal terms at all
+        return Case(ls.SpinBasis(12, 6, 1, S(LAT.chain_symmetries(12, 0))),
+                    ls.Expr("σᶻ₀ σᶻ₁", sites=[list(b) for b in LAT.chain_bonds(12)]))
     if name == "one_row":
         return Case(ls.SpinBasis(12, 1, None, S(LAT.chain_symmetries(12, 0))), LAT.heisenberg(LAT.chain_bonds(12)))
     raise KeyError(name)
 
 
 NAMES = ["chain9", "chain16_inversion", "chain32", "chain33", "chain63", "all_pairs25", "square36",
-         "all_pairs20_inversion", "flips", "one_row"]
+         "all_pairs20_inversion", "flips", "one_row", "diagonal"]
 
 
 @pytest.fixture(scope="module")
