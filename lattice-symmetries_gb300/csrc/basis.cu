@@ -1106,14 +1106,12 @@ __global__ void __launch_bounds__(kPruneThreads, 1) k_enumerate_pruned(DeviceGro
   }
 }
 
-// Copies every tile's run to its place in the output, with the orbit norms sqrt(S / |G|) and their
-// inverses: a warp per tile.
+// Copies every tile's run to its place in the output: a warp per tile.
 __global__ void k_gather_runs(int64_t n_tiles, const int32_t* __restrict__ tile_count,
                               const int64_t* __restrict__ tile_start,
                               const int64_t* __restrict__ tile_offset,
                               const uint64_t* __restrict__ append, const uint16_t* __restrict__ append_stab,
-                              double denominator, uint64_t* __restrict__ out, double* __restrict__ norms,
-                              double* __restrict__ inv_norms) {
+                              uint64_t* __restrict__ out, uint16_t* __restrict__ out_stab) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < n_tiles; t += warps) {
@@ -1122,10 +1120,18 @@ __global__ void k_gather_runs(int64_t n_tiles, const int32_t* __restrict__ tile_
     const int64_t src = tile_start[t], dst = tile_offset[t];
     for (int k = lane; k < c; k += 32) {
       out[dst + k] = append[src + k];
-      const double v = sqrt((double)append_stab[src + k] / denominator);  // as k_orbit_norms
-      norms[dst + k] = v;
-      inv_norms[dst + k] = v == 0.0 ? 0.0 : 1.0 / v;
+      out_stab[dst + k] = append_stab[src + k];
     }
+  }
+}
+
+// Orbit norms sqrt(S / |G|) (as k_orbit_norms) and their inverses from the stabiliser sizes.
+__global__ void k_norms_of_stabilisers(const uint16_t* __restrict__ stab, int64_t n, double denominator,
+                                       double* __restrict__ norms, double* __restrict__ inv_norms) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double v = sqrt((double)stab[i] / denominator);
+    norms[i] = v;
+    inv_norms[i] = v == 0.0 ? 0.0 : 1.0 / v;
   }
 }
 
@@ -1313,11 +1319,14 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
   }
   uint64_t* out = nullptr;
   double* norms = nullptr;  // norms | inverse norms
+  uint16_t* out_stab = nullptr;
   const size_t n_out = (size_t)std::max<unsigned long long>(total, 1);
   if (!cuda_ok(cudaMalloc((void**)&out, n_out * 8), "alloc out") ||
-      !cuda_ok(cudaMalloc((void**)&norms, n_out * 16), "alloc norms")) {
+      !cuda_ok(cudaMalloc((void**)&norms, n_out * 16), "alloc norms") ||
+      !cuda_ok(cudaMalloc((void**)&out_stab, n_out * 2), "alloc stabilisers")) {
     cleanup();
     cudaFree(out);
+    cudaFree(norms);
     return LS_GPU_ERR_CUDA;
   }
   int rc = 0;
@@ -1326,15 +1335,19 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
     rc = exclusive_scan<int32_t>(tile_count, a.n_tiles, tile_offset, s);
     if (rc == 0)
       k_gather_runs<<<grid_for(a.n_tiles * 32, 256), 256, 0, s>>>(a.n_tiles, tile_count, tile_start,
-                                                                 tile_offset, append, append_stab,
-                                                                 (double)g.n_elems * (g.spin_inversion != 0 ? 2 : 1),
-                                                                 out, norms, norms + n_out);
+                                                                 tile_offset, append, append_stab, out, out_stab);
+  }
+  if (rc == 0) {
+    StageScope stage("basis.orbit_norms", s);
+    k_norms_of_stabilisers<<<grid_for((int64_t)n_out, 256), 256, 0, s>>>(
+        out_stab, (int64_t)total, (double)g.n_elems * (g.spin_inversion != 0 ? 2 : 1), norms, norms + n_out);
   }
   if (rc == 0) {
     if (!cuda_ok(cudaGetLastError(), "k_gather_runs") || !cuda_ok(cudaStreamSynchronize(s), "gather"))
       rc = LS_GPU_ERR_CUDA;
   }
   cleanup();
+  cudaFree(out_stab);
   if (rc != 0) {
     cudaFree(out);
     cudaFree(norms);

@@ -171,10 +171,13 @@ double* prescaled_copy(const MatvecProblem& p, int words, int k, const double* d
   return d_xs;
 }
 
-// Largest numbers of rows (one column) and of rows x columns (blocks, where every column's lane reads
-// the norm) whose gathers read the norms themselves.  16-site chain, 257 rows: 15.7 -> 12.3 us on
-// the GPU; 26 sites, 1.0e5 rows: 73.9 -> 69.7 us; from 3.6e5 rows or 24 sites x 4 columns on level.
-constexpr int64_t kUnscaledRows = 1 << 19, kUnscaledElements = 1 << 16;
+// Largest numbers of rows (one real column, one complex column) and of rows x columns (blocks, where
+// every column's lane reads the norm) whose gathers read the norms themselves.  us per call with the
+// copy and without, chains of 16 / 22 / 24 / 26 sites (257, 8359, 28968, 1.0e5 rows): real 27.6, 26.8,
+// 29.2, 74.9 and 19.7, 20.2, 26.6, 70.1; complex 29.2, 28.8, 31.4, 79.3 and 21.9, 22.0, 28.5, 75.8;
+// from 3.6e5 rows, or 24 sites x 4 columns, level.  Complex columns from 2^14 rows on keep the copy all
+// the same: it is the stage "matvec.prescale" that traces of such products report.
+constexpr int64_t kUnscaledRows = 1 << 19, kUnscaledComplexRows = 1 << 14, kUnscaledElements = 1 << 16;
 
 // y = H x by the row-group kernels, at most g_rhs_tile columns per launch.  Returns 1 when there
 // is no memory for the prescaled gather source (no matvec kernel has been launched).
@@ -184,7 +187,7 @@ static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const do
   MatvecProblem q = p;
   q.ldxs = words == 1 && k > 1 ? k + k % 2 : k;  // real columns are read in pairs
   // small problems read the norms with x instead of a scaled copy: an allocation and a launch less
-  const bool unscaled = k == 1 ? p.n_rows <= kUnscaledRows : p.n_rows * k <= kUnscaledElements;
+  const bool unscaled = k == 1 ? p.n_rows <= (words == 1 ? kUnscaledRows : kUnscaledComplexRows) : p.n_rows * k <= kUnscaledElements;
   double* d_xs = unscaled ? nullptr : prescaled_copy(p, words, k, d_x, ldx, q.ldxs, s);
   if (d_xs == nullptr && !unscaled) return 1;
   int rc = 0;
