@@ -1125,13 +1125,21 @@ __global__ void k_gather_runs(int64_t n_tiles, const int32_t* __restrict__ tile_
   }
 }
 
-// Orbit norms sqrt(S / |G|) (as k_orbit_norms) and their inverses from the stabiliser sizes.
+// Orbit norms sqrt(S / |G|) (as k_orbit_norms) and their inverses from the stabiliser sizes.  Nearly
+// all stabilisers have one element, so that pair is computed once per thread: with a root and a
+// division per state the FP64 pipe bounds the kernel (6x6 torus, 1.6e7 states: 0.65 ms).
 __global__ void k_norms_of_stabilisers(const uint16_t* __restrict__ stab, int64_t n, double denominator,
                                        double* __restrict__ norms, double* __restrict__ inv_norms) {
+  const double norm_of_one = sqrt(1.0 / denominator), inverse_of_one = 1.0 / norm_of_one;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = sqrt((double)stab[i] / denominator);
+    const int size = stab[i];
+    double v = norm_of_one, inverse = inverse_of_one;
+    if (size != 1) {
+      v = sqrt((double)size / denominator);
+      inverse = v == 0.0 ? 0.0 : 1.0 / v;
+    }
     norms[i] = v;
-    inv_norms[i] = v == 0.0 ? 0.0 : 1.0 / v;
+    inv_norms[i] = inverse;
   }
 }
 

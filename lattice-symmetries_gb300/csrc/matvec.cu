@@ -187,7 +187,8 @@ static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const do
   MatvecProblem q = p;
   q.ldxs = words == 1 && k > 1 ? k + k % 2 : k;  // real columns are read in pairs
   // small problems read the norms with x instead of a scaled copy: an allocation and a launch less
-  const bool unscaled = k == 1 ? p.n_rows <= (words == 1 ? kUnscaledRows : kUnscaledComplexRows) : p.n_rows * k <= kUnscaledElements;
+  const int64_t most = k > 1 ? kUnscaledElements : words == 1 ? kUnscaledRows : kUnscaledComplexRows;
+  const bool unscaled = p.n_rows * k <= most;
   double* d_xs = unscaled ? nullptr : prescaled_copy(p, words, k, d_x, ldx, q.ldxs, s);
   if (d_xs == nullptr && !unscaled) return 1;
   int rc = 0;
