@@ -1227,11 +1227,11 @@ RowTables diag_rows(const TermTable& t, const int32_t* coupling) {
   return R;
 }
 
-// Device layout: v (double2, 16-byte aligned) first, then m, l, r, x, s (uint64), xinfo (uint32),
+// Appends a table to the host image of a block; its pointers are offsets until upload_block.
+// Layout: v (double2, 16-byte aligned) first, then m, l, r, x, s (uint64), xinfo (uint32),
 // then the row-group tables, each array on a 16-byte boundary.
-int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal, DeviceTermSet* out,
-                 const int32_t* coupling = nullptr, int n_couplings = 0) {
-  std::vector<uint8_t> host;
+void pack_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal, std::vector<uint8_t>& host,
+                DeviceTerms* out, const int32_t* coupling = nullptr, int n_couplings = 0) {
   auto put = [&](const void* src, size_t sz) {
     const size_t at = (host.size() + 15) & ~(size_t)15;
     host.resize(at + std::max<size_t>(sz, 16), 0);
@@ -1261,31 +1261,46 @@ int upload_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal
   const size_t rcv = put(R.cval.data(), R.cval.size() * 8), rcc = put(R.coupling.data(), R.coupling.size() * 4);
   const size_t rcm = put(R.cvec.data(), R.cvec.size() * 8);
   const size_t ocp = put(coupling, coupling ? n * 4 : 0);
-  out->terms.all_two_site = all_two;
-  if (!cuda_ok(cudaMalloc(&out->block, host.size()), "cudaMalloc(terms)")) return LS_GPU_ERR_CUDA;
-  if (!cuda_ok(cudaMemcpy(out->block, host.data(), host.size(), cudaMemcpyHostToDevice), "upload terms"))
-    return LS_GPU_ERR_CUDA;
-  uint8_t* d = (uint8_t*)out->block;
-  out->terms.n = t.n;
-  out->terms.v = (const double2*)(d + ov);
-  out->terms.m = (const uint64_t*)(d + om);
-  out->terms.l = (const uint64_t*)(d + ol);
-  out->terms.r = (const uint64_t*)(d + orr);
-  out->terms.x = (const uint64_t*)(d + ox);
-  out->terms.s = (const uint64_t*)(d + os);
-  out->terms.xinfo = (const uint32_t*)(d + oi);
-  DeviceRowTerms& r = out->terms.rows;
+  out->all_two_site = all_two;
+  out->n = t.n;
+  out->v = (const double2*)ov;
+  out->m = (const uint64_t*)om;
+  out->l = (const uint64_t*)ol;
+  out->r = (const uint64_t*)orr;
+  out->x = (const uint64_t*)ox;
+  out->s = (const uint64_t*)os;
+  out->xinfo = (const uint32_t*)oi;
+  DeviceRowTerms& r = out->rows;
   r = R.shape;
-  r.sm = (const uint64_t*)(d + rsm);
-  r.sl1 = (const uint64_t*)(d + rl1);
-  r.sl2 = (const uint64_t*)(d + rl2);
-  r.st = (const uint32_t*)(d + rst);
-  r.tinfo = (const uint32_t*)(d + rti);
-  r.xmask = (const uint64_t*)(d + rxm);
-  r.cval = (const double2*)(d + rcv);
-  r.coupling = (const uint32_t*)(d + rcc);
-  r.cvec = (const double2*)(d + rcm);
-  out->terms.coupling = coupling ? (const int32_t*)(d + ocp) : nullptr;
+  r.sm = (const uint64_t*)rsm;
+  r.sl1 = (const uint64_t*)rl1;
+  r.sl2 = (const uint64_t*)rl2;
+  r.st = (const uint32_t*)rst;
+  r.tinfo = (const uint32_t*)rti;
+  r.xmask = (const uint64_t*)rxm;
+  r.cval = (const double2*)rcv;
+  r.coupling = (const uint32_t*)rcc;
+  r.cvec = (const double2*)rcm;
+  out->coupling = coupling ? (const int32_t*)ocp : nullptr;
+}
+
+// One allocation and one copy for all the sets of a host image; the first set owns the block.
+int upload_block(const std::vector<uint8_t>& host, std::initializer_list<DeviceTermSet*> sets) {
+  void*& block = (*sets.begin())->block;
+  if (!cuda_ok(cudaMalloc(&block, host.size()), "cudaMalloc(terms)") ||
+      !cuda_ok(cudaMemcpy(block, host.data(), host.size(), cudaMemcpyHostToDevice), "upload terms")) {
+    if (block) cudaFree(block);
+    block = nullptr;
+    return LS_GPU_ERR_CUDA;
+  }
+  auto move = [&](auto&... p) { ((p = (std::decay_t<decltype(p)>)((uintptr_t)p + (uintptr_t)block)), ...); };
+  for (DeviceTermSet* set : sets) {
+    DeviceTerms& t = set->terms;
+    DeviceRowTerms& r = t.rows;
+    move(t.v, t.m, t.l, t.r, t.x, t.s, t.xinfo);
+    if (t.coupling) move(t.coupling);
+    move(r.sm, r.sl1, r.sl2, r.st, r.tinfo, r.xmask, r.cval, r.coupling, r.cvec);
+  }
   return 0;
 }
 
@@ -1307,10 +1322,14 @@ OperatorCache* operator_cache(const ls_hs_operator* op) {
   c->off = read_terms(op->off_diag_terms);
   c->diag = read_terms(op->diag_terms);
   const DeviceConstraint cons = op->basis ? basis_constraint(op->basis) : DeviceConstraint{};
-  if (upload_terms(c->off, cons, false, &c->fwd_off) ||
-      upload_terms(adjoint_terms(c->off), cons, false, &c->adj_off) ||
-      upload_terms(c->diag, cons, true, &c->fwd_diag) ||
-      upload_terms(adjoint_terms(c->diag), cons, true, &c->adj_diag)) {
+  // one block: an upload is an allocation and a synchronous copy (four of them: 134 us for the first
+  // product of an operator on 257 states, one: 112 us)
+  std::vector<uint8_t> host;
+  pack_terms(c->off, cons, false, host, &c->fwd_off.terms);
+  pack_terms(adjoint_terms(c->off), cons, false, host, &c->adj_off.terms);
+  pack_terms(c->diag, cons, true, host, &c->fwd_diag.terms);
+  pack_terms(adjoint_terms(c->diag), cons, true, host, &c->adj_diag.terms);
+  if (upload_block(host, {&c->fwd_off, &c->adj_off, &c->fwd_diag, &c->adj_diag})) {
     free_cache(c);
     return nullptr;
   }
@@ -1330,12 +1349,10 @@ int ensure_norms(IndexData* ix, const OrbitData* od) {
   if (od != nullptr && od->n_elems > 0) {
     const DeviceGroup* dg = orbit_device(od);
     rc = dg ? launch_orbit_norms(*dg, ix->n_states, ix->d_reps, ix->d_norms, s) : LS_GPU_ERR_CUDA;
+    if (rc == 0) rc = launch_inverse_norms(ix->d_norms, ix->n_states, ix->d_norms + n, s);
   } else {
-    std::vector<double> ones((size_t)n, 1.0);
-    rc = cuda_ok(cudaMemcpyAsync(ix->d_norms, ones.data(), ones.size() * 8, cudaMemcpyHostToDevice, s),
-                 "norms") ? 0 : LS_GPU_ERR_CUDA;
+    rc = launch_unit_norms(ix->d_norms, 2 * n, s);
   }
-  if (rc == 0) rc = launch_inverse_norms(ix->d_norms, ix->n_states, ix->d_norms + n, s);
   // The norms are computed on the library's stream but read by kernels on the caller's stream:
   // finish them before any caller can launch.
   if (rc == 0) rc = cuda_ok(cudaStreamSynchronize(s), "orbit norms") ? 0 : LS_GPU_ERR_CUDA;
@@ -1350,7 +1367,8 @@ int ensure_norms(IndexData* ix, const OrbitData* od) {
 // Rank tables of a complete basis without a group: all states of a fixed weight (all below the
 // flipped maximum with spin inversion), or of fixed (N_up, N_down).  Other sets of states (installed
 // by the caller) and more than 40 bits keep the search.
-int ensure_ranks(IndexData* ix, ls_hs_basis const* b) {
+// They are made on the library's stream: *pending tells whether the caller has to wait for it.
+int ensure_ranks(IndexData* ix, ls_hs_basis const* b, bool* pending) {
   if (ix->d_ranks != nullptr || ix->n_states == 0) return 0;
   const int n = basis_number_bits(b);
   if (n > 40) return 0;
@@ -1372,9 +1390,7 @@ int ensure_ranks(IndexData* ix, ls_hs_basis const* b) {
   cudaStream_t s = default_stream();
   const size_t lo = (size_t)1 << split, hi = (size_t)1 << (n - split);
   if (!cuda_ok(cudaMalloc((void**)&ix->d_ranks, (lo + hi) * 4), "cudaMalloc(ranks)")) return LS_GPU_ERR_CUDA;
-  int rc = launch_rank_tables(split, n - split, h, species, n_lo, ix->d_ranks, ix->d_ranks + lo, s);
-  // read by kernels on the caller's stream
-  if (rc == 0) rc = cuda_ok(cudaStreamSynchronize(s), "rank tables") ? 0 : LS_GPU_ERR_CUDA;
+  const int rc = launch_rank_tables(split, n - split, h, species, n_lo, ix->d_ranks, ix->d_ranks + lo, s);
   if (rc != 0) {
     cudaFree(ix->d_ranks);
     ix->d_ranks = nullptr;
@@ -1383,6 +1399,7 @@ int ensure_ranks(IndexData* ix, ls_hs_basis const* b) {
   ix->dev.rank_lo = ix->d_ranks;
   ix->dev.rank_hi = ix->d_ranks + lo;
   ix->dev.rank_split = split;
+  *pending = true;
   return 0;
 }
 
@@ -1398,8 +1415,15 @@ int make_problem(ls_hs_operator const* op, bool adjoint, MatvecProblem* p) {
   if (c == nullptr) return LS_GPU_ERR_CUDA;
   p->projection = !b->requires_projection ? 0 : (has_permutations(b) ? 2 : 1);
   if (p->projection == 1 && b->spin_inversion == 0) return fail(LS_GPU_ERR_INVALID, "projection without symmetries");
-  if (ensure_norms(ix, p->projection == 2 ? od : nullptr) != 0) return LS_GPU_ERR_CUDA;
-  if (p->projection != 2 && !b->state_index_is_identity && ensure_ranks(ix, b) != 0) return LS_GPU_ERR_CUDA;
+  const OrbitData* norms_od = p->projection == 2 ? od : nullptr;
+  const bool have_norms = ix->d_norms != nullptr && ix->norms_for == norms_od;
+  bool pending = false;
+  if (p->projection != 2 && !b->state_index_is_identity && ensure_ranks(ix, b, &pending) != 0)
+    return LS_GPU_ERR_CUDA;
+  // making the norms waits for the same stream
+  if (ensure_norms(ix, norms_od) != 0) return LS_GPU_ERR_CUDA;
+  if (pending && have_norms && !cuda_ok(cudaStreamSynchronize(default_stream()), "rank tables"))
+    return LS_GPU_ERR_CUDA;
   p->group = DeviceGroup{};
   if (p->projection == 2) {
     const DeviceGroup* dg = orbit_device(od);
@@ -1826,18 +1850,17 @@ extern "C" int ls_gpu_coupling_inner_products(ls_hs_operator const* op, int n_co
   for (int t = 0; t < n_terms; ++t)
     if (term_coupling[t] < 0 || term_coupling[t] >= n_couplings)
       return fail(LS_GPU_ERR_INVALID, "term coupling id out of range");
-  if (c->cpl_off.block == nullptr || c->cpl_diag.block == nullptr || c->coupling.size() != (size_t)n_terms || c->n_couplings != n_couplings ||
+  if (c->cpl_off.block == nullptr || c->coupling.size() != (size_t)n_terms || c->n_couplings != n_couplings ||
       (n_terms > 0 && memcmp(c->coupling.data(), term_coupling, (size_t)n_terms * 4) != 0)) {
-    for (DeviceTermSet* s : {&c->cpl_off, &c->cpl_diag}) {
-      if (s->block) cudaFree(s->block);
-      s->block = nullptr;
-    }
+    if (c->cpl_off.block) cudaFree(c->cpl_off.block);
+    c->cpl_off.block = nullptr;
     c->coupling.assign(term_coupling, term_coupling + n_terms);
     c->n_couplings = n_couplings;
     const DeviceConstraint cons = basis_constraint(op->basis);
-    if (upload_terms(c->off, cons, false, &c->cpl_off, term_coupling, n_couplings) ||
-        upload_terms(c->diag, cons, true, &c->cpl_diag, term_coupling + c->off.n))
-      return LS_GPU_ERR_CUDA;
+    std::vector<uint8_t> host;
+    pack_terms(c->off, cons, false, host, &c->cpl_off.terms, term_coupling, n_couplings);
+    pack_terms(c->diag, cons, true, host, &c->cpl_diag.terms, term_coupling + c->off.n);
+    if (upload_block(host, {&c->cpl_off, &c->cpl_diag})) return LS_GPU_ERR_CUDA;
   }
   p.off = c->cpl_off.terms;
   p.diag = c->cpl_diag.terms;

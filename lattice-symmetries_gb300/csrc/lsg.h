@@ -207,6 +207,7 @@ int launch_orbit_norms(const DeviceGroup& g, int64_t n, const uint64_t* d_reps, 
                        cudaStream_t s);
 // inv[i] = 1 / norms[i], or 0 where norms[i] == 0.
 int launch_inverse_norms(const double* d_norms, int64_t n, double* d_inv, cudaStream_t s);
+int launch_unit_norms(double* d_norms, int64_t n, cudaStream_t s);
 int compute_site_images(OrbitData* od);          // host tables (no GPU needed)
 const DeviceGroup* orbit_device(const OrbitData* od);  // uploads on first use; null on failure
 
