@@ -15,8 +15,9 @@
 // conj(g_i) / n_i once per row.  Alike terms of different couplings (Heisenberg and DM on a bond)
 // are one element: the lane then sums per class, and the class sums count for each coupling with the
 // class' coefficient at the very end.  28-site ladder, 1.43e6 rows, 3 couplings: 7.1 ms with one
-// warp per row (k_coupling_products), 2.3 ms with one lane per element; the scan and its
-// bookkeeping bound it.
+// warp per row (k_coupling_products), 2.3 ms with one lane per element, 1.8 ms with alike terms
+// merged (FP64 pipe 75 %: every element was added to every sum under a predicate), 1.4 ms with the
+// element's sum picked by selects and multiply-adds at the rows' ends.
 #include "matvec_launch.cuh"
 #include "rowsums.cuh"
 
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(kCouplingThreads, 1)
   const double2* __restrict__ xs = reinterpret_cast<const double2*>(s.xs);
   const double2* __restrict__ x = reinterpret_cast<const double2*>(s.x);
   const int lane = g.lane;
+  const int n_sums = p.off.rows.merged ? p.off.rows.n_cls : nc;
   double2 tot[kMaxCouplings], dtot[kMaxCouplings];
 #pragma unroll
   for (int c = 0; c < kMaxCouplings; ++c) tot[c] = dtot[c] = make_double2(0.0, 0.0);
@@ -224,13 +226,16 @@ __global__ void __launch_bounds__(kCouplingThreads, 1)
         for (int e = 0; e < E; ++e) xv[e] = j[e] != Group::kAbsent ? __ldg(xs + j[e]) : make_double2(0.0, 0.0);
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-          const bool here = j[e] != Group::kAbsent;
-          const int cid = class_of_off[(g.template tab<uint32_t>(L.off_ti)[term[e]] >> 16) & 0xffu];
-          double2 v = make_double2(0.0, 0.0);
+          // the element's sum is picked and put back by selects: a multiply-add per component, where
+          // an addition to each sum under a predicate took the FP64 pipe for all of them
+          const int of_term = class_of_off[(g.template tab<uint32_t>(L.off_ti)[term[e]] >> 16) & 0xffu];
+          const int cid = j[e] != Group::kAbsent ? of_term : kMaxCouplings;
+          double2 v = acc[0];
+#pragma unroll
+          for (int c = 1; c < kMaxCouplings; ++c) v = c == cid ? acc[c] : v;
           Column<kColComplex>::mac(v, flip_sign(coef[w[e] & 0x7fffffffu], w[e] & 0x80000000u), xv[e]);
 #pragma unroll
-          for (int c = 0; c < kMaxCouplings; ++c)
-            if (here && c == cid) acc[c] = add_v(acc[c], v);
+          for (int c = 0; c < kMaxCouplings; ++c) acc[c] = c == cid ? v : acc[c];
         }
       });
       // this lane's row: conj(g_i) / n_i times its sums
@@ -238,12 +243,10 @@ __global__ void __launch_bounds__(kCouplingThreads, 1)
       const double inv = __shfl_sync(0xffffffffu, g.inv_l, r);
       if (r < g.nr && inv != 0.0) {
         const double2 gi = __ldg(gv + row0 + r);
-        const C2 wi{gi.x * inv, -gi.y * inv};
+        const double2 wi = make_double2(gi.x * inv, -gi.y * inv);
 #pragma unroll
-        for (int c = 0; c < kMaxCouplings; ++c) {
-          const C2 v = cmul(wi, C2{acc[c].x, acc[c].y});
-          tot[c] = add_v(tot[c], make_double2(v.re, v.im));
-        }
+        for (int c = 0; c < kMaxCouplings; ++c)
+          if (c < n_sums) Column<kColComplex>::mac(tot[c], wi, acc[c]);
       }
       // the diagonal: lane r holds row r's counts
       double2 d[kMaxCouplings];
@@ -260,10 +263,8 @@ __global__ void __launch_bounds__(kCouplingThreads, 1)
         const double2 gi = __ldg(gv + row0 + lane), xi = __ldg(x + row0 + lane);
         const C2 gx = cmul_conj_b(C2{xi.x, xi.y}, C2{gi.x, gi.y});  // conj(g_i) x_i
 #pragma unroll
-        for (int c = 0; c < kMaxCouplings; ++c) {
-          const C2 v = cmul(C2{d[c].x, d[c].y}, gx);
-          dtot[c] = add_v(dtot[c], make_double2(v.re, v.im));
-        }
+        for (int c = 0; c < kMaxCouplings; ++c)
+          if (c < nc) Column<kColComplex>::mac(dtot[c], d[c], make_double2(gx.re, gx.im));
       }
     }
   }
