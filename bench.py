@@ -40,10 +40,10 @@ if REPO not in sys.path:
 # DRAM bytes (read + write) of one matvec launch from an ncu capture of the same workload, with the
 # integer (ALU) pipe utilisation of that capture; summaries and commands in profiles/.
 NCU_CAPTURES = {
-    "j1j2_6x6": {"traffic": 34.214e9 + 0.265e9, "alu_pipe_pct": 68.7,
-                 "source": "profiles/k_matvec_packed_j1j2_6x6.md"},
-    "xxz24_sectors": {"traffic": 2.749e9 + 0.681e9, "alu_pipe_pct": 26.0, "fp64_pipe_pct": 80.4,
-                      "source": "profiles/k_matvec_sectors_xxz24.md"},
+    "j1j2_6x6": {"traffic": 35.633e9 + 0.258e9, "alu_pipe_pct": 71.4,
+                 "source": "profiles/k_matvec_rows.md"},
+    "xxz24_sectors": {"traffic": 2.630e9 + 0.800e9, "alu_pipe_pct": 24.5, "fp64_pipe_pct": 89.9,
+                      "source": "profiles/k_matvec_rows.md"},
 }
 
 CONFIGS = {

@@ -328,10 +328,11 @@ int ls_gpu_count_nonzeros(ls_hs_operator const *op, int64_t *nnz);
  * (NUL-terminated, truncated to size); it returns the full length; reset != 0 clears the totals. */
 int ls_gpu_set_tracing(int on);
 int ls_gpu_trace_report(char *buffer, size_t size, int reset);
-/* The kernel a matvec of `op` runs: *form = 2 for the packed projected kernel (its tables fit in
- * shared memory; *slots_per_lane = group elements per lane, 32 lanes per warp), 1 for the
- * fallback projected kernel (*slots_per_lane likewise), 0 for the thread-per-row kernel (no
- * permutation group; *slots_per_lane = 0).  Needs a built basis. */
+/* The kernel family a matvec of `op` runs: *form = 2 when the group's tables fit in shared memory
+ * (one lane per generated element where its tables fit too, else the packed kernel with one warp per
+ * row; *slots_per_lane = group elements per lane of the packed kernel, 32 lanes per warp), 1 for the
+ * fallback projected kernel (*slots_per_lane likewise), 0 without a permutation group
+ * (*slots_per_lane = 0).  Needs a built basis. */
 int ls_gpu_matvec_kernel_info(ls_hs_operator const *op, int *form, int *slots_per_lane);
 
 /* Releases the device copies of an operator's term tables (made on the first GPU use of `op`,
@@ -448,12 +449,13 @@ int ls_gpu_enumerate_noalloc(ls_hs_basis const *basis, uint64_t *d_out, int64_t 
                              int64_t *count, void *stream);
 
 /* Tuning knobs of the projected matvec kernels: threads per CTA (a multiple of 32, at most 1024;
- * 0 = each kernel's own maximum: 1024 for one right-hand side (768 for groups of more than 288
- * elements), 640 for FP64 blocks, 320 for the FP32-pair and batched kernels, lowered until the
- * shared-memory tables fit) and grid waves (the
- * grid is SMs x resident CTAs per SM x waves, one warp per row at a time; 0 = 4).  The fallback
- * kernel for groups whose packed tables do not fit (or 64-bit states) always runs 256-thread
- * CTAs. */
+ * 0 = each kernel's own choice: as many warps as their areas leave room for in shared memory,
+ * at most 1024 threads, for the lane-per-element kernels; for the packed kernels 1024 for
+ * one right-hand side (768 for groups of more than 288 elements), 640 for FP64 blocks, 320 for the
+ * FP32-pair and batched kernels, lowered until the tables fit) and grid waves
+ * (the grid is SMs x resident CTAs per SM x waves; 0 = 1 for the lane-per-element kernels, 4 for the
+ * packed ones).  The fallback kernel for groups whose packed tables do not fit (or 64-bit states) always runs
+ * 256-thread CTAs. */
 int ls_gpu_set_matvec_config(int threads_per_block, int waves);
 /* Arithmetic of complex blocks of 8 or 16 right-hand sides in the plain and the batched
  * multi-sector kernels: 0 (default) = FP64; 1 = FP32 pairs for groups of at most 64 elements,
@@ -465,7 +467,9 @@ int ls_gpu_set_matvec_config(int threads_per_block, int waves);
  * exact sum (an absolute bound: an entry that cancels to near zero keeps that error, where FP64
  * gives ~1e-16 of the same sum); H X agrees with the FP64 form to ~1e-14 relative L2.  With a small group and 16 columns the FP64
  * form is bound by GB300's FP64 pipe (4 FP64 FMAs per element and column); with a large group
- * the integer orbit scan is the bound and FP64 is faster.  One right-hand side, real vectors and
+ * the integer orbit scan is the bound and FP64 is faster.  Since the FP64 form resolves one element
+ * per lane it is the faster one on small groups as well (28-site chain, 56 sectors x 16 columns: 80.5 ms
+ * against 131.6 ms).  One right-hand side, real vectors and
  * blocks of 4 always run in FP64.  Returns LS_GPU_ERR_INVALID for other values. */
 int ls_gpu_set_block_arithmetic(int mode);
 int ls_gpu_get_block_arithmetic(void);
