@@ -990,6 +990,7 @@ struct OperatorCache {
   std::vector<int32_t> coupling;
   int n_couplings = 0;
   DeviceTermSet cpl_off, cpl_diag;
+  bool fwd_leaves = false, adj_leaves = false;  // some term takes a basis state beyond the basis' bits
 };
 
 std::unordered_map<const ls_hs_operator*, OperatorCache*> g_ops;
@@ -1037,6 +1038,23 @@ bool term_breaks_constraint(const DeviceConstraint& c, uint64_t l, uint64_t r) {
   const uint64_t lo = c.half_bits >= 64 ? ~0ull : ((1ull << c.half_bits) - 1);
   return __builtin_popcountll(l & lo) != __builtin_popcountll(r & lo) ||
          __builtin_popcountll(l & ~lo) != __builtin_popcountll(r & ~lo);
+}
+
+// The bits that a state of the operator's basis can have set.
+uint64_t state_bits(const ls_hs_operator* op) { return op->basis ? low_ones(basis_number_bits(op->basis)) : ~0ull; }
+
+// Whether all masks of the terms lie within `bits`.
+bool terms_within(const TermTable& t, uint64_t bits) {
+  uint64_t any = 0;
+  for (int k = 0; k < t.n; ++k) any |= t.m[k] | t.l[k] | t.r[k] | t.x[k] | t.s[k];
+  return (any & ~bits) == 0;
+}
+
+// Whether some term that a state within `bits` can match (through t.l) flips a bit beyond them.
+bool terms_leave(const TermTable& t, uint64_t bits) {
+  for (int k = 0; k < t.n; ++k)
+    if ((t.l[k] & ~bits) == 0 && (t.x[k] & ~bits) != 0) return true;
+  return false;
 }
 
 // Host image of the row-group tables (DeviceRowTerms): one byte block and the offsets of its arrays.
@@ -1230,8 +1248,10 @@ RowTables diag_rows(const TermTable& t, const int32_t* coupling) {
 // Appends a table to the host image of a block; its pointers are offsets until upload_block.
 // Layout: v (double2, 16-byte aligned) first, then m, l, r, x, s (uint64), xinfo (uint32),
 // then the row-group tables, each array on a 16-byte boundary.
-void pack_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal, std::vector<uint8_t>& host,
-                DeviceTerms* out, const int32_t* coupling = nullptr, int n_couplings = 0) {
+// Terms with masks beyond `bits` get no row-group tables: those kernels hold states in words of the
+// basis' width and index tables by its sites.
+void pack_terms(const TermTable& t, uint64_t bits, const DeviceConstraint& cons, bool diagonal,
+                std::vector<uint8_t>& host, DeviceTerms* out, const int32_t* coupling = nullptr, int n_couplings = 0) {
   auto put = [&](const void* src, size_t sz) {
     const size_t at = (host.size() + 15) & ~(size_t)15;
     host.resize(at + std::max<size_t>(sz, 16), 0);
@@ -1250,7 +1270,9 @@ void pack_terms(const TermTable& t, const DeviceConstraint& cons, bool diagonal,
     xinfo[k] = info;
     if (cnt != 2 || (info & kTermNeedsCheck)) all_two = 0;
   }
-  const RowTables R = diagonal ? diag_rows(t, coupling) : off_diag_rows(t, cons, coupling, n_couplings);
+  const RowTables R = !terms_within(t, bits) ? RowTables{}
+                      : diagonal             ? diag_rows(t, coupling)
+                                             : off_diag_rows(t, cons, coupling, n_couplings);
   const size_t n = (size_t)t.n;
   const size_t ov = put(t.v.data(), n * 16), om = put(t.m.data(), n * 8), ol = put(t.l.data(), n * 8);
   const size_t orr = put(t.r.data(), n * 8), ox = put(t.x.data(), n * 8), os = put(t.s.data(), n * 8);
@@ -1325,10 +1347,14 @@ OperatorCache* operator_cache(const ls_hs_operator* op) {
   // one block: an upload is an allocation and a synchronous copy (four of them: 134 us for the first
   // product of an operator on 257 states, one: 112 us)
   std::vector<uint8_t> host;
-  pack_terms(c->off, cons, false, host, &c->fwd_off.terms);
-  pack_terms(adjoint_terms(c->off), cons, false, host, &c->adj_off.terms);
-  pack_terms(c->diag, cons, true, host, &c->fwd_diag.terms);
-  pack_terms(adjoint_terms(c->diag), cons, true, host, &c->adj_diag.terms);
+  const uint64_t bits = state_bits(op);
+  const TermTable adj = adjoint_terms(c->off);
+  c->fwd_leaves = terms_leave(c->off, bits);
+  c->adj_leaves = terms_leave(adj, bits);
+  pack_terms(c->off, bits, cons, false, host, &c->fwd_off.terms);
+  pack_terms(adj, bits, cons, false, host, &c->adj_off.terms);
+  pack_terms(c->diag, bits, cons, true, host, &c->fwd_diag.terms);
+  pack_terms(adjoint_terms(c->diag), bits, cons, true, host, &c->adj_diag.terms);
   if (upload_block(host, {&c->fwd_off, &c->adj_off, &c->fwd_diag, &c->adj_diag})) {
     free_cache(c);
     return nullptr;
@@ -1415,6 +1441,9 @@ int make_problem(ls_hs_operator const* op, bool adjoint, MatvecProblem* p) {
   if (c == nullptr) return LS_GPU_ERR_CUDA;
   p->projection = !b->requires_projection ? 0 : (has_permutations(b) ? 2 : 1);
   if (p->projection == 1 && b->spin_inversion == 0) return fail(LS_GPU_ERR_INVALID, "projection without symmetries");
+  // the group acts on the basis' sites only; without one such states are absent from the index and dropped
+  if (p->projection == 2 && (adjoint ? c->adj_leaves : c->fwd_leaves))
+    return fail(LS_GPU_ERR_INVALID, "an operator term flips a site beyond the basis' sites");
   const OrbitData* norms_od = p->projection == 2 ? od : nullptr;
   const bool have_norms = ix->d_norms != nullptr && ix->norms_for == norms_od;
   bool pending = false;
@@ -1858,8 +1887,9 @@ extern "C" int ls_gpu_coupling_inner_products(ls_hs_operator const* op, int n_co
     c->n_couplings = n_couplings;
     const DeviceConstraint cons = basis_constraint(op->basis);
     std::vector<uint8_t> host;
-    pack_terms(c->off, cons, false, host, &c->cpl_off.terms, term_coupling, n_couplings);
-    pack_terms(c->diag, cons, true, host, &c->cpl_diag.terms, term_coupling + c->off.n);
+    const uint64_t bits = state_bits(op);
+    pack_terms(c->off, bits, cons, false, host, &c->cpl_off.terms, term_coupling, n_couplings);
+    pack_terms(c->diag, bits, cons, true, host, &c->cpl_diag.terms, term_coupling + c->off.n);
     if (upload_block(host, {&c->cpl_off, &c->cpl_diag})) return LS_GPU_ERR_CUDA;
   }
   p.off = c->cpl_off.terms;

@@ -38,7 +38,8 @@ __device__ __forceinline__ bool constraint_ok(const DeviceConstraint& c, uint64_
 // translation unit inlines it).
 __device__ __forceinline__ int64_t mv_index_lookup(const DeviceIndex& ix, uint64_t needle,
                                                    const uint64_t* __restrict__ binom /*65x65*/) {
-  if (ix.identity) return (int64_t)needle;
+  // (a term may flip a site beyond the basis: such states have no index)
+  if (ix.identity) return needle < (uint64_t)ix.n_states ? (int64_t)needle : -1;
   if (ix.combinadic) {
     int64_t i = 0;
     uint64_t a = needle;
@@ -47,7 +48,8 @@ __device__ __forceinline__ int64_t mv_index_lookup(const DeviceIndex& ix, uint64
       a &= a - 1;
       i += (c <= 0 || k > c) ? 0 : (int64_t)__ldg(binom + c * 65 + k);
     }
-    return i - ix.rank_base;
+    i -= ix.rank_base;
+    return i >= 0 && i < ix.n_states ? i : -1;
   }
   int64_t len = ix.range_size;
   if (len <= 0 || needle > ix.max_state) return -1;
