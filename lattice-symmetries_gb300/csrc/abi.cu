@@ -1392,22 +1392,31 @@ int ensure_norms(IndexData* ix, const OrbitData* od) {
 
 // Rank tables of a complete basis without a group: all states of a fixed weight (all below the
 // flipped maximum with spin inversion), or of fixed (N_up, N_down).  Other sets of states (installed
-// by the caller) and bases that rank_tables_for leaves out keep the search.
+// by the caller) and more than 40 bits keep the search.
 // They are made on the library's stream: *pending tells whether the caller has to wait for it.
 int ensure_ranks(IndexData* ix, ls_hs_basis const* b, bool* pending) {
   if (ix->d_ranks != nullptr || ix->n_states == 0) return 0;
-  const bool spins = b->particle_type == LS_HS_SPIN;
-  RankTables t;
-  if (!hamming_fixed(b) ||
-      !rank_tables_for(basis_number_bits(b), spins ? b->number_up : b->number_particles,
-                       b->particle_type == LS_HS_SPINFUL_FERMION ? b->number_up : -1,
-                       spins && b->spin_inversion != 0, &t) ||
-      ix->n_states != t.states)
-    return 0;
+  const int n = basis_number_bits(b);
+  if (n > 40) return 0;
+  int split = (n + 1) / 2, h = 0, species = 0;
+  int64_t n_lo = 0, expected = 0;
+  if (b->particle_type == LS_HS_SPINFUL_FERMION && b->number_up >= 0) {
+    species = 1;
+    split = b->number_sites;
+    h = b->number_particles - b->number_up;
+    n_lo = fixed_hamming_state_to_index(low_ones(b->number_up) << (split - b->number_up)) + 1;
+    expected = n_lo * (fixed_hamming_state_to_index(low_ones(h) << (split - h)) + 1);
+  } else {
+    if (!hamming_fixed(b)) return 0;
+    h = b->particle_type == LS_HS_SPIN ? b->number_up : b->number_particles;
+    expected = fixed_hamming_state_to_index(low_ones(h) << (n - h)) + 1;
+    if (b->particle_type == LS_HS_SPIN && b->spin_inversion != 0) expected /= 2;
+  }
+  if (ix->n_states != expected) return 0;
   cudaStream_t s = default_stream();
-  const size_t lo = (size_t)1 << t.split, hi = (size_t)1 << t.high_bits;
+  const size_t lo = (size_t)1 << split, hi = (size_t)1 << (n - split);
   if (!cuda_ok(cudaMalloc((void**)&ix->d_ranks, (lo + hi) * 4), "cudaMalloc(ranks)")) return LS_GPU_ERR_CUDA;
-  const int rc = launch_rank_tables(t, ix->d_ranks, ix->d_ranks + lo, s);
+  const int rc = launch_rank_tables(split, n - split, h, species, n_lo, ix->d_ranks, ix->d_ranks + lo, s);
   if (rc != 0) {
     cudaFree(ix->d_ranks);
     ix->d_ranks = nullptr;
@@ -1415,7 +1424,7 @@ int ensure_ranks(IndexData* ix, ls_hs_basis const* b, bool* pending) {
   }
   ix->dev.rank_lo = ix->d_ranks;
   ix->dev.rank_hi = ix->d_ranks + lo;
-  ix->dev.rank_split = t.split;
+  ix->dev.rank_split = split;
   *pending = true;
   return 0;
 }

@@ -10,7 +10,6 @@
 #include <cuda_runtime.h>
 
 #include "ls_gb300.h"
-#include "ranks.h"
 #include "trace.h"
 
 namespace lsg {
@@ -286,7 +285,8 @@ double* prescaled_copy(const MatvecProblem& p, int words, int k, const double* d
 bool free_fits(const MatvecProblem& p);
 int launch_free(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y, int64_t ldy,
                 int* d_err, cudaStream_t s);
-int launch_rank_tables(const RankTables& t, uint32_t* d_lo, uint32_t* d_hi, cudaStream_t s);
+int launch_rank_tables(int split, int high_bits, int h, int species, int64_t n_lo, uint32_t* d_lo, uint32_t* d_hi,
+                       cudaStream_t s);
 
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,
                   double* d_y, int64_t ldy, int* d_err, cudaStream_t s);

@@ -83,12 +83,14 @@ __global__ void k_rank_tables(int split, int high_bits, int h, int species, int6
   }
 }
 
-int launch_rank_tables(const RankTables& t, uint32_t* d_lo, uint32_t* d_hi, cudaStream_t s) {
+int launch_rank_tables(int split, int high_bits, int h, int species, int64_t n_lo, uint32_t* d_lo, uint32_t* d_hi,
+                       cudaStream_t s) {
+
   const uint64_t* binom = device_binomials();
   if (binom == nullptr) return LS_GPU_ERR_CUDA;
-  const int64_t n = ((int64_t)1 << t.split) + ((int64_t)1 << t.high_bits);
+  const int64_t n = ((int64_t)1 << split) + ((int64_t)1 << high_bits);
   const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms() * 8);
-  k_rank_tables<<<blocks, 256, 0, s>>>(t.split, t.high_bits, t.h, t.species, t.n_low, binom, d_lo, d_hi);
+  k_rank_tables<<<blocks, 256, 0, s>>>(split, high_bits, h, species, n_lo, binom, d_lo, d_hi);
   return cuda_ok(cudaGetLastError(), "k_rank_tables") ? 0 : LS_GPU_ERR_CUDA;
 }
 
