@@ -499,6 +499,7 @@ extern "C" ls_hs_state_index_binary_search_data* ls_hs_create_state_index_binary
   cudaStream_t s = default_stream();
   auto it = g_pending_device_reps.find(representatives->elts);
   if (it != g_pending_device_reps.end()) {
+    ix->enumerated = true;
     ix->d_reps = it->second.reps;
     ix->d_norms = it->second.norms;
     if (ix->d_norms != nullptr) {
@@ -1391,11 +1392,12 @@ int ensure_norms(IndexData* ix, const OrbitData* od) {
 }
 
 // Rank tables of a complete basis without a group: all states of a fixed weight (all below the
-// flipped maximum with spin inversion), or of fixed (N_up, N_down).  Other sets of states (installed
-// by the caller) and more than 40 bits keep the search.
+// flipped maximum with spin inversion), or of fixed (N_up, N_down).  More than 40 bits keep the search,
+// and so do states installed by the caller that are not the whole basis: the kernels read x at a rank
+// unchecked, so every installed state is compared with its own once.
 // They are made on the library's stream: *pending tells whether the caller has to wait for it.
 int ensure_ranks(IndexData* ix, ls_hs_basis const* b, bool* pending) {
-  if (ix->d_ranks != nullptr || ix->n_states == 0) return 0;
+  if (ix->d_ranks != nullptr || ix->ranks_refused || ix->n_states == 0) return 0;
   const int n = basis_number_bits(b);
   if (n > 40) return 0;
   int split = (n + 1) / 2, h = 0, species = 0;
@@ -1415,11 +1417,24 @@ int ensure_ranks(IndexData* ix, ls_hs_basis const* b, bool* pending) {
   if (ix->n_states != expected) return 0;
   cudaStream_t s = default_stream();
   const size_t lo = (size_t)1 << split, hi = (size_t)1 << (n - split);
-  if (!cuda_ok(cudaMalloc((void**)&ix->d_ranks, (lo + hi) * 4), "cudaMalloc(ranks)")) return LS_GPU_ERR_CUDA;
-  const int rc = launch_rank_tables(split, n - split, h, species, n_lo, ix->d_ranks, ix->d_ranks + lo, s);
-  if (rc != 0) {
+  if (!cuda_ok(cudaMalloc((void**)&ix->d_ranks, (lo + hi + 1) * 4), "cudaMalloc(ranks)")) return LS_GPU_ERR_CUDA;
+  int bad = 0;
+  int* d_bad = (int*)(ix->d_ranks + lo + hi);
+  int rc = launch_rank_tables(split, n - split, h, species, n_lo, ix->d_ranks, ix->d_ranks + lo, s);
+  if (rc == 0 && !ix->enumerated) {
+    if (!cuda_ok(cudaMemsetAsync(d_bad, 0, 4, s), "clear rank check")) rc = LS_GPU_ERR_CUDA;
+    if (rc == 0)
+      rc = launch_check_ranks(split, n, basis_constraint(b), ix->d_reps, ix->n_states, ix->d_ranks, ix->d_ranks + lo,
+                              d_bad, s);
+    if (rc == 0 && (!cuda_ok(cudaMemcpyAsync(&bad, d_bad, 4, cudaMemcpyDeviceToHost, s), "read rank check") ||
+                    !cuda_ok(cudaStreamSynchronize(s), "rank check")))
+      rc = LS_GPU_ERR_CUDA;
+  }
+  if (rc != 0 || bad != 0) {
+    cudaStreamSynchronize(s);
     cudaFree(ix->d_ranks);
     ix->d_ranks = nullptr;
+    ix->ranks_refused = rc == 0;
     return rc;
   }
   ix->dev.rank_lo = ix->d_ranks;

@@ -183,6 +183,8 @@ struct IndexData {
   double* d_norms = nullptr;          // filled lazily when a projected matvec needs them
   const OrbitData* norms_for = nullptr;
   uint32_t* d_ranks = nullptr;        // rank_lo | rank_hi of DeviceIndex, filled by the first matvec without a group
+  bool enumerated = false;            // the states come from this library's enumeration
+  bool ranks_refused = false;         // ... or from the caller, and are not the complete basis
 };
 
 constexpr uint32_t kOrbitMagic = 0x4f524249u;  // "ORBI"
@@ -287,6 +289,8 @@ int launch_free(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int
                 int* d_err, cudaStream_t s);
 int launch_rank_tables(int split, int high_bits, int h, int species, int64_t n_lo, uint32_t* d_lo, uint32_t* d_hi,
                        cudaStream_t s);
+int launch_check_ranks(int split, int n_bits, const DeviceConstraint& constraint, const uint64_t* d_reps, int64_t n,
+                       const uint32_t* d_lo, const uint32_t* d_hi, int* d_bad, cudaStream_t s);
 
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,
                   double* d_y, int64_t ldy, int* d_err, cudaStream_t s);

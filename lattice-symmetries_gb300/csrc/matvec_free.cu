@@ -94,6 +94,25 @@ int launch_rank_tables(int split, int high_bits, int h, int species, int64_t n_l
   return cuda_ok(cudaGetLastError(), "k_rank_tables") ? 0 : LS_GPU_ERR_CUDA;
 }
 
+// Sets *bad unless state i of a caller's set has rank i, the basis' weights and no bit beyond the basis.
+__global__ void k_check_ranks(const uint64_t* __restrict__ reps, int64_t n, DeviceConstraint constraint, int split,
+                              int n_bits, const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
+                              int* __restrict__ bad) {
+  const uint64_t low_mask = ((uint64_t)1 << split) - 1;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t a = __ldg(reps + i);
+    if ((a >> n_bits) != 0 || !constraint_ok(constraint, a) || hi[a >> split] + lo[a & low_mask] != (uint32_t)i)
+      *bad = 1;
+  }
+}
+
+int launch_check_ranks(int split, int n_bits, const DeviceConstraint& constraint, const uint64_t* d_reps, int64_t n,
+                       const uint32_t* d_lo, const uint32_t* d_hi, int* d_bad, cudaStream_t s) {
+  const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms() * 8);
+  k_check_ranks<<<blocks, 256, 0, s>>>(d_reps, n, constraint, split, n_bits, d_lo, d_hi, d_bad);
+  return cuda_ok(cudaGetLastError(), "k_check_ranks") ? 0 : LS_GPU_ERR_CUDA;
+}
+
 template <typename State, bool INV, int COL>
 __global__ void __launch_bounds__(kFreeThreads, 2)
     k_matvec_free(const MatvecProblem p, const FreeLayout L, const double* __restrict__ x_, int64_t ldx,
