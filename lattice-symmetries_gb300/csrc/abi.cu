@@ -1894,6 +1894,9 @@ extern "C" int ls_gpu_coupling_inner_products(ls_hs_operator const* op, int n_co
   for (int t = 0; t < n_terms; ++t)
     if (term_coupling[t] < 0 || term_coupling[t] >= n_couplings)
       return fail(LS_GPU_ERR_INVALID, "term coupling id out of range");
+  // before tables of n_couplings x terms are made (callers try this form first, with any number)
+  rc = coupling_products_allowed(p, n_couplings);
+  if (rc != 0) return rc;
   if (c->cpl_off.block == nullptr || c->coupling.size() != (size_t)n_terms || c->n_couplings != n_couplings ||
       (n_terms > 0 && memcmp(c->coupling.data(), term_coupling, (size_t)n_terms * 4) != 0)) {
     if (c->cpl_off.block) cudaFree(c->cpl_off.block);

@@ -335,14 +335,20 @@ static int launch_coupling_rows(const MatvecProblem& p, int nc, const double* d_
   return rc;
 }
 
-int launch_coupling_products(const MatvecProblem& p, int nc, const double* d_g, const double* d_x, double* d_out,
-                             int* d_err, cudaStream_t s) {
+int coupling_products_allowed(const MatvecProblem& p, int nc) {
   if (nc < 1 || nc > kMaxCouplings)
     return fail(LS_GPU_ERR_INVALID, "the fused coupling kernel handles 1 to 4 couplings");
   if (p.projection != 2 || p.group.gpl < 1 || p.group.gpl > 4 || p.group.onehot_packed == nullptr)
     return fail(LS_GPU_ERR_INVALID, "the fused coupling kernel needs a basis with lattice symmetries of at most "
                                     "128 elements");
   if (p.group.fermionic) return fail(LS_GPU_ERR_INVALID, "the fused coupling kernel has no fermionic signs");
+  return 0;
+}
+
+int launch_coupling_products(const MatvecProblem& p, int nc, const double* d_g, const double* d_x, double* d_out,
+                             int* d_err, cudaStream_t s) {
+  const int allowed = coupling_products_allowed(p, nc);
+  if (allowed != 0) return allowed;
   if (p.off.coupling == nullptr) return fail(LS_GPU_ERR_INVALID, "operator terms carry no coupling ids");
   const uint64_t* binom = device_binomials();
   if (binom == nullptr) return LS_GPU_ERR_CUDA;

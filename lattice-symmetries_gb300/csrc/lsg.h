@@ -321,6 +321,8 @@ int launch_apply_off_diag(const DeviceTerms& off, int64_t count, const uint64_t*
 // out = in^T for a row-major rows x cols matrix of doubles (apply.cu).
 int launch_transpose(const double* d_in, double* d_out, int64_t rows, int64_t cols, cudaStream_t s);
 
+// 0 where launch_coupling_products takes this number of couplings on this basis, else the error code.
+int coupling_products_allowed(const MatvecProblem& p, int n_couplings);
 int launch_coupling_products(const MatvecProblem& p, int n_couplings, const double* d_g,
                              const double* d_x, double* d_out, int* d_err, cudaStream_t s);
 
