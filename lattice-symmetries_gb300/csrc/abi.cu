@@ -1044,6 +1044,13 @@ bool term_breaks_constraint(const DeviceConstraint& c, uint64_t l, uint64_t r) {
 // The bits that a state of the operator's basis can have set.
 uint64_t state_bits(const ls_hs_operator* op) { return op->basis ? low_ones(basis_number_bits(op->basis)) : ~0ull; }
 
+// Whether the terms' coefficients are finite.
+bool terms_finite(const TermTable& t) {
+  for (const double v : t.v)
+    if (!std::isfinite(v)) return false;
+  return true;
+}
+
 // Whether all masks of the terms lie within `bits`.
 bool terms_within(const TermTable& t, uint64_t bits) {
   uint64_t any = 0;
@@ -1250,7 +1257,8 @@ RowTables diag_rows(const TermTable& t, const int32_t* coupling) {
 // Layout: v (double2, 16-byte aligned) first, then m, l, r, x, s (uint64), xinfo (uint32),
 // then the row-group tables, each array on a 16-byte boundary.
 // Terms with masks beyond `bits` get no row-group tables: those kernels hold states in words of the
-// basis' width and index tables by its sites.
+// basis' width and index tables by its sites.  Nor do terms with an infinite coefficient (a hard
+// constraint): counts of a class times its value are no sum over the matching terms then, 0 * inf.
 void pack_terms(const TermTable& t, uint64_t bits, const DeviceConstraint& cons, bool diagonal,
                 std::vector<uint8_t>& host, DeviceTerms* out, const int32_t* coupling = nullptr, int n_couplings = 0) {
   auto put = [&](const void* src, size_t sz) {
@@ -1271,9 +1279,9 @@ void pack_terms(const TermTable& t, uint64_t bits, const DeviceConstraint& cons,
     xinfo[k] = info;
     if (cnt != 2 || (info & kTermNeedsCheck)) all_two = 0;
   }
-  const RowTables R = !terms_within(t, bits) ? RowTables{}
-                      : diagonal             ? diag_rows(t, coupling)
-                                             : off_diag_rows(t, cons, coupling, n_couplings);
+  RowTables R;
+  if (terms_within(t, bits) && terms_finite(t))
+    R = diagonal ? diag_rows(t, coupling) : off_diag_rows(t, cons, coupling, n_couplings);
   const size_t n = (size_t)t.n;
   const size_t ov = put(t.v.data(), n * 16), om = put(t.m.data(), n * 8), ol = put(t.l.data(), n * 8);
   const size_t orr = put(t.r.data(), n * 8), ox = put(t.x.data(), n * 8), os = put(t.s.data(), n * 8);
