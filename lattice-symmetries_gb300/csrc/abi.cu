@@ -1512,9 +1512,13 @@ int make_problem(ls_hs_operator const* op, bool adjoint, MatvecProblem* p) {
 
 // One pinned read and one synchronisation; the word is cleared only when it is set.
 int read_and_clear_error(cudaStream_t s) {
+  int pageable[4] = {0, 0, 0, 0};  // where there is no pinned memory
   int* h = (int*)pinned_scratch(4 * sizeof(int), 11);
+  if (h == nullptr) {
+    cudaGetLastError();
+    h = pageable;
+  }
   int* d = device_error_word();
-  if (h == nullptr) return LS_GPU_ERR_CUDA;
   if (!cuda_ok(cudaMemcpyAsync(h, d, 4 * sizeof(int), cudaMemcpyDeviceToHost, s), "read error word") ||
       !cuda_ok(cudaStreamSynchronize(s), "matvec"))
     return LS_GPU_ERR_CUDA;
