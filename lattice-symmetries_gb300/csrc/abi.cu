@@ -472,11 +472,13 @@ extern "C" void ls_hs_is_representative_halide_kernel(ptrdiff_t batch_size, uint
 // State index (indexing.c:94-125, :273-325)
 // =================================================================================================
 namespace {
-// Device copies of representatives (and their orbit norms) produced by the GPU enumeration, keyed by
-// the host array they were copied to, so that building the index does not upload them again.
+// Device copies of representatives (and their orbit norms or stabilisers) produced by the GPU
+// enumeration, keyed by the host array they were copied to, so that building the index does not upload
+// them again.
 struct PendingStates {
   uint64_t* reps;
-  double* norms;  // norms | inverse norms (projected bases), or null
+  double* norms;   // norms | inverse norms (projected bases), or null
+  uint16_t* stab;  // stabiliser sizes, or null
   const OrbitData* norms_for;
 };
 std::unordered_map<const void*, PendingStates> g_pending_device_reps;
@@ -507,6 +509,8 @@ extern "C" ls_hs_state_index_binary_search_data* ls_hs_create_state_index_binary
       ix->dev.norms = ix->d_norms;
       ix->dev.inv_norms = ix->d_norms + std::max<int64_t>(ix->n_states, 1);
     }
+    ix->d_stab = it->second.stab;
+    ix->stab_for = it->second.norms_for;
     g_pending_device_reps.erase(it);
   } else {
     if (!cuda_ok(cudaMalloc((void**)&ix->d_reps, std::max<int64_t>(ix->n_states, 1) * 8), "cudaMalloc(reps)") ||
@@ -527,6 +531,7 @@ extern "C" ls_hs_state_index_binary_search_data* ls_hs_create_state_index_binary
     report("ls_hs_create_state_index_binary_search_kernel_data");
     cudaFree(ix->d_reps);
     cudaFree(ix->d_norms);
+    cudaFree(ix->d_stab);
     delete ix;
     return nullptr;
   }
@@ -548,6 +553,7 @@ extern "C" void ls_hs_destroy_state_index_binary_search_kernel_data(
   cudaFree(cache->d_offsets);
   cudaFree(cache->d_suffix);
   cudaFree(cache->d_norms);
+  cudaFree(cache->d_stab);
   cudaFree(cache->d_ranks);
   cache->magic = 0;
   delete cache;
@@ -719,7 +725,7 @@ extern "C" int ls_gpu_set_enumeration_rule(int exact) {
   return previous;
 }
 
-static int enumerate_into(ls_hs_basis const* b, uint64_t** d_out, double** d_norms, int64_t* count) {
+static int enumerate_into(ls_hs_basis const* b, uint64_t** d_out, double** d_norms, uint16_t** d_stab, int64_t* count) {
   EnumerateRequest req{};
   uint64_t lo, hi;
   state_estimates(b, &lo, &hi);
@@ -753,7 +759,7 @@ static int enumerate_into(ls_hs_basis const* b, uint64_t** d_out, double** d_nor
     req.spin_inversion = 0;
   }
   if (req.mode == 1 && b->particle_type == LS_HS_SPINFUL_FERMION) req.number_sites = 2 * b->number_sites;
-  return enumerate_states(g, req, d_out, d_norms, count, default_stream());
+  return enumerate_states(g, req, d_out, d_norms, d_stab, count, default_stream());
 }
 
 // Allocation-free enumeration for callers that cannot allocate device memory; see
@@ -810,9 +816,10 @@ extern "C" void ls_chpl_enumerate_representatives(ls_hs_basis* p, uint64_t lower
   }
   uint64_t* d = nullptr;
   double* norms = nullptr;
+  uint16_t* stab = nullptr;
   int64_t n = 0;
   cudaStream_t s = default_stream();
-  if (enumerate_into(p, &d, &norms, &n) != 0) {
+  if (enumerate_into(p, &d, &norms, &stab, &n) != 0) {
     report("ls_chpl_enumerate_representatives");
     return;
   }
@@ -822,10 +829,11 @@ extern "C" void ls_chpl_enumerate_representatives(ls_hs_basis* p, uint64_t lower
       !cuda_ok(cudaStreamSynchronize(s), "enumerate")) {
     cudaFree(d);
     cudaFree(norms);
+    cudaFree(stab);
     report("ls_chpl_enumerate_representatives");
     return;
   }
-  g_pending_device_reps[h] = PendingStates{d, norms, basis_orbit(p)};
+  g_pending_device_reps[h] = PendingStates{d, norms, stab, basis_orbit(p)};
   dest->elts = h;
   dest->num_elts = (uint64_t)n;
   dest->freer = (void*)&free_pinned;
@@ -1383,8 +1391,15 @@ int ensure_norms(IndexData* ix, const OrbitData* od) {
   int rc;
   if (od != nullptr && od->n_elems > 0) {
     const DeviceGroup* dg = orbit_device(od);
-    rc = dg ? launch_orbit_norms(*dg, ix->n_states, ix->d_reps, ix->d_norms, s) : LS_GPU_ERR_CUDA;
-    if (rc == 0) rc = launch_inverse_norms(ix->d_norms, ix->n_states, ix->d_norms + n, s);
+    if (dg == nullptr) {
+      rc = LS_GPU_ERR_CUDA;
+    } else if (ix->d_stab != nullptr && ix->stab_for == od) {
+      rc = launch_norms_of_stabilisers(ix->d_stab, ix->n_states, dg->n_elems * (dg->spin_inversion != 0 ? 2 : 1),
+                                       ix->d_norms, ix->d_norms + n, s);
+    } else {
+      rc = launch_orbit_norms(*dg, ix->n_states, ix->d_reps, ix->d_norms, s);
+      if (rc == 0) rc = launch_inverse_norms(ix->d_norms, ix->n_states, ix->d_norms + n, s);
+    }
   } else {
     rc = launch_unit_norms(ix->d_norms, 2 * n, s);
   }
@@ -1395,6 +1410,10 @@ int ensure_norms(IndexData* ix, const OrbitData* od) {
     ix->norms_for = od;
     ix->dev.norms = ix->d_norms;
     ix->dev.inv_norms = ix->d_norms + n;
+    if (ix->stab_for == od) {
+      cudaFree(ix->d_stab);
+      ix->d_stab = nullptr;
+    }
   }
   return rc;
 }

@@ -714,7 +714,7 @@ struct EnumArgs {
   int32_t* tile_count;
   int64_t* tile_start;
   uint64_t* append;
-  uint16_t* append_stab;  // stabiliser sizes (0: a non-trivial character); at most 2 * kMaxGroupElements
+  uint16_t* append_stab;  // stabiliser sizes (0: a non-trivial character; at most 2 * kMaxGroupElements), or null
   int64_t capacity;
   unsigned long long* counter;
   // Spinful fermions (mode 3): candidate (iB, iA) = (idx / nA, idx % nA) is
@@ -1110,7 +1110,7 @@ __global__ void __launch_bounds__(kPruneThreads, 1) k_enumerate_pruned(DeviceGro
         const int64_t to = at + __popc(m & ((1u << lane) - 1u));
         if (((m >> lane) & 1u) && to < a.capacity) {
           a.append[to] = kept[32 * w + lane];
-          a.append_stab[to] = kept_stab[32 * w + lane];
+          if (a.append_stab != nullptr) a.append_stab[to] = kept_stab[32 * w + lane];
         }
         for (int i = w; i < min(w + kPruneWarps, segments); ++i) at += __popc(flags[i]);
       }
@@ -1132,7 +1132,7 @@ __global__ void k_gather_runs(int64_t n_tiles, const int32_t* __restrict__ tile_
     const int64_t src = tile_start[t], dst = tile_offset[t];
     for (int k = lane; k < c; k += 32) {
       out[dst + k] = append[src + k];
-      out_stab[dst + k] = append_stab[src + k];
+      if (out_stab != nullptr) out_stab[dst + k] = append_stab[src + k];
     }
   }
 }
@@ -1154,6 +1154,19 @@ __global__ void k_norms_of_stabilisers(const uint16_t* __restrict__ stab, int64_
     inv_norms[i] = inverse;
   }
 }
+
+int launch_norms_of_stabilisers(const uint16_t* d_stab, int64_t n, int group_elements, double* d_norms, double* d_inv,
+                                cudaStream_t s) {
+  if (n <= 0) return 0;
+  StageScope stage("basis.orbit_norms", s);
+  k_norms_of_stabilisers<<<grid_for(n, 256), 256, 0, s>>>(d_stab, n, (double)group_elements, d_norms, d_inv);
+  return cuda_ok(cudaGetLastError(), "k_norms_of_stabilisers") ? 0 : LS_GPU_ERR_CUDA;
+}
+
+// Bases of up to this many states get their norms (16 bytes per state: 64 MB) with the states, so that the
+// first product saves an allocation and a wait (of ~110 us for a few hundred states).  Larger ones
+// keep the stabiliser sizes (2 bytes) until norms are asked for: a program that only builds never pays them.
+constexpr int64_t kNormsAtOnce = (int64_t)1 << 22;
 
 // Unprojected: out[i] = unrank(first_rank + i) (fixed weight) or first + i.
 __global__ void k_enumerate_plain(int64_t first_rank, int64_t n, int h, int n_bits,
@@ -1188,10 +1201,19 @@ __global__ void k_enumerate_spinful(int64_t rankA, int64_t nA, int hA, int64_t r
   }
 }
 
+// Device memory that the caller can do without: null when there is none.
+static void* optional_alloc(size_t bytes) {
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
+}
+
 int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_t** d_out,
-                     double** d_norms, int64_t* count, cudaStream_t s) {
+                     double** d_norms, uint16_t** d_stab, int64_t* count, cudaStream_t s) {
   *d_out = nullptr;
   *d_norms = nullptr;
+  *d_stab = nullptr;
   *count = 0;
   if (ensure_binomials() != 0) return LS_GPU_ERR_CUDA;
   const int n_bits = (req.mode == 2 || req.mode == 3) ? 2 * req.number_sites : req.number_sites;
@@ -1307,11 +1329,12 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
   q.next = counter + 1;
   unsigned long long total = 0;
   for (int attempt = 0; attempt < 2; ++attempt) {
-    if (!cuda_ok(cudaMalloc((void**)&append, std::max<int64_t>(capacity, 1) * 8), "alloc append") ||
-        !cuda_ok(cudaMalloc((void**)&append_stab, std::max<int64_t>(capacity, 1) * 2), "alloc append")) {
+    if (!cuda_ok(cudaMalloc((void**)&append, std::max<int64_t>(capacity, 1) * 8), "alloc append")) {
       cleanup();
       return LS_GPU_ERR_CUDA;
     }
+    // without memory for them the norms are computed from the states (launch_orbit_norms)
+    append_stab = (uint16_t*)optional_alloc((size_t)std::max<int64_t>(capacity, 1) * 2);
     a.tile_count = tile_count;
     a.tile_start = tile_start;
     a.append = append;
@@ -1338,17 +1361,14 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
     capacity = (int64_t)total;
   }
   uint64_t* out = nullptr;
-  double* norms = nullptr;  // norms | inverse norms
-  uint16_t* out_stab = nullptr;
   const size_t n_out = (size_t)std::max<unsigned long long>(total, 1);
-  if (!cuda_ok(cudaMalloc((void**)&out, n_out * 8), "alloc out") ||
-      !cuda_ok(cudaMalloc((void**)&norms, n_out * 16), "alloc norms") ||
-      !cuda_ok(cudaMalloc((void**)&out_stab, n_out * 2), "alloc stabilisers")) {
+  if (!cuda_ok(cudaMalloc((void**)&out, n_out * 8), "alloc out")) {
     cleanup();
-    cudaFree(out);
-    cudaFree(norms);
     return LS_GPU_ERR_CUDA;
   }
+  uint16_t* out_stab = append_stab != nullptr ? (uint16_t*)optional_alloc(n_out * 2) : nullptr;
+  double* norms = nullptr;  // norms | inverse norms
+  if (out_stab != nullptr && (int64_t)total <= kNormsAtOnce) norms = (double*)optional_alloc(n_out * 16);
   int rc = 0;
   {
     StageScope stage("basis.enumerate_compact", s);
@@ -1357,17 +1377,18 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
       k_gather_runs<<<grid_for(a.n_tiles * 32, 256), 256, 0, s>>>(a.n_tiles, tile_count, tile_start,
                                                                  tile_offset, append, append_stab, out, out_stab);
   }
-  if (rc == 0) {
-    StageScope stage("basis.orbit_norms", s);
-    k_norms_of_stabilisers<<<grid_for((int64_t)n_out, 256), 256, 0, s>>>(
-        out_stab, (int64_t)total, (double)g.n_elems * (g.spin_inversion != 0 ? 2 : 1), norms, norms + n_out);
-  }
+  if (rc == 0 && norms != nullptr)
+    rc = launch_norms_of_stabilisers(out_stab, (int64_t)total, g.n_elems * (g.spin_inversion != 0 ? 2 : 1), norms,
+                                     norms + n_out, s);
   if (rc == 0) {
     if (!cuda_ok(cudaGetLastError(), "k_gather_runs") || !cuda_ok(cudaStreamSynchronize(s), "gather"))
       rc = LS_GPU_ERR_CUDA;
   }
   cleanup();
-  cudaFree(out_stab);
+  if (rc != 0 || norms != nullptr) {
+    cudaFree(out_stab);
+    out_stab = nullptr;
+  }
   if (rc != 0) {
     cudaFree(out);
     cudaFree(norms);
@@ -1375,6 +1396,7 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
   }
   *d_out = out;
   *d_norms = norms;
+  *d_stab = out_stab;
   *count = (int64_t)total;
   return 0;
 }

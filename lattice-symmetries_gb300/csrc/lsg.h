@@ -182,6 +182,8 @@ struct IndexData {
   uint16_t* d_suffix = nullptr;       // 2-byte key suffixes (shift <= 16)
   double* d_norms = nullptr;          // filled lazily when a projected matvec needs them
   const OrbitData* norms_for = nullptr;
+  uint16_t* d_stab = nullptr;         // stabiliser sizes from the enumeration (group stab_for) until the norms are made
+  const OrbitData* stab_for = nullptr;
   uint32_t* d_ranks = nullptr;        // rank_lo | rank_hi of DeviceIndex, filled by the first matvec without a group
   bool enumerated = false;            // the states come from this library's enumeration
   bool ranks_refused = false;         // ... or from the caller, and are not the complete basis
@@ -223,9 +225,13 @@ struct EnumerateRequest {
   int reference_norm_rule;  // 1: keep a state iff the reference's floating stabiliser sum > 0
 };
 // Enumerates into device memory; *d_out is allocated with cudaMalloc (caller frees).  Projected
-// bases also get *d_norms (cudaMalloc): the orbit norms [n] and their inverses [n], n >= 1; else null.
+// bases also get, where there is memory, *d_norms (cudaMalloc): the orbit norms [n] and their inverses
+// [n], n >= 1; or, for many states, *d_stab: the sizes of the stabilisers, from which
+// launch_norms_of_stabilisers makes them.  Otherwise both are null.
 int enumerate_states(const DeviceGroup* g, const EnumerateRequest& req, uint64_t** d_out,
-                     double** d_norms, int64_t* count, cudaStream_t s);
+                     double** d_norms, uint16_t** d_stab, int64_t* count, cudaStream_t s);
+int launch_norms_of_stabilisers(const uint16_t* d_stab, int64_t n, int group_elements, double* d_norms, double* d_inv,
+                                cudaStream_t s);
 // Enumerates into the caller's d_out (capacity entries) without allocating: all scratch lives in
 // a static device array (see basis.cu).  *count receives the number of states.
 int enumerate_states_noalloc(const OrbitData* od, const EnumerateRequest& req, uint64_t* d_out,
