@@ -64,6 +64,8 @@ def test_symmetric_bases_refuse_a_flip_beyond_them():
     x = torch.from_numpy(np.random.default_rng(3).normal(size=basis.number_states)).cuda()
     plain = ls.Operator(basis, H).apply_device(x)
     with_z = ls.Operator(basis, H + ls.Expr("σᶻ₀", sites=[[8]])).apply_device(x)
-    sign = ls.Operator(basis, ls.Expr("σᶻ₀", sites=[[8]])).apply_diag_to_basis_state(int(basis.states[0]))
+    free = ls.SpinBasis(8, 4)
+    free.build()
+    sign = ls.Operator(free, ls.Expr("σᶻ₀", sites=[[8]])).apply_diag_to_basis_state(int(basis.states[0]))
     assert abs(sign) == 1.0
     assert float((with_z - plain - sign * x).norm()) <= RTOL * float(plain.norm())
