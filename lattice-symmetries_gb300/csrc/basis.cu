@@ -16,7 +16,7 @@
 //  * enumeration: candidates in increasing order (combinadics unrank + Gosper steps,
 //    StatesEnumeration.chpl:29-32) in tiles; tiles whose common top bits already have a smaller
 //    image are dropped whole, the others tested against the group elements that those bits leave
-//    open; a run per tile in an append buffer, an exclusive scan over tile counts, and a final
+//    open (small groups: every candidate by a thread of its own); a run per tile in an append buffer, an exclusive scan over tile counts, and a final
 //    ordered gather; the output is sorted.
 //  * state index: the prefix-bucket table of kernels/indexing.c:45-117 built on the GPU and
 //    a branch-free window search (indexing.c:196-215).
@@ -1118,6 +1118,82 @@ __global__ void __launch_bounds__(kPruneThreads, 1) k_enumerate_pruned(DeviceGro
   }
 }
 
+// Projected enumeration, a thread per candidate: 16 consecutive candidates each, a Benes network per group
+// element until an image is smaller, survivors to a run per tile.  With few images most candidates
+// fall to one of the first or are kept, and the block tests above cost more than they save: 2.7e6
+// candidates of 24 spins, groups of 2 / 8 / 12 / 24 elements, 0.08 / 0.15 / 0.16 / 0.24 ms here and
+// 0.49 / 0.24 / 0.20 / 0.18 ms by pruned blocks.
+template <int DEPTH>
+__global__ void __launch_bounds__(kEnumThreads) k_enumerate_candidates(DeviceGroup g, EnumArgs a) {
+  __shared__ int64_t warp_sums[32];
+  __shared__ int64_t total;
+  __shared__ unsigned long long base_slot;
+  __shared__ uint16_t stabilisers[kEnumTile];
+  uint16_t* stab = stabilisers + threadIdx.x * kEnumPerThread;
+  for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
+    const int64_t first = tile * kEnumTile + (int64_t)threadIdx.x * kEnumPerThread;
+    uint32_t bits = 0;
+    int cnt = 0;
+    if (first < a.n_candidates) {
+      uint64_t v = candidate_at(a, first);
+      const int todo = (int)min((int64_t)kEnumPerThread, a.n_candidates - first);
+      for (int k = 0; k < todo; ++k) {
+        const IsRepResult r = is_rep<DEPTH>(g, v, a.lane_width, true);
+        if (r.ok && (a.reference_rule ? r.sum > 0 : r.trivial && r.exact_count > 0)) {
+          bits |= 1u << k;
+          ++cnt;
+          stab[k] = (uint16_t)(r.trivial ? r.exact_count : 0);
+        }
+        if (k + 1 < todo) v = candidate_next(a, v);
+      }
+    }
+    const int64_t excl = block_exclusive_scan((int64_t)cnt, warp_sums, &total);
+    if (threadIdx.x == 0) {
+      base_slot = total > 0 ? atomicAdd(a.counter, (unsigned long long)total) : 0ull;
+      a.tile_count[tile] = (int32_t)total;
+      a.tile_start[tile] = (int64_t)base_slot;
+    }
+    __syncthreads();
+    if (cnt > 0) {
+      int64_t pos = (int64_t)base_slot + excl;
+      uint64_t v = candidate_at(a, first);
+      for (int k = 0; bits != 0; ++k) {
+        if (bits & 1u) {
+          if (pos < a.capacity) {
+            a.append[pos] = v;
+            if (a.append_stab != nullptr) a.append_stab[pos] = stab[k];
+          }
+          ++pos;
+        }
+        bits >>= 1;
+        if (bits) v = candidate_next(a, v);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int D>
+struct RunEnumerateCandidates {
+  static void run(const DeviceGroup& g, const EnumArgs& a, cudaStream_t s) {
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(a.n_tiles, (int64_t)num_sms() * 8));
+    k_enumerate_candidates<D><<<(unsigned)blocks, kEnumThreads, 0, s>>>(g, a);
+  }
+};
+
+// Images below which a thread per candidate is faster than pruned blocks (flipped images cost the
+// networks less than others).  Kernel times in ms, candidates / blocks: 28 spins, weight 14, 4, 7 and 14
+// elements 1.05 / 3.6, 1.3 / 2.5, 1.8 / 1.7; with inversion 0.83 / 2.0, 1.1 / 1.35, 1.6 / 0.88; 30 spins, 10
+// and 15 elements 5.7 / 6.8, 6.7 / 5.4; 60 spins, weight 4, 15 and 30 elements 0.14 / 0.21, 0.22 / 0.20;
+// 1e5 candidates of 20 spins, 2 and 5 elements with inversion 0.045 / 0.087, 0.065 / 0.063; below 2^15
+// candidates level.
+static bool enumerate_by_candidates(const DeviceGroup& g, int n_bits, int64_t n_candidates) {
+  const double images = g.n_elems * (g.spin_inversion != 0 ? 1.6 : 1.0);
+  if (n_candidates < (int64_t)1 << 15) return false;
+  if (n_candidates < (int64_t)1 << 17) return images < 4.0;
+  return images < std::max(14.0, 0.45 * n_bits);
+}
+
 // Copies every tile's run to its place in the output: a warp per tile.
 __global__ void k_gather_runs(int64_t n_tiles, const int32_t* __restrict__ tile_count,
                               const int64_t* __restrict__ tile_start,
@@ -1282,12 +1358,13 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
   DeviceGroup g = strip(*g0);
   EnumArgs a{};
   projected_candidates(req, n_bits, &a);
+  const bool by_candidates = enumerate_by_candidates(g, n_bits, a.n_candidates);
   // tiles small enough that every SM gets several, work items of many tiles only for long ranges
   const int sms = num_sms();
   PruneArgs q{};
   q.tile = kPruneTile;
   while (q.tile > 256 && a.n_candidates < (int64_t)q.tile * sms * 8) q.tile /= 2;
-  a.n_tiles = (a.n_candidates + q.tile - 1) / q.tile;
+  if (!by_candidates) a.n_tiles = (a.n_candidates + q.tile - 1) / q.tile;
   q.super = a.n_tiles >= (int64_t)sms * 8 * kPruneSuper ? kPruneSuper : 1;
   q.n_items = (a.n_tiles + q.super - 1) / q.super;
   const size_t table_bytes = (size_t)n_bits * g.n_elems * 8;
@@ -1345,9 +1422,10 @@ int enumerate_states(const DeviceGroup* g0, const EnumerateRequest& req, uint64_
     cudaMemsetAsync(tile_count, 0, (size_t)a.n_tiles * 4, s);  // pruned tiles write nothing
     {
       StageScope stage("basis.enumerate", s);
-      kernel<<<(unsigned)std::min<int64_t>(q.n_items, sms), kPruneThreads, smem, s>>>(g, a, q);
+      if (by_candidates) dispatch_depth<RunEnumerateCandidates>(g.depth, group_is_standard(*g0), g, a, s);
+      else kernel<<<(unsigned)std::min<int64_t>(q.n_items, sms), kPruneThreads, smem, s>>>(g, a, q);
     }
-    if (!cuda_ok(cudaGetLastError(), "k_enumerate_pruned") ||
+    if (!cuda_ok(cudaGetLastError(), by_candidates ? "k_enumerate_candidates" : "k_enumerate_pruned") ||
         !cuda_ok(cudaMemcpyAsync(&total, counter, 8, cudaMemcpyDeviceToHost, s), "read count") ||
         !cuda_ok(cudaStreamSynchronize(s), "enumerate")) {
       cleanup();
