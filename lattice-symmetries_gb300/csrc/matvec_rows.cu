@@ -8,16 +8,27 @@
 
 namespace lsg {
 
-// Planes of the bit-plane scan: enough for about 2^-4 ties per target, log2 |G| + 4 bits at half
-// filling, more where the particle number leaves less than a bit per site.
-static int rows_planes(const MatvecProblem& p) {
+// Planes of the bit-plane scan (of `words` words): enough for about 2^-4 ties per target, log2 |G| + 4
+// bits at half filling.  Away from half filling a bit says less: on average its entropy, but the smallest
+// images of a dilute orbit begin with zeros, which say -log2(1 - f) each; the mean of the two serves
+// best where the patterns' table leaves room for it (half the shared memory; with 16 words on the 6x6
+// torus under C6v it does not: 7 up 711 / 1492).  us for one real column, entropy alone / mean:
+// 6x6 torus, 288 images, 7 of 36 spins up 194 / 148, 8 up 436 / 343; 7x7 translations, 6 of 49 up
+// 726 / 529; 48-site chain, 5 up 511 / 383.
+static int rows_planes(const MatvecProblem& p, int words) {
   const int n = p.group.n_bits, inv = p.group.spin_inversion != 0 ? 1 : 0;
   double f = 0.5;
   if (p.constraint.kind == 1) f = (double)p.constraint.w0 / n;
   if (p.constraint.kind == 2) f = (double)(p.constraint.w0 + p.constraint.w1) / n;
   const double entropy = f <= 0.0 || f >= 1.0 ? 0.0 : -(f * std::log2(f) + (1.0 - f) * std::log2(1.0 - f));
-  const double want = std::log2((double)std::max(p.group.n_elems, 1)) / std::max(entropy, 0.2) + 4.0;
-  return std::max(1, std::min({(int)std::ceil(want), n - inv, 32}));
+  auto planes = [&](double bits) {
+    const double want = std::log2((double)std::max(p.group.n_elems, 1)) / std::max(bits, 0.2) + 4.0;
+    return std::max(1, std::min({(int)std::ceil(want), n - inv, 32}));
+  };
+  const int least = planes(entropy);
+  if (f <= 0.0 || f >= 0.5) return least;
+  const int room = (int)(kMaxDynamicSmem / 2 / ((size_t)std::max(p.off.rows.n_pat, 1) * words * 4));
+  return std::max(least, std::min(planes(0.5 * (entropy - std::log2(1.0 - f))), room));
 }
 
 // Dynamic shared memory of a row-group kernel (the coupling products keep 2.2 KB more, statically).
@@ -56,7 +67,7 @@ static bool rows_layout(const MatvecProblem& p, int mode, bool complex_elements,
   if (mode == kModeN32) {
     L.words = (L.G + 7) / 8 * 8;
   } else {
-    L.planes = rows_planes(p);
+    L.planes = rows_planes(p, mode);
     L.nlow = n - inv - L.planes;
     L.nlow_pad = (L.nlow + 3) / 4 * 4;
     const int pw = L.nlow_pad / 4 + 1;  // and the top bit's source
@@ -125,7 +136,7 @@ static bool rows_mode_allowed(const MatvecProblem& p, int mode) {
 static double rows_scan_cost(const MatvecProblem& p, int mode) {
   const int inv = p.group.spin_inversion != 0 ? 1 : 0;
   if (mode == kModeN32) return (p.group.n_elems + 7) / 8 * 8 * (3.5 + inv) + 60.0;
-  const int planes = rows_planes(p);
+  const int planes = rows_planes(p, mode);
   return planes * (4.5 * mode + 5.0) + (p.constraint.kind == 2 ? 8.0 : 2.5) * (30.0 + 4.0 * (p.group.n_bits - planes));
 }
 
