@@ -334,6 +334,12 @@ int ls_gpu_trace_report(char *buffer, size_t size, int reset);
  * fallback projected kernel (*slots_per_lane likewise), 0 without a permutation group
  * (*slots_per_lane = 0).  Needs a built basis. */
 int ls_gpu_matvec_kernel_info(ls_hs_operator const *op, int *form, int *slots_per_lane);
+/* The kernels that a matvec of `op` on k real or complex columns runs: *family = 0 a thread per row with
+ * a search (no permutation group), 1 the fallback projected kernel, 2 the packed kernels (a warp per
+ * row), 3 the lane-per-element kernels, 4 two-table ranks (no permutation group).  *detail = slots per
+ * lane (1, 2); for 3 the scan: 0 whole 32-bit states, else the words of a bit plane.  Needs a built
+ * basis. */
+int ls_gpu_matvec_route(ls_hs_operator const *op, int k, int complex_columns, int *family, int *detail);
 
 /* Releases the device copies of an operator's term tables (made on the first GPU use of `op`,
  * keyed by its address).  Call before freeing or reusing the ls_hs_operator; no-op otherwise. */

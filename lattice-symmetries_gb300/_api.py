@@ -786,10 +786,22 @@ class Operator(_LinearOperator):
         return int(n.value)
 
     def kernel_info(self):
-        """(form, slots_per_lane) of the matvec kernel: form "packed", "fallback" or "plain"."""
+        """(form, slots_per_lane) of the matvec kernels: "packed" where the group's tables fit in shared
+        memory, else "fallback"; "plain" without a permutation group.  ``kernel_route`` says which
+        kernels a product runs."""
         form, slots = c_int(0), c_int(0)
         N.check(self._lib.ls_gpu_matvec_kernel_info(self._payload, byref(form), byref(slots)), "kernel_info")
         return ("plain", "fallback", "packed")[form.value], int(slots.value)
+
+    def kernel_route(self, k: int = 1, complex_columns: bool = True):
+        """(family, detail) of the kernels that ``apply_device`` runs for k columns: "plain" (a thread
+        per row with a search) and "free" (two-table ranks) without a permutation group, "fallback"
+        and "packed" (a warp per row; detail: slots per lane), "rows" (a lane per generated element;
+        detail: 0 for whole 32-bit states, else the words of a bit plane)."""
+        family, detail = c_int(0), c_int(0)
+        N.check(self._lib.ls_gpu_matvec_route(self._payload, int(k), int(bool(complex_columns)), byref(family),
+                                              byref(detail)), "kernel_route")
+        return ("plain", "fallback", "packed", "rows", "free")[family.value], int(detail.value)
 
 
 def load_library():

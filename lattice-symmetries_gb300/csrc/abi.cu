@@ -1799,6 +1799,17 @@ extern "C" int ls_gpu_matvec_kernel_info(ls_hs_operator const* op, int* form, in
   return 0;
 }
 
+extern "C" int ls_gpu_matvec_route(ls_hs_operator const* op, int k, int complex_columns, int* family, int* detail) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if (op == nullptr || family == nullptr || detail == nullptr || k < 1)
+    return fail(LS_GPU_ERR_INVALID, "operator and outputs must not be NULL, k must be positive");
+  MatvecProblem p;
+  const int rc = make_problem(op, false, &p);
+  if (rc != 0) return rc;
+  *family = (int)matvec_family(p, complex_columns != 0 ? Scalar::Complex : Scalar::Real, k, detail);
+  return 0;
+}
+
 extern "C" int ls_gpu_count_nonzeros(ls_hs_operator const* op, int64_t* nnz) {
   int64_t n = 0;
   {

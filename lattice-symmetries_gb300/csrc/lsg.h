@@ -281,6 +281,8 @@ struct MatvecProblem {
 // real: at most 32) from the prescaled gather source p.xs (leading dimension p.ldxs; even for two
 // or more real columns).
 bool rows_fit(const MatvecProblem& p, int n_sectors = 0);
+// The scan mode for k columns.
+int rows_mode(const MatvecProblem& p, Scalar sc, int k);
 int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y, int64_t ldy,
                 int* d_err, const uint64_t* binom, cudaStream_t s);
 
@@ -300,8 +302,12 @@ int launch_check_ranks(int split, int n_bits, const DeviceConstraint& constraint
 
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,
                   double* d_y, int64_t ldy, int* d_err, cudaStream_t s);
-// The kernel launch_matvec picks for p: 2 packed (*gpl slots per lane), 1 fallback, 0 plain.
+// What ls_gpu_matvec_kernel_info reports: 2 where the group's tables fit in shared memory (*gpl slots per
+// lane of the packed kernels), 1 fallback, 0 without a group.
 int matvec_kernel_form(const MatvecProblem& p, int* gpl);
+// The kernels that launch_matvec runs for k columns, and their scan mode (Rows) or slots per lane.
+enum class MatvecFamily { Plain = 0, Fallback = 1, Packed = 2, Rows = 3, Free = 4 };
+MatvecFamily matvec_family(const MatvecProblem& p, Scalar sc, int k, int* detail = nullptr);
 
 // Sector plans (matvec.cu): y_s = H_s x_s (complex, k right-hand sides, leading dimensions
 // ldx/ldy) for many sectors.  When the sectors share the group's site images, the terms and the

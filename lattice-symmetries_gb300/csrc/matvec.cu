@@ -202,10 +202,39 @@ static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const do
   return rc;
 }
 
-// Row-group kernels wherever their tables fit (faster than the packed kernels at every measured size
-// and group: 2.3x at 576 images, 2.3x at 56 with 16 columns, 10.6x at 150 with five; 1.2x at 257
-// rows, where launches count); otherwise splits k right-hand sides into launches of
-// 16, 8, 4 and 1 columns of the packed kernels.
+// Columns per launch of the packed kernels: 16, 8, 4 and 1 (real pairs: 2).
+static std::vector<int> packed_chunks(const MatvecProblem& p, bool cplx, int k) {
+  std::vector<int> chunks;
+  for (int done = 0; done < k;) {
+    const int left = k - done;
+    const int most = std::min(left, g_rhs_tile);
+    int chunk = most >= 16 ? 16 : most >= 8 ? 8 : most >= 4 ? 4 : 1;
+    if (!cplx && left == 2 && g_rhs_tile >= 2) chunk = 2;
+    if (p.group.fermionic && !cplx) chunk = 1;  // fermionic real path: one column per launch
+    chunks.push_back(chunk);
+    done += chunk;
+  }
+  return chunks;
+}
+
+// Row-group kernels wherever their tables fit (2.3x the packed ones at 576 images, 2.3x at 56 with 16
+// columns, 10.6x at 150 with five; 1.2x at 257 rows, where launches count).
+MatvecFamily matvec_family(const MatvecProblem& p, Scalar sc, int k, int* detail) {
+  const bool cplx = sc == Scalar::Complex;
+  auto is = [&](MatvecFamily f, int d) {
+    if (detail != nullptr) *detail = d;
+    return f;
+  };
+  if (p.projection != 2) return is(free_fits(p) ? MatvecFamily::Free : MatvecFamily::Plain, 0);
+  const bool packed = packed_fits(p);
+  // counting elements needs the norms of the columns, the FP32-pair arithmetic its own kernels
+  const bool pairs = cplx && k >= 8 && g_rhs_tile >= 8 && packed && use_pairs(p.group.gpl);
+  if (p.nnz_counter == nullptr && p.index.norms != nullptr && !pairs && rows_fit(p)) {
+    return is(MatvecFamily::Rows, detail != nullptr ? rows_mode(p, sc, std::min(k, g_rhs_tile)) : 0);
+  }
+  return packed ? is(MatvecFamily::Packed, p.group.gpl) : is(MatvecFamily::Fallback, pick_gpl_for(p.group.n_elems));
+}
+
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,
                   double* d_y, int64_t ldy, int* d_err, cudaStream_t s) {
   if (p.n_rows == 0 || k == 0) return 0;
@@ -215,25 +244,13 @@ int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, i
   const size_t scalar_words = cplx ? 2 : 1;  // doubles per element
   if (p.projection == 2) {
     const bool inv = p.group.spin_inversion != 0;
-    // counting elements needs the norms of the columns, the FP32-pair arithmetic its own kernels
-    const bool pairs = cplx && k >= 8 && g_rhs_tile >= 8 && packed_fits(p) && use_pairs(p.group.gpl);
-    if (p.nnz_counter == nullptr && p.index.norms != nullptr && !pairs && rows_fit(p)) {
+    if (matvec_family(p, sc, k) == MatvecFamily::Rows) {
       const int rc = launch_matvec_rows(p, sc, k, d_x, ldx, d_y, ldy, d_err, binom, s);
       if (rc != 1) return rc;
     }
     if (packed_fits(p)) {
-      // Right-hand-side chunks of 16, 8, 4 and 1 columns; complex chunks of 8 or 16 run the
-      // FP32-pair kernels (g_block_pairs).
-      std::vector<int> chunks;
-      for (int done = 0; done < k;) {
-        const int left = k - done;
-        const int most = std::min(left, g_rhs_tile);
-        int chunk = most >= 16 ? 16 : most >= 8 ? 8 : most >= 4 ? 4 : 1;
-        if (!cplx && left == 2 && g_rhs_tile >= 2) chunk = 2;
-        if (p.group.fermionic && !cplx) chunk = 1;  // fermionic real path: one column per launch
-        chunks.push_back(chunk);
-        done += chunk;
-      }
+      // complex chunks of 8 or 16 columns run the FP32-pair kernels (g_block_pairs)
+      const std::vector<int> chunks = packed_chunks(p, cplx, k);
       // Gather sources x_j * n_j for all k columns (one streaming pass each), so that the kernels
       // read no norm per generated element: FP64 for the FP64 kernels, float pairs for the pair
       // kernels.  Not when counting elements (the count needs the norms).

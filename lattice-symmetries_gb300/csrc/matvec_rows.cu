@@ -150,14 +150,21 @@ bool rows_fit(const MatvecProblem& p, int n_sectors) {
   return false;
 }
 
+// The modes that p can run, N32 and the group's bit planes, the cheaper scan first; their number.
+static int rows_modes(const MatvecProblem& p, int (&modes)[2]) {
+  int n = 0;
+  for (const int m : kRowModes)
+    if (rows_mode_allowed(p, m)) modes[n++] = m;
+  if (n == 2 && rows_scan_cost(p, modes[1]) < rows_scan_cost(p, modes[0])) std::swap(modes[0], modes[1]);
+  return n;
+}
+
 // Shape for p (rows_fit): the cheapest number of rows per warp among those that leave enough warps
 // their area.
 static bool rows_shape(const MatvecProblem& p, bool complex_elements, bool keep, int64_t n_rows, int n_sectors,
                        int max_warps, int sms, int* mode, RowsLayout* L) {
-  int modes[2], n_modes = 0;  // N32 and the group's bit planes, the cheaper scan first
-  for (const int m : kRowModes)
-    if (rows_mode_allowed(p, m)) modes[n_modes++] = m;
-  if (n_modes == 2 && rows_scan_cost(p, modes[1]) < rows_scan_cost(p, modes[0])) std::swap(modes[0], modes[1]);
+  int modes[2];
+  const int n_modes = rows_modes(p, modes);
   for (int k = 0; k < n_modes; ++k) {
     const int m = modes[k];
     RowsLayout t[4];
@@ -231,15 +238,25 @@ bool rows_plan(const MatvecProblem& p, int col, int k, int64_t n_rows, int n_sec
   return true;
 }
 
+static bool launch_plan(const MatvecProblem& p, Scalar sc, int k, RowsLaunch* q, int* col) {
+  const bool cplx = sc == Scalar::Complex;
+  *col = cplx ? (p.real_elements ? kColPair : kColComplex) : (k == 1 ? kColReal : kColPair);
+  q->s.real_cols = (!cplx && *col == kColPair) ? k : 0;
+  return rows_plan(p, *col, k, p.n_rows, 0, q);
+}
+
+int rows_mode(const MatvecProblem& p, Scalar sc, int k) {
+  RowsLaunch q{};
+  int col = 0;
+  return launch_plan(p, sc, k, &q, &col) ? q.mode : -1;
+}
+
 int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y, int64_t ldy,
                 int* d_err, const uint64_t* binom, cudaStream_t st) {
-  const bool cplx = sc == Scalar::Complex;
-  const int col = cplx ? (p.real_elements ? kColPair : kColComplex) : (k == 1 ? kColReal : kColPair);
   RowsLaunch q{};
   RowsSums& s = q.s;
-  s.real_cols = (!cplx && col == kColPair) ? k : 0;
-  if (!rows_plan(p, col, k, p.n_rows, 0, &q))
-    return fail(LS_GPU_ERR_INVALID, "row-group tables do not fit in shared memory");
+  int col = 0;
+  if (!launch_plan(p, sc, k, &q, &col)) return fail(LS_GPU_ERR_INVALID, "row-group tables do not fit in shared memory");
   s.x = d_x;
   s.xs = p.xs != nullptr ? p.xs : d_x;
   s.norms = p.xs != nullptr ? nullptr : p.index.norms;
