@@ -281,7 +281,9 @@ struct MatvecProblem {
 // real: at most 32) from the prescaled gather source p.xs (leading dimension p.ldxs; even for two
 // or more real columns).
 bool rows_fit(const MatvecProblem& p, int n_sectors = 0);
-// The scan mode for k columns.
+// Whether the problem has so few rows that a warp per row is faster (k columns in one launch of the packed
+// kernels with that many slots, 0: only the kernel without shared tables); the scan mode for k columns.
+bool rows_few(const MatvecProblem& p, int k, int slots);
 int rows_mode(const MatvecProblem& p, Scalar sc, int k);
 int launch_rows(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx, double* d_y, int64_t ldy,
                 int* d_err, const uint64_t* binom, cudaStream_t s);

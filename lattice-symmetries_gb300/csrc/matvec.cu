@@ -218,7 +218,8 @@ static std::vector<int> packed_chunks(const MatvecProblem& p, bool cplx, int k) 
 }
 
 // Row-group kernels wherever their tables fit (2.3x the packed ones at 576 images, 2.3x at 56 with 16
-// columns, 10.6x at 150 with five; 1.2x at 257 rows, where launches count).
+// columns, 10.6x at 150 with five; 1.2x at 257 rows, where launches count), but for few rows and columns
+// that the packed kernels take in one launch (rows_few).
 MatvecFamily matvec_family(const MatvecProblem& p, Scalar sc, int k, int* detail) {
   const bool cplx = sc == Scalar::Complex;
   auto is = [&](MatvecFamily f, int d) {
@@ -230,7 +231,11 @@ MatvecFamily matvec_family(const MatvecProblem& p, Scalar sc, int k, int* detail
   // counting elements needs the norms of the columns, the FP32-pair arithmetic its own kernels
   const bool pairs = cplx && k >= 8 && g_rhs_tile >= 8 && packed && use_pairs(p.group.gpl);
   if (p.nnz_counter == nullptr && p.index.norms != nullptr && !pairs && rows_fit(p)) {
-    return is(MatvecFamily::Rows, detail != nullptr ? rows_mode(p, sc, std::min(k, g_rhs_tile)) : 0);
+    const bool one_launch = packed ? packed_chunks(p, cplx, k).size() == 1
+                                   : k == 1 && !p.group.fermionic && pick_gpl_for(p.group.n_elems) > 0 &&
+                                         make_layout(p, true).total <= kMaxDynamicSmem;
+    if (!(one_launch && rows_few(p, k, packed ? 32 * p.group.gpl : 0)))
+      return is(MatvecFamily::Rows, detail != nullptr ? rows_mode(p, sc, std::min(k, g_rhs_tile)) : 0);
   }
   return packed ? is(MatvecFamily::Packed, p.group.gpl) : is(MatvecFamily::Fallback, pick_gpl_for(p.group.n_elems));
 }

@@ -159,6 +159,34 @@ static int rows_modes(const MatvecProblem& p, int (&modes)[2]) {
   return n;
 }
 
+// Few rows: at most about one per warp of the packed kernels, which then take no longer than a row's
+// latency, while here the tables of every CTA and the ties of a lane's elements do.  us of one product
+// (k columns in one launch), a warp per row / a lane per element: 6x6 torus, 288 images, 3 up (40 rows),
+// one real column 28 / 91, 6 up (7278 rows) 58 / 76; C6v, 432 images, 5 up (964 rows), 16 complex
+// columns 68 / 210; 48-site chain, 4 up (4060 rows), one column 26 / 42; 4D hypercube, 384 images,
+// 58 rows 42 / 97; 4x4 Hubbard, 128 images, 2 + 2 (2506 rows), 16 columns 30 / 40.
+// Not so
+//  - up to 32 bits for one column (24 sites, 48 images: 25 / 20) or a dozen rows (4x4 torus, 10 rows 20.5 / 18);
+//  - for small groups (48 sites, 3 images, 5776 rows: 36 / 24) or one column of many terms (36 sites, all
+//    pairs, 4 up: 94 / 65);
+//  - where slots of the packed kernels are empty: they repeat element 0 and tie with it (216 images
+//    on 6x6, 9212 rows, 165 / 98; 5x5, 150 images, 98 rows 55 / 26).
+// slots: of the packed kernels, or 0 where only the kernel without shared tables could run (one column).
+bool rows_few(const MatvecProblem& p, int k, int slots) {
+  int modes[2];
+  if (rows_modes(p, modes) == 0) return false;
+  const int64_t sms = num_sms(), n = p.n_rows;
+  const int G = p.group.n_elems;
+  const bool wide = p.group.n_bits > 32, full = G == slots;
+  if (k == 1 && p.off.rows.n_slots > 256) return false;
+  if (slots == 0) return modes[0] != kModeN32 && k == 1 && n <= 16 * sms;
+  if (modes[0] == 16) return n <= (full ? 48 : 32) * sms;
+  if (!wide) return k > 1 && G > 64 && full && n * G > 12288 && n <= 32 * sms;
+  if (G <= 32) return false;
+  if (G <= 128) return n <= 32 * sms;
+  return n <= (full ? 48 : 4) * sms;
+}
+
 // Shape for p (rows_fit): the cheapest number of rows per warp among those that leave enough warps
 // their area.
 static bool rows_shape(const MatvecProblem& p, bool complex_elements, bool keep, int64_t n_rows, int n_sectors,
