@@ -153,14 +153,35 @@ void rows_launch_config(int* max_threads, int* waves) {
   if (g_blocks_per_sm_override > 0) *waves = g_blocks_per_sm_override;
 }
 
+// Stream-ordered memory that a kernel can do without, or null.  In a captured graph an allocation only
+// fails when the graph is launched, where nothing can take the other route any more, so while
+// capturing the memory has to be there: free on the device, or unused in the graphs' own pool.
+static void* optional_async(size_t bytes, cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) == cudaSuccess && status == cudaStreamCaptureStatusActive) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    size_t free_bytes = 0, total = 0;
+    uint64_t reserved = 0, used = 0;
+    int dev = 0;
+    const bool ok = cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess &&
+                    cudaDeviceGetGraphMemAttribute(dev, cudaGraphMemAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+                    cudaDeviceGetGraphMemAttribute(dev, cudaGraphMemAttrUsedMemCurrent, &used) == cudaSuccess;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) cudaGetLastError();
+    if (ok && bytes > free_bytes + (reserved > used ? reserved - used : 0)) return nullptr;
+  }
+  void* p = nullptr;
+  if (cudaMallocAsync(&p, bytes, s) == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
+}
+
 double* prescaled_copy(const MatvecProblem& p, int words, int k, const double* d_x, int64_t ldx, int64_t ldxs,
                        cudaStream_t s) {
   const int64_t elems = p.n_rows * ldxs * words;
-  double* d_xs = nullptr;
-  if (cudaMallocAsync((void**)&d_xs, (size_t)elems * sizeof(double), s) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
+  double* d_xs = (double*)optional_async((size_t)elems * sizeof(double), s);
+  if (d_xs == nullptr) return nullptr;
   StageScope stage("matvec.prescale", s);
   const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((elems + 255) / 256, (int64_t)num_sms() * 16));
   k_prescale<<<(unsigned)blocks, 256, 0, s>>>(d_x, ldx, p.index.norms, p.n_rows, k, words, d_xs, ldxs);
@@ -202,19 +223,12 @@ static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const do
   return rc;
 }
 
-// Columns per launch of the packed kernels: 16, 8, 4 and 1 (real pairs: 2).
-static std::vector<int> packed_chunks(const MatvecProblem& p, bool cplx, int k) {
-  std::vector<int> chunks;
-  for (int done = 0; done < k;) {
-    const int left = k - done;
-    const int most = std::min(left, g_rhs_tile);
-    int chunk = most >= 16 ? 16 : most >= 8 ? 8 : most >= 4 ? 4 : 1;
-    if (!cplx && left == 2 && g_rhs_tile >= 2) chunk = 2;
-    if (p.group.fermionic && !cplx) chunk = 1;  // fermionic real path: one column per launch
-    chunks.push_back(chunk);
-    done += chunk;
-  }
-  return chunks;
+// Columns of the packed kernels' next launch with `left` to go: 16, 8, 4 or 1 (real pairs: 2).
+static int packed_chunk(const MatvecProblem& p, bool cplx, int left) {
+  if (p.group.fermionic && !cplx) return 1;  // fermionic real path: one column per launch
+  if (!cplx && left == 2 && g_rhs_tile >= 2) return 2;
+  const int most = std::min(left, g_rhs_tile);
+  return most >= 16 ? 16 : most >= 8 ? 8 : most >= 4 ? 4 : 1;
 }
 
 // Row-group kernels wherever their tables fit (2.3x the packed ones at 576 images, 2.3x at 56 with 16
@@ -230,13 +244,12 @@ MatvecFamily matvec_family(const MatvecProblem& p, Scalar sc, int k, int* detail
   const bool packed = packed_fits(p);
   // counting elements needs the norms of the columns, the FP32-pair arithmetic its own kernels
   const bool pairs = cplx && k >= 8 && g_rhs_tile >= 8 && packed && use_pairs(p.group.gpl);
-  if (p.nnz_counter == nullptr && p.index.norms != nullptr && !pairs && rows_fit(p)) {
-    const bool one_launch = packed ? packed_chunks(p, cplx, k).size() == 1
-                                   : k == 1 && !p.group.fermionic && pick_gpl_for(p.group.n_elems) > 0 &&
-                                         make_layout(p, true).total <= kMaxDynamicSmem;
-    if (!(one_launch && rows_few(p, k, packed ? 32 * p.group.gpl : 0)))
-      return is(MatvecFamily::Rows, detail != nullptr ? rows_mode(p, sc, std::min(k, g_rhs_tile)) : 0);
-  }
+  const bool one_launch = packed ? packed_chunk(p, cplx, k) == k
+                                 : k == 1 && !p.group.fermionic && pick_gpl_for(p.group.n_elems) > 0 &&
+                                       make_layout(p, true).total <= kMaxDynamicSmem;
+  if (p.nnz_counter == nullptr && p.index.norms != nullptr && !pairs &&
+      !(one_launch && rows_few(p, k, packed ? 32 * p.group.gpl : 0)) && rows_fit(p))
+    return is(MatvecFamily::Rows, detail != nullptr ? rows_mode(p, sc, std::min(k, g_rhs_tile)) : 0);
   return packed ? is(MatvecFamily::Packed, p.group.gpl) : is(MatvecFamily::Fallback, pick_gpl_for(p.group.n_elems));
 }
 
@@ -255,7 +268,8 @@ int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, i
     }
     if (packed_fits(p)) {
       // complex chunks of 8 or 16 columns run the FP32-pair kernels (g_block_pairs)
-      const std::vector<int> chunks = packed_chunks(p, cplx, k);
+      std::vector<int> chunks;
+      for (int done = 0; done < k; done += chunks.back()) chunks.push_back(packed_chunk(p, cplx, k - done));
       // Gather sources x_j * n_j for all k columns (one streaming pass each), so that the kernels
       // read no norm per generated element: FP64 for the FP64 kernels, float pairs for the pair
       // kernels.  Not when counting elements (the count needs the norms).
@@ -486,11 +500,8 @@ __global__ void k_prescale_sectors(const SectorDesc* __restrict__ desc, int n_se
 // gather source (nothing has been launched).
 static int sector_plan_run_rows(const SectorPlan* plan, int* d_err, const uint64_t* binom, cudaStream_t s) {
   const int n = plan->n_sectors;
-  double2* d_xs = nullptr;
-  if (cudaMallocAsync((void**)&d_xs, (size_t)plan->total_rows * plan->k * sizeof(double2), s) != cudaSuccess) {
-    cudaGetLastError();
-    return 1;
-  }
+  double2* d_xs = (double2*)optional_async((size_t)plan->total_rows * plan->k * sizeof(double2), s);
+  if (d_xs == nullptr) return 1;
   int rc = 0;
   {
     const int64_t per_sector = (plan->total_rows * plan->k + n - 1) / n;
