@@ -496,6 +496,17 @@ __global__ void k_prescale_sectors(const SectorDesc* __restrict__ desc, int n_se
   }
 }
 
+// Few rows in all sectors together (16 per SM; the packed kernel has 10 warps per CTA) and as many launches
+// either way: the packed kernel needs no scaled copy and fills smaller tables.  us per run, packed /
+// row groups: 12 sites, 24 sectors, 924 rows, 1 and 16 columns 14 / 21, 15 / 22; two sectors of 16 sites
+// (~800 rows), 4 columns 14 / 20; 14 sites, 3432 rows, 1 and 16 columns 28 / 26, 31 / 27; 13 columns
+// (three launches against one) 37 / 22 already at 10 sites.
+static bool sectors_few_rows(const SectorPlan* plan) {
+  const size_t launches = ((size_t)plan->k + 15) / 16;
+  return plan->total_rows <= (int64_t)num_sms() * 16 && plan->chunks.size() <= launches &&
+         packed_fits(plan->shared, plan->n_sectors);
+}
+
 // The batched launch by the row-group kernels.  Returns 1 when there is no memory for the prescaled
 // gather source (nothing has been launched).
 static int sector_plan_run_rows(const SectorPlan* plan, int* d_err, const uint64_t* binom, cudaStream_t s) {
@@ -540,7 +551,8 @@ int sector_plan_run(const SectorPlan* plan, int* d_err, cudaStream_t s) {
   // chunks of 8 or 16 columns run the FP32-pair kernels from a prescaled pair copy of all
   // sectors' columns (one streaming pass); the others gather x and the norms in FP64
   float4* d_xp = nullptr;
-  if (plan->rows && !(use_pairs(plan->shared.group.gpl) && packed_fits(plan->shared, plan->n_sectors))) {
+  if (plan->rows && !(use_pairs(plan->shared.group.gpl) && packed_fits(plan->shared, plan->n_sectors)) &&
+      !sectors_few_rows(plan)) {
     const int rc = sector_plan_run_rows(plan, d_err, binom, s);
     if (rc != 1) return rc;
     if (!packed_fits(plan->shared, plan->n_sectors)) return fail(LS_GPU_ERR_CUDA, "no memory for the scaled vectors");
