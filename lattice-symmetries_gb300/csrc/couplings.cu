@@ -352,13 +352,17 @@ int launch_coupling_products(const MatvecProblem& p, int nc, const double* d_g, 
   if (p.off.coupling == nullptr) return fail(LS_GPU_ERR_INVALID, "operator terms carry no coupling ids");
   const uint64_t* binom = device_binomials();
   if (binom == nullptr) return LS_GPU_ERR_CUDA;
-  if (p.n_rows > 0 && p.index.norms != nullptr && rows_fit(p, 0)) {
-    const int rc = launch_coupling_rows(p, nc, d_g, d_x, d_out, d_err, binom, s);
-    if (rc != 1) return rc;
-  }
   const PackedLayout L = make_packed_layout(p, 0, 256);
   const size_t off_cpl = (L.total + 15) & ~(size_t)15;
   const size_t smem = off_cpl + (size_t)(p.off.n + p.diag.n) * 4;
+  // Few rows (one per warp of a CTA per SM) stay with a warp per row, which needs no scaled copy and fills smaller
+  // tables: us per call from Python, warp per row / row groups, ladders of 12 and 16 sites (84 and 820
+  // rows) 115 / 157, 125 / 156, 20 sites (9278 rows) 299 / 171; 6x6 translations, 1649 rows, 153 / 155.
+  const bool few = p.n_rows <= (int64_t)num_sms() * 8 && smem <= kMaxDynamicSmem;
+  if (p.n_rows > 0 && p.index.norms != nullptr && !few && rows_fit(p, 0)) {
+    const int rc = launch_coupling_rows(p, nc, d_g, d_x, d_out, d_err, binom, s);
+    if (rc != 1) return rc;
+  }
   if (smem > kMaxDynamicSmem) return fail(LS_GPU_ERR_INVALID, "term tables too large for shared memory");
   const int blocks = std::max(1, std::min(num_sms() * 8, (int)((p.n_rows + 7) / 8)));
   double2* partial = (double2*)scratch((size_t)blocks * nc * sizeof(double2), 6);
