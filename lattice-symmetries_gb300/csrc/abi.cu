@@ -201,7 +201,12 @@ extern "C" int ls_hs_internal_dec_refcount(ls_gb300_refcount* rc) {
   return __atomic_fetch_sub(rc, 1, __ATOMIC_SEQ_CST);
 }
 
-static void free_pinned(void* p) {
+static void drop_pending_states(const void* elts);
+
+// Representatives from the enumeration: their device copies go with them when no index took them.
+static void free_states(void* p) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  drop_pending_states(p);
   if (p) cudaFreeHost(p);
 }
 static void free_malloced(void* p) { free(p); }
@@ -482,6 +487,15 @@ struct PendingStates {
   const OrbitData* norms_for;
 };
 std::unordered_map<const void*, PendingStates> g_pending_device_reps;
+}
+
+static void drop_pending_states(const void* elts) {
+  auto it = g_pending_device_reps.find(elts);
+  if (it == g_pending_device_reps.end()) return;
+  cudaFree(it->second.reps);
+  cudaFree(it->second.norms);
+  cudaFree(it->second.stab);
+  g_pending_device_reps.erase(it);
 }
 
 struct ls_hs_state_index_binary_search_data : IndexData {};
@@ -833,10 +847,11 @@ extern "C" void ls_chpl_enumerate_representatives(ls_hs_basis* p, uint64_t lower
     report("ls_chpl_enumerate_representatives");
     return;
   }
+  drop_pending_states(h);
   g_pending_device_reps[h] = PendingStates{d, norms, stab, basis_orbit(p)};
   dest->elts = h;
   dest->num_elts = (uint64_t)n;
-  dest->freer = (void*)&free_pinned;
+  dest->freer = (void*)&free_states;
 }
 
 // reference.c:173-194
