@@ -6,11 +6,9 @@
 // element's contribution conj(g_i) / n_i * v_t (-1)^popcount(beta & s_t) conj(chi) n_j x_j goes to
 // the accumulator of its term's coupling instead of to y_i.  Per-lane sums are reduced per block,
 // the block partials by one more small kernel in a fixed order (deterministic).
-#include <type_traits>
-
 //
 // k_coupling_rows does the same on the row-group orbit scan (one lane per element, rowgroup.cuh),
-// wherever its tables fit: a lane keeps one sum per coupling over its row's elements, with
+// where its tables fit and the rows are not few: a lane keeps one sum per coupling over its row's elements, with
 // x_j n_j from a prescaled copy and coefficients from the (class, element) table, and multiplies by
 // conj(g_i) / n_i once per row.  Alike terms of different couplings (Heisenberg and DM on a bond)
 // are one element: the lane then sums per class, and the class sums count for each coupling with the
@@ -18,6 +16,8 @@
 // warp per row (k_coupling_products), 2.3 ms with one lane per element, 1.8 ms with alike terms
 // merged (FP64 pipe 75 %: every element was added to every sum under a predicate), 1.4 ms with the
 // element's sum picked by selects and multiply-adds at the rows' ends.
+#include <type_traits>
+
 #include "matvec_launch.cuh"
 #include "rowsums.cuh"
 

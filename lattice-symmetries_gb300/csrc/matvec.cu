@@ -208,8 +208,11 @@ static int launch_matvec_rows(const MatvecProblem& p, Scalar sc, int k, const do
   MatvecProblem q = p;
   q.ldxs = words == 1 && k > 1 ? k + k % 2 : k;  // real columns are read in pairs
   // small problems read the norms with x instead of a scaled copy: an allocation and a launch less
+  // -- unless y overlaps x: the copy lets a product overwrite its argument
   const int64_t most = k > 1 ? kUnscaledElements : words == 1 ? kUnscaledRows : kUnscaledComplexRows;
-  const bool unscaled = p.n_rows * k <= most;
+  const double* x_end = d_x + ((p.n_rows - 1) * ldx + k) * words;
+  const double* y_end = d_y + ((p.n_rows - 1) * ldy + k) * words;
+  const bool unscaled = p.n_rows * k <= most && (x_end <= d_y || y_end <= d_x);
   double* d_xs = unscaled ? nullptr : prescaled_copy(p, words, k, d_x, ldx, q.ldxs, s);
   if (d_xs == nullptr && !unscaled) return 1;
   int rc = 0;
