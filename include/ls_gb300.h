@@ -328,11 +328,10 @@ int ls_gpu_count_nonzeros(ls_hs_operator const *op, int64_t *nnz);
  * (NUL-terminated, truncated to size); it returns the full length; reset != 0 clears the totals. */
 int ls_gpu_set_tracing(int on);
 int ls_gpu_trace_report(char *buffer, size_t size, int reset);
-/* The kernel family a matvec of `op` runs: *form = 2 when the group's tables fit in shared memory
- * (one lane per generated element where its tables fit too, else the packed kernel with one warp per
- * row; *slots_per_lane = group elements per lane of the packed kernel, 32 lanes per warp), 1 for the
- * fallback projected kernel (*slots_per_lane likewise), 0 without a permutation group
- * (*slots_per_lane = 0).  Needs a built basis. */
+/* The kernels with a warp per row that `op` can run: *form = 2 for the packed projected kernels (their
+ * tables fit in shared memory; *slots_per_lane = group elements per lane, 32 lanes per warp), 1 for
+ * the fallback projected kernel (*slots_per_lane likewise), 0 without a permutation group
+ * (*slots_per_lane = 0).  ls_gpu_matvec_route says which kernels a product runs.  Needs a built basis. */
 int ls_gpu_matvec_kernel_info(ls_hs_operator const *op, int *form, int *slots_per_lane);
 /* The kernels that a matvec of `op` on k real or complex columns runs: *family = 0 a thread per row with
  * a search (no permutation group), 1 the fallback projected kernel, 2 the packed kernels (a warp per

@@ -786,9 +786,9 @@ class Operator(_LinearOperator):
         return int(n.value)
 
     def kernel_info(self):
-        """(form, slots_per_lane) of the matvec kernels: "packed" where the group's tables fit in shared
-        memory, else "fallback"; "plain" without a permutation group.  ``kernel_route`` says which
-        kernels a product runs."""
+        """(form, slots_per_lane) of the kernels with a warp per row: "packed" where their tables fit in
+        shared memory, else "fallback"; "plain" without a permutation group.  ``kernel_route`` says
+        which kernels a product runs."""
         form, slots = c_int(0), c_int(0)
         N.check(self._lib.ls_gpu_matvec_kernel_info(self._payload, byref(form), byref(slots)), "kernel_info")
         return ("plain", "fallback", "packed")[form.value], int(slots.value)

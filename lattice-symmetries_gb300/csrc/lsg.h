@@ -304,8 +304,8 @@ int launch_check_ranks(int split, int n_bits, const DeviceConstraint& constraint
 
 int launch_matvec(const MatvecProblem& p, Scalar sc, int k, const double* d_x, int64_t ldx,
                   double* d_y, int64_t ldy, int* d_err, cudaStream_t s);
-// What ls_gpu_matvec_kernel_info reports: 2 where the group's tables fit in shared memory (*gpl slots per
-// lane of the packed kernels), 1 fallback, 0 without a group.
+// What ls_gpu_matvec_kernel_info reports: 2 where the packed kernels' tables fit in shared memory (*gpl slots
+// per lane), 1 fallback, 0 without a group.
 int matvec_kernel_form(const MatvecProblem& p, int* gpl);
 // The kernels that launch_matvec runs for k columns, and their scan mode (Rows) or slots per lane.
 enum class MatvecFamily { Plain = 0, Fallback = 1, Packed = 2, Rows = 3, Free = 4 };

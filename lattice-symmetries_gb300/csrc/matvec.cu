@@ -134,13 +134,13 @@ static bool packed_fits(const MatvecProblem& p, int n_sectors = 0) {
          make_packed_layout(p, n_sectors, 64).total <= kMaxDynamicSmem;
 }
 
-// Which kernel launch_matvec runs for `p`: 2 packed projected (*gpl = slots per lane), 1 the
-// fallback projected kernel (*gpl = its slots per lane), 0 the thread-per-row kernel.
+// Whether the packed kernels can run `p`: 2 (*gpl = slots per lane), else 1 (*gpl = slots of the fallback
+// kernel); 0 without a group.
 int matvec_kernel_form(const MatvecProblem& p, int* gpl) {
   *gpl = 0;
   if (p.projection != 2) return 0;
-  if (packed_fits(p) || rows_fit(p)) {
-    *gpl = p.group.gpl > 0 ? p.group.gpl : pick_gpl_for(p.group.n_elems);
+  if (packed_fits(p)) {
+    *gpl = p.group.gpl;
     return 2;
   }
   *gpl = pick_gpl_for(p.group.n_elems);

@@ -100,3 +100,10 @@ def test_fermions_of_few_rows():
         assert float((y[:, j] - one).norm()) <= RTOL * float(one.norm())
     three = op.apply_device(x[:, :3].contiguous())
     assert float((y[:, :3] - three).norm()) <= RTOL * float(three.norm())
+
+
+def test_kernel_info_is_that_of_the_warp_per_row_kernels(cases):
+    """It keeps its meaning where the lane-per-element kernels run: whether the packed tables fit."""
+    assert cases["chain60_h3"][0].op.kernel_info() == ("fallback", 2)
+    assert cases["chain36_h5"][0].op.kernel_info() == ("packed", 2)
+    assert cases["free"][0].op.kernel_info() == ("plain", 0)
