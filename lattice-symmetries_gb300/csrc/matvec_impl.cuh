@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // ------------------------------------------------------------------------------------------------
-// Packed projected kernel (default for projected bases).
+// Packed projected kernel (few rows, element counts, tables that the row-group kernels cannot hold).
 //
 // Same gather as k_matvec_projected, with a cheaper orbit scan:
 //  * the site-image table is pre-shifted to the top bits and padded to GPL*32 slots, and the low

@@ -50,6 +50,12 @@ CASES = {
     "hypercube": (lambda: Case(ls.SpinBasis(16, 8, 1, ls.Symmetries(LAT.hypercube_symmetries(4))),
                                LAT.heisenberg(LAT.hypercube_bonds(4))),
                   {(1, False): ("packed", 12), (16, True): ("packed", 12), (3, True): ("rows", 16)}),
+    "square4_inversion": (lambda: Case(ls.SpinBasis(16, 8, -1, ls.Symmetries(LAT.square_symmetries(4, 2, 2))),
+                                       LAT.heisenberg(LAT.square_bonds(4))),
+                          {(1, False): ("rows", 5), (1, True): ("rows", 5), (3, True): ("rows", 5), (5, False): ("rows", 5)}),
+    "triangular4_inversion": (lambda: Case(ls.SpinBasis(16, 8, 1, ls.Symmetries(LAT.triangular_symmetries(4, 0, 0, 0, 0))),
+                                           LAT.heisenberg(LAT.triangular_bonds(4))),
+                              {(1, True): ("rows", 9), (3, True): ("rows", 9), (2, True): ("rows", 9)}),
     "free": (lambda: Case(ls.SpinBasis(12, 5), LAT.heisenberg(LAT.chain_bonds(12))), {(1, True): ("free", 0)}),
     "free41": (lambda: Case(ls.SpinBasis(41, 2), LAT.heisenberg(LAT.chain_bonds(41))), {(1, True): ("plain", 0)}),
 }
