@@ -204,8 +204,8 @@ extern "C" int ls_hs_internal_dec_refcount(ls_gb300_refcount* rc) {
 static void drop_pending_states(const void* elts);
 
 // Representatives from the enumeration: their device copies go with them when no index took them.
+// (A finaliser may run inside an error handler that is called with g_mutex held.)
 static void free_states(void* p) {
-  std::lock_guard<std::mutex> lock(g_mutex);
   drop_pending_states(p);
   if (p) cudaFreeHost(p);
 }
@@ -487,15 +487,25 @@ struct PendingStates {
   const OrbitData* norms_for;
 };
 std::unordered_map<const void*, PendingStates> g_pending_device_reps;
+std::mutex g_pending_mutex;  // of the map, held for its look-ups only
+
+// Takes the device copies of the states at `elts` out of the map; false when there are none.
+bool take_pending_states(const void* elts, PendingStates* out) {
+  std::lock_guard<std::mutex> lock(g_pending_mutex);
+  auto it = g_pending_device_reps.find(elts);
+  if (it == g_pending_device_reps.end()) return false;
+  *out = it->second;
+  g_pending_device_reps.erase(it);
+  return true;
+}
 }
 
 static void drop_pending_states(const void* elts) {
-  auto it = g_pending_device_reps.find(elts);
-  if (it == g_pending_device_reps.end()) return;
-  cudaFree(it->second.reps);
-  cudaFree(it->second.norms);
-  cudaFree(it->second.stab);
-  g_pending_device_reps.erase(it);
+  PendingStates states{};
+  if (!take_pending_states(elts, &states)) return;
+  cudaFree(states.reps);
+  cudaFree(states.norms);
+  cudaFree(states.stab);
 }
 
 struct ls_hs_state_index_binary_search_data : IndexData {};
@@ -513,19 +523,18 @@ extern "C" ls_hs_state_index_binary_search_data* ls_hs_create_state_index_binary
   ix->number_bits = number_bits;
   ix->prefix_bits = std::min(prefix_bits, number_bits);
   cudaStream_t s = default_stream();
-  auto it = g_pending_device_reps.find(representatives->elts);
-  if (it != g_pending_device_reps.end()) {
+  PendingStates states{};
+  if (take_pending_states(representatives->elts, &states)) {
     ix->enumerated = true;
-    ix->d_reps = it->second.reps;
-    ix->d_norms = it->second.norms;
+    ix->d_reps = states.reps;
+    ix->d_norms = states.norms;
     if (ix->d_norms != nullptr) {
-      ix->norms_for = it->second.norms_for;
+      ix->norms_for = states.norms_for;
       ix->dev.norms = ix->d_norms;
       ix->dev.inv_norms = ix->d_norms + std::max<int64_t>(ix->n_states, 1);
     }
-    ix->d_stab = it->second.stab;
-    ix->stab_for = it->second.norms_for;
-    g_pending_device_reps.erase(it);
+    ix->d_stab = states.stab;
+    ix->stab_for = states.norms_for;
   } else {
     if (!cuda_ok(cudaMalloc((void**)&ix->d_reps, std::max<int64_t>(ix->n_states, 1) * 8), "cudaMalloc(reps)") ||
         (ix->n_states > 0 &&
@@ -848,6 +857,7 @@ extern "C" void ls_chpl_enumerate_representatives(ls_hs_basis* p, uint64_t lower
     return;
   }
   drop_pending_states(h);
+  std::lock_guard<std::mutex> pending(g_pending_mutex);
   g_pending_device_reps[h] = PendingStates{d, norms, stab, basis_orbit(p)};
   dest->elts = h;
   dest->num_elts = (uint64_t)n;
