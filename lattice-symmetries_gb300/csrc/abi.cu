@@ -485,6 +485,7 @@ struct PendingStates {
   double* norms;   // norms | inverse norms (projected bases), or null
   uint16_t* stab;  // stabiliser sizes, or null
   const OrbitData* norms_for;
+  uint64_t count;
 };
 std::unordered_map<const void*, PendingStates> g_pending_device_reps;
 std::mutex g_pending_mutex;  // of the map, held for its look-ups only
@@ -524,7 +525,14 @@ extern "C" ls_hs_state_index_binary_search_data* ls_hs_create_state_index_binary
   ix->prefix_bits = std::min(prefix_bits, number_bits);
   cudaStream_t s = default_stream();
   PendingStates states{};
-  if (take_pending_states(representatives->elts, &states)) {
+  bool enumerated = take_pending_states(representatives->elts, &states);
+  if (enumerated && states.count != representatives->num_elts) {  // part of the array
+    cudaFree(states.reps);
+    cudaFree(states.norms);
+    cudaFree(states.stab);
+    enumerated = false;
+  }
+  if (enumerated) {
     ix->enumerated = true;
     ix->d_reps = states.reps;
     ix->d_norms = states.norms;
@@ -858,7 +866,7 @@ extern "C" void ls_chpl_enumerate_representatives(ls_hs_basis* p, uint64_t lower
   }
   drop_pending_states(h);
   std::lock_guard<std::mutex> pending(g_pending_mutex);
-  g_pending_device_reps[h] = PendingStates{d, norms, stab, basis_orbit(p)};
+  g_pending_device_reps[h] = PendingStates{d, norms, stab, basis_orbit(p), (uint64_t)n};
   dest->elts = h;
   dest->num_elts = (uint64_t)n;
   dest->freer = (void*)&free_states;
