@@ -1477,7 +1477,11 @@ int ensure_ranks(IndexData* ix, ls_hs_basis const* b, bool* pending) {
   if (ix->n_states != expected) return 0;
   cudaStream_t s = default_stream();
   const size_t lo = (size_t)1 << split, hi = (size_t)1 << (n - split);
-  if (!cuda_ok(cudaMalloc((void**)&ix->d_ranks, (lo + hi + 1) * 4), "cudaMalloc(ranks)")) return LS_GPU_ERR_CUDA;
+  if (cudaMalloc((void**)&ix->d_ranks, (lo + hi + 1) * 4) != cudaSuccess) {  // the search needs none
+    cudaGetLastError();
+    ix->d_ranks = nullptr;
+    return 0;
+  }
   int bad = 0;
   int* d_bad = (int*)(ix->d_ranks + lo + hi);
   int rc = launch_rank_tables(split, n - split, h, species, n_lo, ix->d_ranks, ix->d_ranks + lo, s);
