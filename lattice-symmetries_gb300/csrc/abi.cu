@@ -533,7 +533,6 @@ extern "C" ls_hs_state_index_binary_search_data* ls_hs_create_state_index_binary
     enumerated = false;
   }
   if (enumerated) {
-    ix->enumerated = true;
     ix->d_reps = states.reps;
     ix->d_norms = states.norms;
     if (ix->d_norms != nullptr) {
@@ -888,6 +887,9 @@ extern "C" void ls_hs_build_representatives(ls_hs_basis* basis, uint64_t lower, 
   basis->kernels->state_index_data =
       ls_hs_create_state_index_binary_search_kernel_data(&basis->representatives, number_bits, 22);
   basis->kernels->state_index_kernel = &ls_hs_state_index_binary_search_kernel;
+  // (another host may have put its own enumeration into the table)
+  if (IndexData* ix = basis_index(basis))
+    ix->enumerated = (void*)kernels->enumerate_states == (void*)&ls_chpl_enumerate_representatives;
 }
 
 // reference.c:196-211

@@ -185,7 +185,7 @@ struct IndexData {
   uint16_t* d_stab = nullptr;         // stabiliser sizes from the enumeration (group stab_for) until the norms are made
   const OrbitData* stab_for = nullptr;
   uint32_t* d_ranks = nullptr;        // rank_lo | rank_hi of DeviceIndex, filled by the first matvec without a group
-  bool enumerated = false;            // the states come from this library's enumeration
+  bool enumerated = false;            // the states are this library's enumeration of the basis
   bool ranks_refused = false;         // ... or from the caller, and are not the complete basis
 };
 

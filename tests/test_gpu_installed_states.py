@@ -55,3 +55,24 @@ def test_complete_two_species_states():
     e = ls.Expr("c†₀↑ c₁↑ + c†₁↑ c₀↑ + c†₀↓ c₁↓ + c†₁↓ c₀↓", sites=[[i, i + 1] for i in range(4)])
     x = torch.from_numpy(np.random.default_rng(5).normal(size=len(states))).cuda()
     assert torch.equal(ls.Operator(basis, e).apply_device(x), ls.Operator(loaded, e).apply_device(x))
+
+
+def test_states_enumerated_for_another_basis():
+    """56 states of weight 3 of 8 sites installed as those of weight 5, from the enumeration's own array."""
+    from ctypes import byref
+    import torch
+    N = ls._native
+    lib = N.lib()
+    source, basis = ls.SpinlessFermionBasis(8, 3), ls.SpinlessFermionBasis(8, 5)
+    array = N.chpl_external_array(None, 0, None)
+    lib.ls_chpl_enumerate_representatives(source._payload, 0, 0, byref(array))
+    N.check()
+    assert int(array.num_elts) == len(FULL)
+    lib.ls_hs_unchecked_set_representatives(basis._payload, byref(array), 22)
+    N.check()
+    op = ls.Operator(basis, ls.Expr("n₀", sites=[[i] for i in range(4)]))
+    x = np.random.default_rng(11).normal(size=len(FULL))
+    y = op.apply_device(torch.from_numpy(x).cuda()).cpu().numpy()
+    # at most 3 ones a row
+    assert np.allclose(y, x * [bin(s & 15).count("1") for s in FULL], rtol=1e-15)
+    assert op.kernel_route(1, False) == ("plain", 0)
