@@ -173,12 +173,12 @@ static int rows_modes(const MatvecProblem& p, int (&modes)[2]) {
 //    on 6x6, 9212 rows, 165 / 98; 5x5, 150 images, 98 rows 55 / 26).
 // slots: of the packed kernels, or 0 where only the kernel without shared tables could run (one column).
 bool rows_few(const MatvecProblem& p, int k, int slots) {
-  int modes[2];
-  if (rows_modes(p, modes) == 0) return false;
   const int64_t sms = num_sms(), n = p.n_rows;
   const int G = p.group.n_elems;
   const bool wide = p.group.n_bits > 32, full = G == slots;
-  if (k == 1 && p.off.rows.n_slots > 256) return false;
+  if (n > 48 * sms || (k == 1 && (p.off.rows.n_slots > 256 || (!wide && G <= 32 * 9)))) return false;
+  int modes[2];
+  if (rows_modes(p, modes) == 0) return false;
   if (slots == 0) return modes[0] != kModeN32 && k == 1 && n <= 16 * sms;
   if (modes[0] == 16) return n <= (full ? 48 : 32) * sms;
   if (!wide) return k > 1 && G > 64 && full && n * G > 12288 && n <= 32 * sms;
